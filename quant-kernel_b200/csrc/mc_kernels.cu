@@ -24,6 +24,7 @@
 // the std::max(s, 1e-12) floor is the same map as x + a floored at
 // log(1e-12/spot), and it removes the per-step exp; sqrt(v) times the
 // Box-Muller radius is taken as one square root.
+#include "fp64_math.cuh"
 #include "mc_device.cuh"
 #include "mc_launch.h"
 
@@ -109,38 +110,39 @@ __device__ __forceinline__ double clamp_unit(double u) {
 // path k (plain); with an odd antithetic path count, normal n_pairs drives the
 // lone last path.
 // ----------------------------------------------------------------------------
-template <int UPT, bool ANTI>
-__device__ __forceinline__ void sim_terminal(const McOption& o, uint32_t unit0, uint32_t stride,
-                                             uint32_t k0, uint32_t k1, Acc& acc) {
+//
+// terminal_unit is one unit with CUDA's FP64 functions, for any constants
+// (terminal_quad below is the fast form); out of line, so that its registers
+// do not count against the fast loop.
+template <bool ANTI>
+__device__ __noinline__ Acc terminal_unit(const McOption* __restrict__ rec, uint32_t unit) {
+    const McOption& o = *rec;
+    const uint32_t k0 = (uint32_t)o.seed, k1 = (uint32_t)(o.seed >> 32);
     const double d0 = o.d[0], d1 = o.d[1];
     const uint32_t n_pairs = (uint32_t)o.paths >> 1;
     const uint32_t n_norm = ANTI ? (uint32_t)(o.paths - (int32_t)n_pairs) : (uint32_t)o.paths;
-    const bool odd = (o.paths & 1) != 0;
+    Acc acc;
+    double z[4];
+    normals4_f64(unit, ANTI ? 0u : 1u, k0, k1, z);
 #pragma unroll
-    for (int k = 0; k < UPT; ++k) {
-        const uint32_t unit = unit0 + (uint32_t)k * stride;
-        if (unit * 4u >= n_norm) continue;
-        double z[4];
-        normals4_f64(unit, ANTI ? 0u : 1u, k0, k1, z);
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            const uint32_t idx = unit * 4u + (uint32_t)s;
-            if (idx >= n_norm) break;
-            const double dz = __dmul_rn(d1, z[s]);
-            const double su = o.spot * exp(__dadd_rn(d0, dz));
-            const double a = payoff(su, o.strike, o.option_type);
-            if (ANTI) {
-                if (idx < n_pairs) {
-                    const double sd = o.spot * exp(__dadd_rn(d0, -dz));
-                    acc.add_pair(a, payoff(sd, o.strike, o.option_type));
-                } else if (odd) {
-                    acc.add_lone(a);
-                }
+    for (int s = 0; s < 4; ++s) {
+        const uint32_t idx = unit * 4u + (uint32_t)s;
+        if (idx >= n_norm) break;
+        const double dz = __dmul_rn(d1, z[s]);
+        const double su = o.spot * exp(__dadd_rn(d0, dz));
+        const double a = payoff(su, o.strike, o.option_type);
+        if (ANTI) {
+            if (idx < n_pairs) {
+                const double sd = o.spot * exp(__dadd_rn(d0, -dz));
+                acc.add_pair(a, payoff(sd, o.strike, o.option_type));
             } else {
-                acc.add_plain(a);
+                acc.add_lone(a);  // the last path of an odd count
             }
+        } else {
+            acc.add_plain(a);
         }
     }
+    return acc;
 }
 
 // ----------------------------------------------------------------------------
@@ -540,108 +542,417 @@ __device__ __forceinline__ void sim_heston(const McOption& o, uint32_t unit0, ui
 //                      Corput sequence in Gray-code order (Sobol, dimension
 //                      one) or natural order (Halton base 2), z = Acklam(u)
 // ----------------------------------------------------------------------------
-template <int UPT>
-__device__ __forceinline__ void sim_vr(const McOption& o, uint32_t unit0, uint32_t stride,
-                                       uint32_t k0, uint32_t k1, Acc& acc) {
+//
+// vr_unit is one unit with CUDA's FP64 functions, for any constants (vr_quad
+// below is the fast form).
+__device__ __noinline__ Acc vr_unit(const McOption* __restrict__ rec, uint32_t unit) {
+    const McOption& o = *rec;
+    const uint32_t k0 = (uint32_t)o.seed, k1 = (uint32_t)(o.seed >> 32);
     const uint32_t n = (uint32_t)o.paths;
     const int32_t m = o.model;
     const double d0 = o.d[0], d1 = o.d[1], shift = o.d[2], mean_st = o.d[3];
-#pragma unroll
-    for (int k = 0; k < UPT; ++k) {
-        const uint32_t unit = unit0 + (uint32_t)k * stride;
-        if (unit * 4u >= n) continue;
-        double z[4];
-        if (m == kQmcSobol || m == kQmcHalton) {
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                const uint32_t i1 = unit * 4u + (uint32_t)s + 1u;
-                // quasi_monte_carlo.cpp:23-24 / 46-47 with internal_util.h:104-130:
-                // bit j of the (Gray-coded) index goes to bit 31 - j.
-                const uint32_t x = __brev(m == kQmcSobol ? (i1 ^ (i1 >> 1)) : i1);
-                const double u = m == kQmcSobol ? ((double)x + 0.5) / 4294967296.0
-                                                : (double)x * 0x1p-32;
-                z[s] = acklam_inv(clamp_unit(u));
-            }
-        } else if (m == kStratified) {
-            const U4 w = philox4x32_10(unit, 0u, 0u, 2u, k0, k1);
-            const uint32_t bits[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                const double ui = ((double)bits[s] + 0.5) * 0x1p-32;
-                const double u = ((double)(unit * 4u + (uint32_t)s) + ui) / (double)n;
-                z[s] = acklam_inv(clamp_unit(u));
-            }
-        } else {
-            normals4_f64(unit, 1u, k0, k1, z);
-        }
-        double y[4];
+    Acc acc;
+    double z[4];
+    if (m == kQmcSobol || m == kQmcHalton) {
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-            const bool valid = unit * 4u + (uint32_t)s < n;
-            double zz = z[s];
-            double w = 1.0;
-            if (m == kImportanceSampling) {
-                zz = z[s] + shift;
-                w = exp(-shift * zz + 0.5 * shift * shift);
-            }
-            const double st = o.spot * exp(d0 + d1 * zz);
-            const double pay = payoff(st, o.strike, o.option_type) * w;
-            y[s] = pay;
-            if (!valid) continue;
-            acc.sy = dd_add(acc.sy, pay);
-            if (m != kStratified) acc.q = dd_add(acc.q, pay * pay);
-            if (m == kControlVariates) {
-                const double c = st - mean_st;
-                acc.cx += c;
-                acc.cxx += c * c;
-                acc.cxy += c * pay;
-            }
+            const uint32_t i1 = unit * 4u + (uint32_t)s + 1u;
+            // quasi_monte_carlo.cpp:23-24 / 46-47 with internal_util.h:104-130:
+            // bit j of the (Gray-coded) index goes to bit 31 - j.
+            const uint32_t x = __brev(m == kQmcSobol ? (i1 ^ (i1 >> 1)) : i1);
+            const double u = m == kQmcSobol ? ((double)x + 0.5) / 4294967296.0
+                                            : (double)x * 0x1p-32;
+            z[s] = acklam_inv(clamp_unit(u));
         }
-        if (m == kStratified) {
+    } else if (m == kStratified) {
+        const U4 w = philox4x32_10(unit, 0u, 0u, 2u, k0, k1);
+        const uint32_t bits[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-            for (int s = 0; s < 4; s += 2) {
-                if (unit * 4u + (uint32_t)s + 1u < n) {
-                    const double dy = y[s] - y[s + 1];
-                    acc.q = dd_add(acc.q, dy * dy);
-                }
+        for (int s = 0; s < 4; ++s) {
+            const double ui = ((double)bits[s] + 0.5) * 0x1p-32;
+            const double u = ((double)(unit * 4u + (uint32_t)s) + ui) / (double)n;
+            z[s] = acklam_inv(clamp_unit(u));
+        }
+    } else {
+        normals4_f64(unit, 1u, k0, k1, z);
+    }
+    double y[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        const bool valid = unit * 4u + (uint32_t)s < n;
+        double zz = z[s];
+        double w = 1.0;
+        if (m == kImportanceSampling) {
+            zz = z[s] + shift;
+            w = exp(-shift * zz + 0.5 * shift * shift);
+        }
+        const double st = o.spot * exp(d0 + d1 * zz);
+        const double pay = payoff(st, o.strike, o.option_type) * w;
+        y[s] = pay;
+        if (!valid) continue;
+        acc.sy = dd_add(acc.sy, pay);
+        if (m != kStratified) acc.q = dd_add(acc.q, pay * pay);
+        if (m == kControlVariates) {
+            const double c = st - mean_st;
+            acc.cx += c;
+            acc.cxx += c * c;
+            acc.cxy += c * pay;
+        }
+    }
+    if (m == kStratified) {
+#pragma unroll
+        for (int s = 0; s < 4; s += 2) {
+            if (unit * 4u + (uint32_t)s + 1u < n) {
+                const double dy = y[s] - y[s + 1];
+                acc.q = dd_add(acc.q, dy * dy);
             }
         }
     }
+    return acc;
+}
+
+// ----------------------------------------------------------------------------
+// The FP64 families (terminal, variance reduction), fast form.
+//
+// Bound by the FP64 pipe and by issue: with CUDA's functions an antithetic
+// pair took 110 FP64 instructions of 259 in all, a Sobol point 165.  Here the
+// functions of fp64_math.cuh serve options whose constants bound every
+// argument (fp64_bounds), payoffs take one FMA and an integer sign mask, and
+// the double-double sums start at a power of two above every term, so that
+// each addition's error comes from a three-operation FastTwoSum instead of
+// TwoSum's six and its finiteness test.
+// Measured: 64 x 131072 antithetic paths, kernel 49.5 -> 33 us; 64 x 2^20
+// paths end to end, importance sampling 719 -> 483 us, control variates 634 ->
+// 437, stratified 635 -> 413, Halton 762 -> 360, Sobol 944 -> 378 us.
+// ----------------------------------------------------------------------------
+
+// Largest |z|: Box-Muller radii reach sqrt(2 53 ln 2) = 8.572, Acklam's inverse
+// 7.1 at the clamp.
+constexpr double kZMax = 8.6;
+
+// Whether option o stays inside fp64_math's ranges, and then the starting
+// values of its sums: powers of two above 4 max y and 16 max y^2, from the
+// exponents of spot, strike and the largest path and weight factors.
+// Factors up to e^300 with spot, strike in [1e-100, 1e20] keep every y below
+// 1e152, so y^2 and its sums stay finite.  NaN constants fail the comparison.
+__device__ __forceinline__ bool fp64_bounds(const McOption& o, double& b_y, double& b_q) {
+    const double sh = o.model == kImportanceSampling ? fabs(o.d[2]) : 0.0;
+    const double path = fabs(o.d[0]) + fabs(o.d[1]) * (kZMax + sh);
+    const double weight = sh * (kZMax + 1.5 * sh);
+    if (!(path + weight <= 300.0 && o.spot >= 1e-100 && o.spot <= 1e20 && o.strike >= 1e-100 &&
+          o.strike <= 1e20))
+        return false;
+    const int32_t top = max(__double2hiint(o.spot), __double2hiint(o.strike)) >> 20;
+    const int32_t grow = (int32_t)((float)(path + weight) * 1.4427f);
+    // y <= (spot + strike) 2^(grow + 1) < 2^(top + grow + 3), biased exponent
+    b_y = __hiloint2double((top + grow + 5) << 20, 0);
+    b_q = b_y * b_y;
+    return true;
+}
+
+// A double-double sum of terms in [0, b) that starts at b (so hi >= every term).
+struct BiasedSum {
+    double hi, lo;
+    __device__ __forceinline__ void add(double y) {
+        const double s = __dadd_rn(hi, y);
+        lo = __dadd_rn(lo, __dsub_rn(y, __dsub_rn(s, hi)));
+        hi = s;
+    }
+};
+
+// max(x, 0) for finite x by its sign bit.
+__device__ __forceinline__ double relu_bits(double x) {
+    const int32_t keep = ~(__double2hiint(x) >> 31);
+    return __hiloint2double(__double2hiint(x) & keep, __double2loint(x) & keep);
+}
+
+// box_muller_f64 with fp64_math: the same words and normals.  The angle
+// pi g = pi ((gb + 1/2) 2^-51 - 1) is j pi/16 plus a remainder r in +-pi/32,
+// both straight from the bits: with gb rounded to a multiple of 2^47, the
+// 47 bits f left over (offset by 2^46) give r = (f - 2^46 + 1/2) pi 2^-51,
+// formed as y - (1 + 2^-2 - 2^-49) (exact) with f 2^-48 in the mantissa of 1.0.
+__device__ __forceinline__ void box_muller_fast(U4 x, const Fp64Tables& t, double& za, double& zb) {
+    const double u = __hiloint2double(0x3FF00000 | (int32_t)(x.x >> 12),
+                                      (int32_t)((x.x << 20) | (x.y >> 12))) -
+                     0x1.fffffffffffffp-1;
+    const uint32_t zr = x.z + (1u << 26);
+    const double y = __hiloint2double(0x3FF00000 | (int32_t)((zr >> 8) & 0x7FFFFu),
+                                      (int32_t)((zr << 24) | ((x.w >> 8) & 0x00FFFFF0u)));
+    const double r = (y - (1.25 - 0x1p-49)) * 0x1.921fb54442d18p-2;  // pi / 8
+    double sn, cs;
+    fp64_sincos_at((int32_t)(zr >> 27) + 16, r, t, sn, cs);
+    const double rad = fp64_sqrt(-2.0 * fp64_log(u, t));
+    za = rad * cs;
+    zb = rad * sn;
+}
+
+__device__ __forceinline__ void normals4_fast(uint32_t unit, uint32_t c3, uint32_t k0, uint32_t k1,
+                                              const Fp64Tables& t, double z[4]) {
+    box_muller_fast(philox4x32_10(unit, 0u, 0u, c3, k0, k1), t, z[0], z[1]);
+    box_muller_fast(philox4x32_10(unit, 1u, 0u, c3, k0, k1), t, z[2], z[3]);
+}
+
+// Acklam's published coefficients (as in acklam_inv), read from the constant
+// bank: centre numerator and denominator, tail numerator and denominator,
+// highest power first (denominators end in 1).
+__constant__ double c_acklam[21] = {
+    -3.969683028665376e+01, 2.209460984245205e+02,  -2.759285104469687e+02, 1.383577518672690e+02,
+    -3.066479806614716e+01, 2.506628277459239e+00,  -5.447609879822406e+01, 1.615858368580409e+02,
+    -1.556989798598866e+02, 6.680131188771972e+01,  -1.328068155288572e+01, -7.784894002430293e-03,
+    -3.223964580411365e-01, -2.400758277161838e+00, -2.549732539343734e+00, 4.374664141464968e+00,
+    2.938163982698783e+00,  7.784695709041462e-03,  3.224671290700398e-01,  2.445134137142996e+00,
+    3.754408661907416e+00};
+
+// acklam_inv for p = 1/2 + h, 0 < p < 1, Horner steps fused.
+__device__ __forceinline__ double acklam_fast(double p, double h, const Fp64Tables& t) {
+    double num, den;
+    if (fabs(h) > 0.47575) {  // p < 0.02425 or p > 1 - 0.02425
+        const double x = fp64_sqrt(-2.0 * fp64_log(h < 0.0 ? p : 1.0 - p, t));
+        num = fma(c_acklam[11], x, c_acklam[12]);
+#pragma unroll
+        for (int i = 13; i < 17; ++i) num = fma(num, x, c_acklam[i]);
+        den = fma(c_acklam[17], x, c_acklam[18]);
+        den = fma(den, x, c_acklam[19]);
+        den = fma(den, x, c_acklam[20]);
+        den = fma(den, x, 1.0);
+        num = h < 0.0 ? num : -num;
+    } else {
+        const double x = h * h;
+        num = fma(c_acklam[0], x, c_acklam[1]);
+#pragma unroll
+        for (int i = 2; i < 6; ++i) num = fma(num, x, c_acklam[i]);
+        num *= h;
+        den = fma(c_acklam[6], x, c_acklam[7]);
+#pragma unroll
+        for (int i = 8; i < 11; ++i) den = fma(den, x, c_acklam[i]);
+        den = fma(den, x, 1.0);
+    }
+    return num * fp64_rcp(den);
+}
+
+// One full quad of a terminal option (every normal drives a path or a pair).
+template <bool ANTI>
+__device__ __forceinline__ void terminal_quad(const McOption& o, double spot, double strike,
+                                              uint32_t unit, uint32_t k0, uint32_t k1,
+                                              const Fp64Tables& t, BiasedSum& sy, BiasedSum& q) {
+    double z[4];
+    normals4_fast(unit, ANTI ? 0u : 1u, k0, k1, t, z);
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        double y = relu_bits(fma(spot, fp64_exp<true>(fma(o.d[1], z[s], o.d[0]), t), strike));
+        // antithetic: twice the pair mean
+        if (ANTI)
+            y += relu_bits(fma(spot, fp64_exp<true>(fma(-o.d[1], z[s], o.d[0]), t), strike));
+        sy.add(y);
+        q.add(__dmul_rn(y, y));
+    }
+}
+
+// One full quad of a variance-reduction option; MODEL is uniform in the launch's tile.
+template <int32_t MODEL>
+__device__ __forceinline__ void vr_quad(const McOption& o, double spot, double strike,
+                                        double inv_n, uint32_t unit, uint32_t k0, uint32_t k1,
+                                        const Fp64Tables& t, BiasedSum& sy, BiasedSum& q, Acc& cv) {
+    double z[4];
+    if constexpr (MODEL == kQmcSobol || MODEL == kQmcHalton) {
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const uint32_t i1 = unit * 4u + (uint32_t)s + 1u;
+            const uint32_t x = __brev(MODEL == kQmcSobol ? (i1 ^ (i1 >> 1)) : i1);
+            // u - 1/2, exactly: x in the top mantissa bits of 1.0 (i1 >= 1, so
+            // u and 1 - u are above the reference's clamp of 1e-12)
+            const double h = __hiloint2double(0x3FF00000 | (int32_t)(x >> 12), (int32_t)(x << 20)) -
+                             (MODEL == kQmcSobol ? 1.5 - 0x1p-33 : 1.5);
+            z[s] = acklam_fast(h + 0.5, h, t);
+        }
+    } else if constexpr (MODEL == kStratified) {
+        const U4 w = philox4x32_10(unit, 0u, 0u, 2u, k0, k1);
+        const uint32_t bits[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            // the stratum and (bits + 1/2) 2^-32, both exact, from their bits
+            const uint32_t i = unit * 4u + (uint32_t)s;
+            const double ui = __hiloint2double(0x3FF00000 | (int32_t)(bits[s] >> 12),
+                                               (int32_t)(bits[s] << 20)) - (1.0 - 0x1p-33);
+            const double id = __hiloint2double(0x43300000, (int32_t)i) - 0x1p+52;
+            // the quotient: q0 and the residual it leaves
+            const double num = id + ui, n = (double)o.paths;
+            const double q0 = num * inv_n;
+            const double u = fma(fma(-q0, n, num), inv_n, q0);
+            const double c = clamp_unit(u);
+            z[s] = acklam_fast(c, c - 0.5, t);
+        }
+    } else {
+        normals4_fast(unit, 1u, k0, k1, t, z);
+    }
+    double y[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        if constexpr (MODEL == kControlVariates) {
+            const double st = o.spot * fp64_exp<true>(fma(o.d[1], z[s], o.d[0]), t);
+            y[s] = relu_bits(spot > 0.0 ? st + strike : strike - st);
+            const double c = st - o.d[3];
+            cv.cx += c;
+            cv.cxx = fma(c, c, cv.cxx);
+            cv.cxy = fma(c, y[s], cv.cxy);
+        } else if constexpr (MODEL == kImportanceSampling) {
+            const double sh = o.d[2], zz = z[s] + sh;
+            const double w = fp64_exp<true>(fma(-sh, zz, 0.5 * sh * sh), t);
+            y[s] = relu_bits(fma(spot, fp64_exp<true>(fma(o.d[1], zz, o.d[0]), t), strike)) * w;
+        } else {
+            y[s] = relu_bits(fma(spot, fp64_exp<true>(fma(o.d[1], z[s], o.d[0]), t), strike));
+        }
+        sy.add(y[s]);
+        if (MODEL != kStratified) q.add(__dmul_rn(y[s], y[s]));
+    }
+    if constexpr (MODEL == kStratified) {
+#pragma unroll
+        for (int s = 0; s < 4; s += 2) {
+            const double dy = y[s] - y[s + 1];
+            q.add(__dmul_rn(dy, dy));
+        }
+    }
+}
+
+__device__ __forceinline__ void acc_merge(Acc& a, const Acc& b) {
+    a.sy = dd_merge(a.sy, b.sy);
+    a.q = dd_merge(a.q, b.q);
+    a.lone = __dadd_rn(a.lone, b.lone);
+    a.cx = __dadd_rn(a.cx, b.cx);
+    a.cxx = __dadd_rn(a.cxx, b.cxx);
+    a.cxy = __dadd_rn(a.cxy, b.cxy);
+}
+
+// The thread's units of one tile of an FP64 option: `per_thread` units, unit k
+// at first + k BLOCK + thread, or -- quasi-Monte Carlo -- at first +
+// thread * per_thread + k.  Neighbouring quasi-random points fall all over
+// (0, 1), so with neighbouring points in a warp half of its Acklam evaluations
+// met a tail (2.4% of the points) in some lane and ran both branches; with a
+// thread's units in a row the lanes of a step share the index's low bits and
+// so the point's high bits, and an eighth (Halton) or a quarter (Sobol) do.
+// Ragged last quads and options outside fp64_bounds take the general unit.
+template <int BLOCK, class Quad, class General>
+__device__ __forceinline__ void fp64_units(bool fast, bool in_row, uint32_t first,
+                                           uint32_t per_thread, uint32_t units, uint32_t full,
+                                           const Quad& quad, const General& general) {
+    for (uint32_t k = 0; k < per_thread; ++k) {
+        const uint32_t unit = in_row ? first + threadIdx.x * per_thread + k
+                                     : first + k * (uint32_t)BLOCK + threadIdx.x;
+        if (unit >= units) break;
+        if (fast && unit < full)
+            quad(unit);
+        else
+            general(unit);
+    }
+}
+
+template <int FAMILY, int BLOCK, bool ANTI>
+__device__ __forceinline__ void sim_fp64_tile(const McOption& o, const McOption* __restrict__ rec,
+                                              uint32_t first, uint32_t per_thread,
+                                              const Fp64Tables& t, Acc& acc) {
+    const uint32_t k0 = (uint32_t)o.seed, k1 = (uint32_t)(o.seed >> 32);
+    double b_y = 0.0, b_q = 0.0;
+    const bool fast = fp64_bounds(o, b_y, b_q);  // uniform in the CTA
+    const double sign = o.option_type == 0 ? 1.0 : -1.0;
+    const double spot = sign * o.spot, strike = -sign * o.strike;
+    BiasedSum sy{b_y, 0.0}, q{b_q, 0.0};
+    const uint32_t units = (uint32_t)o.units;
+    double scale_y = 1.0;
+    if constexpr (FAMILY == kFamTerminal) {
+        const uint32_t full = (ANTI ? (uint32_t)o.paths >> 1 : (uint32_t)o.paths) >> 2;
+        if (ANTI) scale_y = 0.5;
+        fp64_units<BLOCK>(
+            fast, false, first, per_thread, units, full,
+            [&](uint32_t unit) { terminal_quad<ANTI>(o, spot, strike, unit, k0, k1, t, sy, q); },
+            [&](uint32_t unit) { acc_merge(acc, terminal_unit<ANTI>(rec, unit)); });
+    } else {
+        const uint32_t full = (uint32_t)o.paths >> 2;
+        const double inv_n = 1.0 / (double)o.paths;
+        auto general = [&](uint32_t unit) { acc_merge(acc, vr_unit(rec, unit)); };
+        switch (o.model) {
+#define QK_VR(M)                                                                              \
+    case M:                                                                                   \
+        fp64_units<BLOCK>(                                                                    \
+            fast, M == kQmcSobol || M == kQmcHalton, first, per_thread, units, full,          \
+            [&](uint32_t unit) { vr_quad<M>(o, spot, strike, inv_n, unit, k0, k1, t, sy, q, acc); }, \
+            general);                                                                         \
+        break;
+            QK_VR(kControlVariates)
+            QK_VR(kImportanceSampling)
+            QK_VR(kStratified)
+            QK_VR(kQmcSobol)
+            QK_VR(kQmcHalton)
+#undef QK_VR
+            default: break;
+        }
+    }
+    // the biases leave exactly; twice the pair means scale back exactly
+    const double ys = q.hi - b_q;
+    acc.sy = dd_merge(acc.sy, DD{(sy.hi - b_y) * scale_y, sy.lo * scale_y});
+    acc.q = dd_merge(acc.q, DD{ys * (scale_y * scale_y), q.lo * (scale_y * scale_y)});
 }
 
 // ----------------------------------------------------------------------------
 // Fixed-order CTA reduction of (sy, q) into the tile's slot.
 // ----------------------------------------------------------------------------
+//
+// A warp sums sy in its lower half and q in its upper half (the halves swap
+// the other's values first), so each of the five levels merges one
+// double-double per lane: half the shuffles and merges of two full trees.
+// The rarely present parts -- the unpaired path, the control variate's sums
+// -- cost a vote when absent.
 template <int BLOCK, bool CV>
 __device__ __forceinline__ void reduce_tile(Acc acc, TilePartial* __restrict__ out, DD* smem) {
     constexpr int W = BLOCK / 32;
-    DD a = acc.sy, b = acc.q;
-    double lone = acc.lone;  // nonzero in at most one thread: plain sums are exact
-    double cx = acc.cx, cxx = acc.cxx, cxy = acc.cxy;
+    constexpr uint32_t kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool low = lane < 16;
+    const DD give = low ? acc.q : acc.sy;
+    DD a = low ? acc.sy : acc.q;
+    a = dd_merge(a, DD{__shfl_xor_sync(kAll, give.hi, 16), __shfl_xor_sync(kAll, give.lo, 16)});
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        a = dd_merge(a, dd_shfl_down(a, off));
-        b = dd_merge(b, dd_shfl_down(b, off));
-        lone = __dadd_rn(lone, __shfl_down_sync(0xffffffffu, lone, off));
-        if (CV) {
-            cx = __dadd_rn(cx, __shfl_down_sync(0xffffffffu, cx, off));
-            cxx = __dadd_rn(cxx, __shfl_down_sync(0xffffffffu, cxx, off));
-            cxy = __dadd_rn(cxy, __shfl_down_sync(0xffffffffu, cxy, off));
+    for (int off = 8; off > 0; off >>= 1)
+        a = dd_merge(a, DD{__shfl_xor_sync(kAll, a.hi, off), __shfl_xor_sync(kAll, a.lo, off)});
+    // nonzero (or NaN) in at most one thread: plain sums are exact
+    double lone = 0.0;
+    if (__any_sync(kAll, acc.lone != 0.0)) {
+        lone = acc.lone;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+            lone = __dadd_rn(lone, __shfl_down_sync(kAll, lone, off));
+    }
+    double cx = 0.0, cxx = 0.0, cxy = 0.0;
+    if (CV && __any_sync(kAll, acc.cxx != 0.0)) {
+        cx = acc.cx;
+        cxx = acc.cxx;
+        cxy = acc.cxy;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            cx = __dadd_rn(cx, __shfl_down_sync(kAll, cx, off));
+            cxx = __dadd_rn(cxx, __shfl_down_sync(kAll, cxx, off));
+            cxy = __dadd_rn(cxy, __shfl_down_sync(kAll, cxy, off));
         }
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) {
         smem[warp] = a;
-        smem[W + warp] = b;
         smem[2 * W + warp] = DD{lone, 0.0};
         if (CV) {
             smem[3 * W + warp] = DD{cx, cxx};
             smem[4 * W + warp] = DD{cxy, 0.0};
         }
     }
+    if (lane == 16) smem[W + warp] = a;
     __syncthreads();
+    // two threads of different warps, one sum each
+    if (threadIdx.x == 32) {
+        DD tb = smem[W];
+#pragma unroll
+        for (int w = 1; w < W; ++w) tb = dd_merge(tb, smem[W + w]);
+        out->q_hi = tb.hi;
+        out->q_lo = tb.lo;
+    }
     if (threadIdx.x == 0) {
-        DD ta = smem[0], tb = smem[W];
+        DD ta = smem[0];
         double tl = smem[2 * W].hi;
         double tx = 0.0, txx = 0.0, txy = 0.0;
         if (CV) {
@@ -652,7 +963,6 @@ __device__ __forceinline__ void reduce_tile(Acc acc, TilePartial* __restrict__ o
 #pragma unroll
         for (int w = 1; w < W; ++w) {
             ta = dd_merge(ta, smem[w]);
-            tb = dd_merge(tb, smem[W + w]);
             tl = __dadd_rn(tl, smem[2 * W + w].hi);
             if (CV) {
                 tx = __dadd_rn(tx, smem[3 * W + w].hi);
@@ -660,24 +970,26 @@ __device__ __forceinline__ void reduce_tile(Acc acc, TilePartial* __restrict__ o
                 txy = __dadd_rn(txy, smem[4 * W + w].hi);
             }
         }
-        TilePartial t;
-        t.sy_hi = ta.hi;
-        t.sy_lo = ta.lo;
-        t.q_hi = tb.hi;
-        t.q_lo = tb.lo;
-        t.lone = tl;
-        t.cx = tx;
-        t.cxx = txx;
-        t.cxy = txy;
-        *out = t;
+        out->sy_hi = ta.hi;
+        out->sy_lo = ta.lo;
+        out->lone = tl;
+        out->cx = tx;
+        out->cxx = txx;
+        out->cxy = txy;
     }
     __syncthreads();
 }
 
 // Option owning `tile`: the last i with tile_begin[i] <= tile (tile_begin is
-// non-decreasing, n + 1 entries, tile_begin[n] = total tiles).
+// non-decreasing, n + 1 entries, tile_begin[n] = total tiles).  Options of one
+// size, the common batch, have the owner at the proportional place: two loads
+// instead of the search's chain of log2(n).
 __device__ __forceinline__ int32_t find_option(const int64_t* __restrict__ tile_begin, int32_t n,
                                                int64_t tile) {
+    const int64_t t0 = __ldg(tile_begin), total = __ldg(tile_begin + n) - t0;
+    // half a tile in: rounding cannot reach the next option's first tile
+    const int32_t i = min((int32_t)(((double)(tile - t0) + 0.5) * ((double)n * fp64_rcp((double)total))), n - 1);
+    if (__ldg(tile_begin + i) <= tile && tile < __ldg(tile_begin + i + 1)) return i;
     int32_t lo = 0, hi = n - 1;
     while (lo < hi) {
         const int32_t mid = (lo + hi + 1) >> 1;
@@ -689,30 +1001,38 @@ __device__ __forceinline__ int32_t find_option(const int64_t* __restrict__ tile_
     return lo;
 }
 
+template <int FAMILY>
+constexpr bool kIsFp64 = FAMILY == kFamTerminal || FAMILY == kFamVr;
+
 template <int FAMILY, int UPT, bool ANTI, int SU>
 __device__ __forceinline__ void sim_family(const McOption& o, uint32_t unit0, uint32_t stride,
                                            uint32_t k0, uint32_t k1, Acc& acc) {
-    if (FAMILY == kFamTerminal) sim_terminal<UPT, ANTI>(o, unit0, stride, k0, k1, acc);
     if (FAMILY == kFamEuler) sim_stepwise<UPT, ANTI, false, SU>(o, unit0, stride, k0, k1, acc);
     if (FAMILY == kFamMilstein) sim_stepwise<UPT, ANTI, true, SU>(o, unit0, stride, k0, k1, acc);
     if (FAMILY == kFamHeston) sim_heston<UPT, ANTI, false, SU>(o, unit0, stride, k0, k1, acc);
     if (FAMILY == kFamHestonLr) sim_heston<UPT, ANTI, true, SU>(o, unit0, stride, k0, k1, acc);
-    if (FAMILY == kFamVr) sim_vr<UPT>(o, unit0, stride, k0, k1, acc);
 }
 
 // One tile: all UPT * unit_iters units of every thread, then the reduction.
+// `tables` is read by the FP64 families only.
 template <int FAMILY, int BLOCK, int UPT, bool ANTI, int SU = 1>
-__device__ __forceinline__ void run_tile(const McOption& o, int64_t tile, TilePartial* partials,
-                                         DD* smem) {
+__device__ __forceinline__ void run_tile(const McOption& o, const McOption* __restrict__ rec,
+                                         int64_t tile, TilePartial* partials, DD* smem,
+                                         const Fp64Tables* tables) {
     const uint32_t k0 = (uint32_t)o.seed, k1 = (uint32_t)(o.seed >> 32);
     const int64_t local = tile - o.tile_begin;
     const uint32_t per_iter = (uint32_t)(BLOCK * UPT);
     const uint32_t first = (uint32_t)(local * (int64_t)per_iter * o.unit_iters);
     Acc acc;
-    for (int32_t it = 0; it < o.unit_iters; ++it) {
-        const uint32_t base = first + (uint32_t)it * per_iter;
-        if (base >= (uint32_t)o.units) break;
-        sim_family<FAMILY, UPT, ANTI, SU>(o, base + threadIdx.x, (uint32_t)BLOCK, k0, k1, acc);
+    if constexpr (kIsFp64<FAMILY>) {
+        sim_fp64_tile<FAMILY, BLOCK, ANTI>(o, rec, first, (uint32_t)(UPT * o.unit_iters), *tables,
+                                           acc);
+    } else {
+        for (int32_t it = 0; it < o.unit_iters; ++it) {
+            const uint32_t base = first + (uint32_t)it * per_iter;
+            if (base >= (uint32_t)o.units) break;
+            sim_family<FAMILY, UPT, ANTI, SU>(o, base + threadIdx.x, (uint32_t)BLOCK, k0, k1, acc);
+        }
     }
     reduce_tile<BLOCK, FAMILY == kFamVr>(acc, partials + tile, smem);
 }
@@ -724,16 +1044,31 @@ __device__ __forceinline__ void run_tile(const McOption& o, int64_t tile, TilePa
 // No register cap: the kernel is issue- and special-function-bound, and
 // forcing 64 registers (4 CTAs of 256 per SM) added instructions and ran
 // slower on B200 than the compiler's 70 (3 CTAs).
+//
+// The FP64 families are held to 80 registers (six CTAs of 128 per SM): their
+// independent paths fill the FP64 pipe's latency with 24 warps as well as
+// with 32 (64 registers, a few spills) or 20 (within 2% on the 64-option
+// batches).
+template <int FAMILY, int BLOCK>
+constexpr int kMinCtas = kIsFp64<FAMILY> ? 6 * 128 / BLOCK : 0;
+
 template <int FAMILY, int BLOCK, int UPT, bool ANTI, int SU>
-__global__ void __launch_bounds__(BLOCK)
+__global__ void __launch_bounds__(BLOCK, kMinCtas<FAMILY, BLOCK>)
     mc_simulate_kernel(const McOption* __restrict__ opts, const int64_t* __restrict__ tile_begin,
                        int32_t n, int64_t tile0, int64_t n_tiles, TilePartial* __restrict__ partials) {
     __shared__ DD smem[5 * (BLOCK / 32)];
+    Fp64Tables* tables = nullptr;
+    if constexpr (kIsFp64<FAMILY>) {
+        __shared__ Fp64Tables s_tables;
+        fp64_load_tables(s_tables);
+        __syncthreads();
+        tables = &s_tables;
+    }
     for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
         const int64_t tile = tile0 + t;  // tile_begin holds absolute tile indices
         const int32_t oi = find_option(tile_begin, n, tile);
         const McOption o = opts[oi];
-        run_tile<FAMILY, BLOCK, UPT, ANTI, SU>(o, tile, partials, smem);
+        run_tile<FAMILY, BLOCK, UPT, ANTI, SU>(o, opts + oi, tile, partials, smem, tables);
     }
 }
 
@@ -782,14 +1117,15 @@ __device__ __noinline__ int64_t run_group(const McOption* __restrict__ opts,
                                           int32_t opt_hi, int64_t tile_hi,
                                           TilePartial* __restrict__ partials,
                                           unsigned long long* __restrict__ work_counter, DD* smem,
-                                          long long* s_tile, int64_t tile) {
+                                          const Fp64Tables* tables, long long* s_tile,
+                                          int64_t tile) {
     int32_t oi = advance_option(tile_begin, opt_lo, opt_hi, tile);
     McOption o = opts[oi];
     for (;;) {
         // claim the next tile now; thread 0 first uses the result below
         long long next = 0;
         if (threadIdx.x == 0) next = (long long)atomicAdd(work_counter, 1ull);
-        run_tile<FAMILY, BLOCK, UPT, ANTI>(o, tile, partials, smem);  // ends in a CTA barrier
+        run_tile<FAMILY, BLOCK, UPT, ANTI>(o, opts + oi, tile, partials, smem, tables);  // ends in a CTA barrier
         if (threadIdx.x == 0) *s_tile = next;
         __syncthreads();
         // every thread reads s_tile here, and the next write to it follows the
@@ -814,6 +1150,8 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
                          const GroupTable* __restrict__ groups) {
     __shared__ DD smem[5 * (BLOCK / 32)];
     __shared__ long long s_tile;
+    __shared__ Fp64Tables tables;
+    fp64_load_tables(tables);
     if (threadIdx.x == 0) s_tile = (long long)atomicAdd(work_counter, 1ull);
     __syncthreads();
     int64_t tile = s_tile;
@@ -829,7 +1167,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
 #define QK_GROUP(FAM, UPT, ANTI)                                                                  \
     case FAM * 2 + (ANTI ? 1 : 0):                                                               \
         tile = run_group<FAM, BLOCK, UPT, ANTI>(opts, tile_begin, lo, hi, th, partials,          \
-                                                work_counter, smem, &s_tile, tile);              \
+                                                work_counter, smem, &tables, &s_tile, tile);              \
         break;
             QK_GROUP(kFamTerminal, kFamilyUpt<kFamTerminal>, true)
             QK_GROUP(kFamTerminal, kFamilyUpt<kFamTerminal>, false)
