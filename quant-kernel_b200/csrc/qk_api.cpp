@@ -631,12 +631,9 @@ int32_t qk_cf_heston_price_cf_batch(const double* spot, const double* strike, co
                              {integration_limit, "integration_limit"}, {out_prices, "out_prices"}};
     if (int32_t rc = check_nulls(ptrs)) return rc;
     if (n <= 0) return fail_size(n);
-    std::vector<qkb::CfOption> recs(static_cast<size_t>(n));
-    for (int32_t i = 0; i < n; ++i)
-        recs[i] = qkb::pack_cf_option(spot[i], strike[i], t[i], r[i], q[i], v0[i], kappa[i],
-                                      theta[i], sigma[i], rho[i], option_type[i],
-                                      integration_steps[i], integration_limit[i]);
-    cudaError_t e = qkb::heston_cf_price_host(recs.data(), n, out_prices);
+    const qkb::FourierColumns c = {{spot, strike, t, r, q, v0, kappa, theta, sigma, rho,
+                                    integration_limit}, option_type, integration_steps};
+    cudaError_t e = qkb::heston_fourier_price_host(qkb::FourierMethod::kCf, c, n, out_prices);
     return e == cudaSuccess ? QK_OK : fail_cuda(e, "qk_cf_heston_price_cf_batch");
 }
 
@@ -652,12 +649,9 @@ int32_t qk_ftm_cos_fang_oosterlee_heston_price_batch(
                              {truncation_width, "truncation_width"}, {out_prices, "out_prices"}};
     if (int32_t rc = check_nulls(ptrs)) return rc;
     if (n <= 0) return fail_size(n);
-    std::vector<qkb::CfOption> recs(static_cast<size_t>(n));
-    for (int32_t i = 0; i < n; ++i)
-        recs[i] = qkb::pack_cos_option(spot[i], strike[i], t[i], r[i], q[i], v0[i], kappa[i],
-                                       theta[i], sigma[i], rho[i], option_type[i], n_terms[i],
-                                       truncation_width[i]);
-    cudaError_t e = qkb::heston_cf_price_host(recs.data(), n, out_prices);
+    const qkb::FourierColumns c = {{spot, strike, t, r, q, v0, kappa, theta, sigma, rho,
+                                    truncation_width}, option_type, n_terms};
+    cudaError_t e = qkb::heston_fourier_price_host(qkb::FourierMethod::kCos, c, n, out_prices);
     return e == cudaSuccess ? QK_OK : fail_cuda(e, "qk_ftm_cos_fang_oosterlee_heston_price_batch");
 }
 
