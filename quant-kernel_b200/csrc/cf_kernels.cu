@@ -745,8 +745,8 @@ cudaError_t heston_fourier_price_host(FourierMethod method, const FourierColumns
     double* d_out = static_cast<double*>(s.d_out.p);
     double* h_out = static_cast<double*>(s.h_out.p);
     int k = 0;
-    for (int32_t i0 = 0; i0 < n && e == cudaSuccess; i0 += kFourierChunk, k ^= 1) {
-        const int32_t m = std::min(kFourierChunk, n - i0);
+    for (int64_t i0 = 0; i0 < n && e == cudaSuccess; i0 += kFourierChunk, k ^= 1) {
+        const int32_t m = (int32_t)std::min<int64_t>(kFourierChunk, n - i0);
         const size_t at = kFourierRow * static_cast<size_t>(i0), bytes = kFourierRow * static_cast<size_t>(m);
         char* h = static_cast<char*>(s.h_in.p) + at;
         char* d = static_cast<char*>(s.d_in.p) + at;

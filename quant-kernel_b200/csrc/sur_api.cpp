@@ -67,8 +67,6 @@ int32_t sur_status(cudaError_t e, const char* where) {
     return qkb::fail_cuda(e, where);
 }
 
-double smax0(double x) { return (0.0 < x) ? x : 0.0; }
-
 }  // namespace
 
 extern "C" {
@@ -232,71 +230,39 @@ int32_t qk_sur_heston_price_batch(qk_sur_model* model, const double* spot, const
     for (int i = 0; i < 12; ++i)
         if (!ptrs[i]) return qkb::fail_null(names[i]);
     if (n <= 0) return qkb::fail_size(n);
-    const double nan = std::numeric_limits<double>::quiet_NaN();
-    std::vector<int32_t> sur_idx, mc_idx;
-    std::vector<double> feats;
-    for (int32_t i = 0; i < n; ++i) {
-        const int32_t ot = option_type[i];
-        // entry checks of heston_monte_carlo.cpp:18-26
-        const bool bad = !(ot == 0 || ot == 1) || spot[i] <= 0.0 || strike[i] <= 0.0 || t[i] < 0.0 ||
-                         v0[i] < 0.0 || kappa[i] < 0.0 || theta[i] < 0.0 || sigma[i] < 0.0 ||
-                         rho[i] < -1.0 || rho[i] > 1.0;
-        if (bad) {
-            out_prices[i] = nan;
-            if (out_source) out_source[i] = 2;
-            continue;
-        }
-        if (t[i] <= 1e-12) {
-            out_prices[i] = ot == 0 ? smax0(spot[i] - strike[i]) : smax0(strike[i] - spot[i]);
-            if (out_source) out_source[i] = 2;
-            continue;
-        }
-        const double f[qkb::kSurIn] = {spot[i] / strike[i], t[i], r[i], q[i], v0[i],
-                                       kappa[i], theta[i], sigma[i], rho[i]};
-        if (model->m.in_box(f)) {
-            sur_idx.push_back(i);
-            feats.insert(feats.end(), f, f + qkb::kSurIn);
-        } else {
-            mc_idx.push_back(i);
-        }
+    // entry checks, routing, features, the network and put-call parity all
+    // run on the GPU; only the options outside the box come back to the host
+    std::vector<int32_t> own_route;
+    if (!out_source) {
+        own_route.resize(static_cast<size_t>(n));
+        out_source = own_route.data();
     }
-    if (!sur_idx.empty()) {
-        std::vector<double> y(sur_idx.size());
-        int32_t rc = sur_status(model->m.predict(feats.data(), static_cast<int64_t>(sur_idx.size()), y.data()),
-                                "qk_sur_heston_price_batch");
-        if (rc != QK_OK) return rc;
-        for (size_t k = 0; k < sur_idx.size(); ++k) {
-            const int32_t i = sur_idx[k];
-            const double call = spot[i] * y[k];
-            out_prices[i] = option_type[i] == 0
-                                ? call
-                                : call - spot[i] * std::exp(-q[i] * t[i]) + strike[i] * std::exp(-r[i] * t[i]);
-            if (out_source) out_source[i] = 0;
-        }
-    }
+    const double* const cols[10] = {spot, strike, t, r, q, v0, kappa, theta, sigma, rho};
+    int32_t rc = sur_status(model->m.price_quotes(cols, option_type, n, out_prices, out_source),
+                            "qk_sur_heston_price_batch");
+    if (rc != QK_OK) return rc;
+    std::vector<int32_t> mc_idx;
+    for (int32_t i = 0; i < n; ++i)
+        if (out_source[i] == 1) mc_idx.push_back(i);
     if (!mc_idx.empty()) {
         const size_t m = mc_idx.size();
         std::vector<double> a[10];
         for (auto& v : a) v.resize(m);
         std::vector<int32_t> ot(m), pp(m, fallback_paths), st(m, fallback_steps);
         std::vector<uint64_t> sd(m);
-        const double* src[10] = {spot, strike, t, r, q, v0, kappa, theta, sigma, rho};
         for (size_t k = 0; k < m; ++k) {
             const int32_t i = mc_idx[k];
-            for (int c = 0; c < 10; ++c) a[c][k] = src[c][i];
+            for (int c = 0; c < 10; ++c) a[c][k] = cols[c][i];
             ot[k] = option_type[i];
             sd[k] = fallback_seed + static_cast<uint64_t>(i);
         }
         std::vector<double> out(m);
-        int32_t rc = qk_mcm_heston_monte_carlo_price_batch(
+        rc = qk_mcm_heston_monte_carlo_price_batch(
             a[0].data(), a[1].data(), a[2].data(), a[3].data(), a[4].data(), a[5].data(), a[6].data(),
             a[7].data(), a[8].data(), a[9].data(), ot.data(), pp.data(), st.data(), sd.data(),
             static_cast<int32_t>(m), out.data());
         if (rc != QK_OK) return rc;
-        for (size_t k = 0; k < m; ++k) {
-            out_prices[mc_idx[k]] = out[k];
-            if (out_source) out_source[mc_idx[k]] = 1;
-        }
+        for (size_t k = 0; k < m; ++k) out_prices[mc_idx[k]] = out[k];
     }
     return QK_OK;
 }

@@ -22,11 +22,14 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <memory>
 #include <numeric>
 #include <random>
 #include <vector>
 
 #include "mc_device.cuh"
+#include "mc_plan.h"
 #include "sur_gemm.cuh"
 
 namespace qkb {
@@ -157,6 +160,77 @@ features_kernel(const double* __restrict__ f, int64_t n, SurBox box, int32_t kin
         const int64_t row = row0 + r;
         if (row < n) out[row * 8 + c] = c < 2 ? stage[r][c] : zero;
     }
+}
+
+// The host pricing call, read straight from its pinned slot: ten double
+// columns (spot, strike, t, r, q, v0, kappa, theta, sigma, rho), then
+// option_type, n each, coalesced.  One thread per option decides its route --
+// 0: the network, 1: Monte Carlo (outside the box; NaN until priced), 2: entry
+// checks of heston_monte_carlo.cpp:18-26 -- and writes the network's row (its
+// first 32 bytes, all that the fused kernel reads) and base; other routes get
+// a row of zeros.  fix holds what quote_price_kernel needs: (spot, S e^-qT, K
+// e^-rT) for a put, (spot, 0, 0) for a call, (0, -result, 0) for routes 1, 2.
+// Bound by the copy into the slot and PCIe (84 bytes an option): on the host,
+// the checks, bf16 rows and base took 180 ns an option on one thread (20,000
+// quotes 3.70 ms a call, now 0.23; 200,000 34 ms, now 1.46).
+__global__ void __launch_bounds__(kFeatRows)
+quote_features_kernel(const double* __restrict__ in, int64_t n, SurBox box, int32_t kind,
+                      __nv_bfloat16* __restrict__ rows, float* __restrict__ base,
+                      double* __restrict__ fix, int32_t* __restrict__ out_route) {
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * kFeatRows + threadIdx.x;
+    if (i >= n) return;
+    double c[10];
+#pragma unroll
+    for (int k = 0; k < 10; ++k) c[k] = in[k * n + i];
+    const int32_t ot = reinterpret_cast<const int32_t*>(in + 10 * n)[i];
+    const double spot = c[0], strike = c[1], t = c[2];
+    int32_t to = 2;
+    unsigned short b[16] = {};
+    float base_i = 0.0f;
+    double f0 = 0.0, f1 = 0.0, f2 = 0.0;
+    if (!(ot == 0 || ot == 1) || spot <= 0.0 || strike <= 0.0 || t < 0.0 || c[5] < 0.0 ||
+        c[6] < 0.0 || c[7] < 0.0 || c[8] < 0.0 || c[9] < -1.0 || c[9] > 1.0) {
+        f1 = __longlong_as_double(0x7FF8000000000000ll);
+    } else if (t <= 1e-12) {
+        const double d = ot == 0 ? spot - strike : strike - spot;
+        f1 = (0.0 < d) ? -d : 0.0;
+    } else {
+        const double x[kSurIn] = {spot / strike, t, c[3], c[4], c[5], c[6], c[7], c[8], c[9]};
+        bool inside = true;
+#pragma unroll
+        for (int k = 0; k < kSurIn; ++k) inside = inside && x[k] >= box.lo[k] && x[k] <= box.hi[k];
+        to = inside ? 0 : 1;
+        if (!inside) {
+            f1 = __longlong_as_double(0x7FF8000000000000ll);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kSurIn; ++k) b[k] = sur_norm_bits(x[k], box.lo[k], box.hi[k]);
+            if (kind == kSurBaseBsmMeanVar) base_i = static_cast<float>(sur_base(x));
+            f0 = spot;
+            if (ot == 1) {
+                f1 = spot * exp(-c[4] * t);
+                f2 = strike * exp(-c[3] * t);
+            }
+        }
+    }
+    out_route[i] = to;
+    base[i] = base_i;
+    fix[i] = f0;
+    fix[n + i] = f1;
+    fix[2 * n + i] = f2;
+    uint4* row = reinterpret_cast<uint4*>(rows + i * kSurInPad);
+    row[0] = make_uint4(b[0] | (static_cast<uint32_t>(b[1]) << 16), b[2] | (static_cast<uint32_t>(b[3]) << 16),
+                        b[4] | (static_cast<uint32_t>(b[5]) << 16), b[6] | (static_cast<uint32_t>(b[7]) << 16));
+    row[1] = make_uint4(b[8], 0u, 0u, 0u);
+}
+
+// The call from price / S, puts by put-call parity, straight into the pinned
+// slot (coalesced).
+__global__ void __launch_bounds__(kFeatRows)
+quote_price_kernel(const double* __restrict__ fix, int64_t n, const float* __restrict__ y,
+                   double* __restrict__ out) {
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * kFeatRows + threadIdx.x;
+    if (i < n) out[i] = fix[i] * static_cast<double>(y[i]) - fix[n + i] + fix[2 * n + i];
 }
 
 // out[r] = sum_j X[r][j] * (w ? w[j] : 1), one warp per row, fixed order.
@@ -296,6 +370,7 @@ SurModel::~SurModel() {
         if (p) cudaFree(p);
     if (perm_) cudaFree(perm_);
     if (state_) cudaFree(state_);
+    if (d_in_) cudaFree(d_in_);
     for (cudaEvent_t& e : ev_)
         if (e) cudaEventDestroy(e);
     for (cudaStream_t& a : aux_)
@@ -360,13 +435,6 @@ cudaError_t SurModel::features_device(const double* f, int64_t n, __nv_bfloat16*
     features_kernel<<<static_cast<unsigned>(blocks), kFeatRows, 0, st ? st : stream_>>>(
         f, n, box_, base_kind_, rows, base);
     return cudaGetLastError();
-}
-
-bool SurModel::in_box(const double* f) const {
-    for (int c = 0; c < kSurIn; ++c) {
-        if (!(f[c] >= box_.lo[c] && f[c] <= box_.hi[c])) return false;
-    }
-    return true;
 }
 
 cudaError_t SurModel::refresh_bf16(cudaStream_t st) {
@@ -612,14 +680,30 @@ cudaError_t SurModel::train(int epochs, int batch, float lr0, uint64_t shuffle_s
     return cudaSuccess;
 }
 
-cudaError_t SurModel::ensure_predict_buffers(int64_t rows) {
-    if (rows <= pred_rows_) return cudaSuccess;
-    QK_TRY(dalloc(&PX_, static_cast<size_t>(rows) * kSurInPad));
+cudaError_t SurModel::ensure_predict_buffers(int64_t rows, size_t in_row) {
+    if (rows > pred_rows_) {
+        pred_rows_ = 0;
+        QK_TRY(dalloc(&PX_, static_cast<size_t>(rows) * kSurInPad));
+        QK_TRY(dalloc(&Py_, static_cast<size_t>(rows)));
+        QK_TRY(dalloc(&Pbase_, static_cast<size_t>(rows)));
+        pred_rows_ = rows;
+    }
+    const size_t bytes = in_row * static_cast<size_t>(rows);
+    if (bytes > d_in_bytes_) {
+        d_in_bytes_ = 0;
+        QK_TRY(dalloc(&d_in_, bytes / sizeof(double) + 1));
+        d_in_bytes_ = bytes;
+    }
+    return cudaSuccess;
+}
+
+// Hidden activations of the layer-by-layer path.
+cudaError_t SurModel::ensure_layered_buffers(int64_t rows) {
+    if (rows <= layered_rows_) return cudaSuccess;
+    layered_rows_ = 0;
     QK_TRY(dalloc(&PH1_, static_cast<size_t>(rows) * kSurHid));
     QK_TRY(dalloc(&PH2_, static_cast<size_t>(rows) * kSurHid));
-    QK_TRY(dalloc(&Py_, static_cast<size_t>(rows)));
-    QK_TRY(dalloc(&Pbase_, static_cast<size_t>(rows)));
-    pred_rows_ = rows;
+    layered_rows_ = rows;
     return cudaSuccess;
 }
 
@@ -647,7 +731,7 @@ cudaError_t SurModel::predict_device(const __nv_bfloat16* x, const float* base, 
         ia.err = &state_->err;
         return launch_mlp_infer(tx, tw1, tw2, tw3, ia, sm_count_, st);
     }
-    QK_TRY(ensure_predict_buffers(std::min<int64_t>(n, kPredChunk)));
+    QK_TRY(ensure_layered_buffers(std::min<int64_t>(n, kPredChunk)));
     for (int64_t off = 0; off < n; off += kPredChunk) {
         const int64_t m = std::min<int64_t>(kPredChunk, n - off);
         CUtensorMap tx, tw1, th1, tw2, th2, tw3;
@@ -673,30 +757,132 @@ cudaError_t SurModel::predict_device(const __nv_bfloat16* x, const float* base, 
     return cudaSuccess;
 }
 
+namespace {
+
+// Two pinned slots of the calling thread (pinning 2 MB takes milliseconds, so
+// a new model's first call must not pay for its own): each holds at most one
+// chunk, a call drains both before it returns, and they go with the thread.
+struct HostStage {
+    PinnedBuf in[2], out[2];
+    cudaEvent_t done[2] = {nullptr, nullptr};
+    cudaError_t ensure(int slot, size_t in_bytes, size_t out_bytes) {
+        QK_TRY(in[slot].ensure(in_bytes));
+        QK_TRY(out[slot].ensure(out_bytes));
+        if (!done[slot]) QK_TRY(cudaEventCreateWithFlags(&done[slot], cudaEventDisableTiming));
+        return cudaSuccess;
+    }
+    ~HostStage() {
+        for (int s = 0; s < 2; ++s) {
+            in[s].release();
+            out[s].release();
+            if (done[s]) cudaEventDestroy(done[s]);
+        }
+    }
+};
+
+HostStage& thread_host_stage(int device) {
+    thread_local std::map<int, std::unique_ptr<HostStage>> stages;
+    auto& p = stages[device];
+    if (!p) p.reset(new HostStage());
+    return *p;
+}
+
+}  // namespace
+
+// Host calls run in chunks of kPredChunk options through two pinned slots: a
+// chunk's inputs are copied into its slot while the GPU works on the chunk
+// before it, and a chunk's results leave its slot when the slot comes up
+// again.  fill(h_in, off, m) copies inputs in, enqueue(h_in, h_out, m) queues
+// the chunk's work on stream_, its results ending in h_out, drain(h_out, off,
+// m) copies them to the caller.
+template <class Fill, class Enqueue, class Drain>
+cudaError_t SurModel::run_chunked(int64_t n, size_t in_row, size_t out_row, const Fill& fill,
+                                  const Enqueue& enqueue, const Drain& drain) {
+    const int64_t chunk = std::min<int64_t>(n, kPredChunk);
+    QK_TRY(ensure_predict_buffers(chunk, in_row));
+    HostStage& stage = thread_host_stage(device_);
+    for (int s = 0; s < (n > chunk ? 2 : 1); ++s)
+        QK_TRY(stage.ensure(s, in_row * static_cast<size_t>(chunk), out_row * static_cast<size_t>(chunk)));
+    struct Pending {
+        int64_t off = 0, m = 0;
+    } pending[2];
+    cudaError_t e = cudaSuccess;
+    auto finish = [&](int s) {
+        if (pending[s].m == 0) return cudaSuccess;
+        const cudaError_t es = cudaEventSynchronize(stage.done[s]);
+        if (es == cudaSuccess) drain(static_cast<const char*>(stage.out[s].p), pending[s].off, pending[s].m);
+        pending[s].m = 0;
+        return es;
+    };
+    int s = 0;
+    for (int64_t off = 0; off < n && e == cudaSuccess; off += chunk, s ^= 1) {
+        e = finish(s);
+        if (e != cudaSuccess) break;
+        const int64_t m = std::min<int64_t>(chunk, n - off);
+        fill(static_cast<char*>(stage.in[s].p), off, m);
+        e = enqueue(static_cast<char*>(stage.in[s].p), static_cast<char*>(stage.out[s].p), m);
+        if (e == cudaSuccess) e = cudaEventRecord(stage.done[s], stream_);
+        if (e == cudaSuccess) pending[s] = {off, m};
+    }
+    for (int k = 0; k < 2; ++k, s ^= 1) {
+        const cudaError_t es = finish(s);
+        if (e == cudaSuccess) e = es;
+    }
+    if (e != cudaSuccess) cudaStreamSynchronize(stream_);  // nothing of the call stays in flight
+    return e;
+}
+
 cudaError_t SurModel::predict(const double* features, int64_t n, double* out) {
     DeviceGuard g(device_);
-    const int64_t chunk = std::min<int64_t>(n, kPredChunk);
-    QK_TRY(ensure_predict_buffers(chunk));
-    std::vector<__nv_bfloat16> rows(static_cast<size_t>(chunk) * kSurInPad);
-    std::vector<float> y(static_cast<size_t>(chunk)), b(static_cast<size_t>(chunk));
-    __nv_bfloat16* xin = PX_;  // the chunk's inputs; predict_device uses PH1_/PH2_
-    cudaError_t e = cudaSuccess;
-    for (int64_t off = 0; off < n && e == cudaSuccess; off += chunk) {
-        const int64_t m = std::min<int64_t>(chunk, n - off);
-        normalise(features + off * kSurIn, m, rows.data());
-        base_host(features + off * kSurIn, m, b.data());
-        e = cudaMemcpyAsync(xin, rows.data(), static_cast<size_t>(m) * kSurInPad * sizeof(__nv_bfloat16),
-                            cudaMemcpyHostToDevice, stream_);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(Pbase_, b.data(), static_cast<size_t>(m) * sizeof(float), cudaMemcpyHostToDevice,
-                                stream_);
-        if (e == cudaSuccess) e = predict_device(xin, Pbase_, m, Py_, stream_);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(y.data(), Py_, static_cast<size_t>(m) * sizeof(float), cudaMemcpyDeviceToHost, stream_);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
-        for (int64_t i = 0; i < m && e == cudaSuccess; ++i) out[off + i] = y[i];
-    }
-    return e;
+    const size_t row = kSurIn * sizeof(double);
+    return run_chunked(
+        n, row, sizeof(float),
+        [&](char* h, int64_t off, int64_t m) {
+            std::memcpy(h, features + off * kSurIn, row * static_cast<size_t>(m));
+        },
+        [&](char* h_in, char* h_out, int64_t m) -> cudaError_t {
+            QK_TRY(cudaMemcpyAsync(d_in_, h_in, row * static_cast<size_t>(m), cudaMemcpyHostToDevice, stream_));
+            QK_TRY(features_device(d_in_, m, PX_, Pbase_, stream_));
+            QK_TRY(predict_device(PX_, Pbase_, m, Py_, stream_));
+            return cudaMemcpyAsync(h_out, Py_, sizeof(float) * static_cast<size_t>(m), cudaMemcpyDeviceToHost,
+                                   stream_);
+        },
+        [&](const char* h, int64_t off, int64_t m) {
+            const float* y = reinterpret_cast<const float*>(h);
+            for (int64_t i = 0; i < m; ++i) out[off + i] = y[i];
+        });
+}
+
+cudaError_t SurModel::price_quotes(const double* const (&cols)[10], const int32_t* option_type,
+                                   int64_t n, double* out, int32_t* route) {
+    DeviceGuard g(device_);
+    const size_t in_row = 10 * sizeof(double) + sizeof(int32_t);
+    const size_t out_row = sizeof(double) + sizeof(int32_t);
+    return run_chunked(
+        n, in_row, out_row,
+        [&](char* h, int64_t off, int64_t m) {
+            for (const double* c : cols) {
+                std::memcpy(h, c + off, sizeof(double) * static_cast<size_t>(m));
+                h += sizeof(double) * static_cast<size_t>(m);
+            }
+            std::memcpy(h, option_type + off, sizeof(int32_t) * static_cast<size_t>(m));
+        },
+        [&](char* h_in, char* h_out, int64_t m) -> cudaError_t {
+            const unsigned blocks = static_cast<unsigned>((m + kFeatRows - 1) / kFeatRows);
+            const double* in = reinterpret_cast<const double*>(h_in);
+            double* price = reinterpret_cast<double*>(h_out);
+            quote_features_kernel<<<blocks, kFeatRows, 0, stream_>>>(
+                in, m, box_, base_kind_, PX_, Pbase_, d_in_, reinterpret_cast<int32_t*>(price + m));
+            QK_TRY(cudaGetLastError());
+            QK_TRY(predict_device(PX_, Pbase_, m, Py_, stream_));
+            quote_price_kernel<<<blocks, kFeatRows, 0, stream_>>>(d_in_, m, Py_, price);
+            return cudaGetLastError();
+        },
+        [&](const char* h, int64_t off, int64_t m) {
+            std::memcpy(out + off, h, sizeof(double) * static_cast<size_t>(m));
+            std::memcpy(route + off, h + sizeof(double) * static_cast<size_t>(m),
+                        sizeof(int32_t) * static_cast<size_t>(m));
+        });
 }
 
 cudaError_t SurModel::gradients(const double* features, const double* target, int n, double* grads,

@@ -72,13 +72,17 @@ public:
     cudaError_t features_device(const double* features, int64_t n, __nv_bfloat16* rows,
                                 float* base, cudaStream_t st);
     int32_t base_kind() const { return base_kind_; }
-    bool in_box(const double* f) const;
 
     cudaError_t set_dataset(const double* features, const double* target, int64_t n);
     cudaError_t train(int epochs, int batch, float lr0, uint64_t shuffle_seed, float* out_loss_last,
                       float* out_epoch_loss);
     // price / spot of calls for raw features, host in and out.
     cudaError_t predict(const double* features, int64_t n, double* out);
+    // The host pricing call: columns spot, strike, t, r, q, v0, kappa, theta,
+    // sigma, rho and option_type, n each.  route[i]: 0 priced by the network,
+    // 1 outside the box (out[i] is NaN), 2 decided by the entry checks.
+    cudaError_t price_quotes(const double* const (&cols)[10], const int32_t* option_type, int64_t n,
+                             double* out, int32_t* route);
     // Device-resident inference on normalised bf16 rows [n][64] plus the
     // rows' base (required when base_kind() != kSurBaseNone): the fused kernel
     // (all three layers per 128-row tile in one persistent launch), or with
@@ -99,7 +103,11 @@ public:
 
 private:
     cudaError_t ensure_batch_buffers(int batch);
-    cudaError_t ensure_predict_buffers(int64_t rows);
+    cudaError_t ensure_predict_buffers(int64_t rows, size_t in_row);
+    cudaError_t ensure_layered_buffers(int64_t rows);
+    template <class Fill, class Enqueue, class Drain>
+    cudaError_t run_chunked(int64_t n, size_t in_row, size_t out_row, const Fill& fill,
+                            const Enqueue& enqueue, const Drain& drain);
     cudaError_t run_step(cudaStream_t st, bool update);
     cudaError_t refresh_bf16(cudaStream_t st);
 
@@ -144,6 +152,10 @@ private:
     __nv_bfloat16 *PX_ = nullptr, *PH1_ = nullptr, *PH2_ = nullptr;
     float* Py_ = nullptr;
     float* Pbase_ = nullptr;
+    // host calls: device room for one chunk's inputs
+    double* d_in_ = nullptr;
+    size_t d_in_bytes_ = 0;
+    int64_t layered_rows_ = 0;
 };
 
 }  // namespace qkb
