@@ -51,6 +51,18 @@ __device__ __forceinline__ float ptx_max_nan(float a, float b) {
     asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
     return y;
 }
+// Three-operand min and max (sm_100), NaN-propagating: one instruction adds two
+// values to a running extreme.
+__device__ __forceinline__ float ptx_min3_nan(float a, float b, float c) {
+    float y;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+}
+__device__ __forceinline__ float ptx_max3_nan(float a, float b, float c) {
+    float y;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+}
 __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
 // Packed FP32 pairs (sm_100 f32x2 FMA / multiply / add: one instruction for

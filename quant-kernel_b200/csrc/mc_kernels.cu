@@ -156,16 +156,27 @@ __device__ __noinline__ Acc terminal_unit(const McOption* __restrict__ rec, uint
 // more independent work per iteration for larger SU (the autotuner's step
 // unrolling).
 // ----------------------------------------------------------------------------
-template <int UPT, bool ANTI, bool MIL, int SU>
-__device__ __forceinline__ void sim_stepwise(const McOption& o, uint32_t unit0, uint32_t stride,
-                                             uint32_t k0, uint32_t k1, Acc& acc) {
+//
+// FLOOR = false leaves the per-step floors out.  They are 2 of a pair-step's 17
+// instructions and almost never bind: a step multiplies s by 1 + inc >= g (from
+// the largest |z| a 23-bit radius gives), so a state of at least fl / g^6 at
+// the start of a block of six cannot meet the floor inside it (the host puts
+// that limit into the record).  The loop
+// checks that once per block (one three-operand min per two states); where it
+// fails for a thread, or meets a NaN, the thread's paths are run again with the
+// floors.  The same bits either way.  (48 options x 100001 paths x 126 steps:
+// Milstein 303 -> 291 us, Euler 292 -> 281; the 4096-option mixed plan 50.8 ->
+// 48.6 ms.  The same on Heston's floor, 1.8 of 37 instructions, ran 1.5%
+// slower: its loop is bound by the special-function unit.)
+template <int UPT, bool ANTI, bool MIL, int SU, bool FLOOR>
+__device__ __forceinline__ bool stepwise_states(const McOption& o, uint32_t unit0, uint32_t stride,
+                                                uint32_t k0, uint32_t k1, float block_min,
+                                                float (&su)[UPT], float (&sd)[UPT]) {
     // Philox6 normals are z / kBmRadius: the vol and Milstein constants take
     // the factor (b z = (b kBmRadius)(z / kBmRadius), likewise c z^2)
     const float m0 = o.p[0], b = o.p[1] * kBmRadius, fl = o.p[2], c = o.p[3] * kBmRadius2;
     const int32_t steps = o.steps;
-    const uint32_t units = (uint32_t)o.units;
     const uint32_t c3 = ANTI ? 0u : 1u;
-    float su[UPT], sd[UPT];
 #pragma unroll
     for (int k = 0; k < UPT; ++k) {
         su[k] = 1.0f;
@@ -187,7 +198,7 @@ __device__ __forceinline__ void sim_stepwise(const McOption& o, uint32_t unit0, 
     // at even s), packed (units 2p, 2p + 1 as one pair) or scalar.
     float2 zp2[NP][2];
     float zp[UPT][2];
-    auto step = [&](const Philox6 (&r)[UPT], int s) {
+    auto step = [&](const Philox6 (&r)[UPT], int s, bool floored) {
         if constexpr (PK) {
 #pragma unroll
             for (int p = 0; p < NP; ++p) {
@@ -202,10 +213,10 @@ __device__ __forceinline__ void sim_stepwise(const McOption& o, uint32_t unit0, 
                     id = fma2(neg2(b2), zz, m02);
                 }
                 const float2 u = fma2(su2[p], iu, su2[p]);
-                su2[p] = f2(fmaxf(u.x, fl), fmaxf(u.y, fl));
+                su2[p] = floored ? f2(fmaxf(u.x, fl), fmaxf(u.y, fl)) : u;
                 if (ANTI) {
                     const float2 d = fma2(sd2[p], id, sd2[p]);
-                    sd2[p] = f2(fmaxf(d.x, fl), fmaxf(d.y, fl));
+                    sd2[p] = floored ? f2(fmaxf(d.x, fl), fmaxf(d.y, fl)) : d;
                 }
             }
         } else {
@@ -221,9 +232,26 @@ __device__ __forceinline__ void sim_stepwise(const McOption& o, uint32_t unit0, 
                     iu = fma_rn(b, zz, m0);
                     id = fma_rn(-b, zz, m0);
                 }
-                su[k] = fmaxf(fma_rn(su[k], iu, su[k]), fl);
-                if (ANTI) sd[k] = fmaxf(fma_rn(sd[k], id, sd[k]), fl);
+                const float u = fma_rn(su[k], iu, su[k]);
+                su[k] = floored ? fmaxf(u, fl) : u;
+                if (ANTI) {
+                    const float d = fma_rn(sd[k], id, sd[k]);
+                    sd[k] = floored ? fmaxf(d, fl) : d;
+                }
             }
+        }
+    };
+    float low = 1.0f;  // smallest state at a block's end
+    auto check = [&]() {
+        if constexpr (PK) {
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                low = ptx_min3_nan(low, su2[p].x, su2[p].y);
+                if (ANTI) low = ptx_min3_nan(low, sd2[p].x, sd2[p].y);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < UPT; ++k) low = ptx_min3_nan(low, su[k], ANTI ? sd[k] : su[k]);
         }
     };
     auto philox_block = [&](Philox6 (&r)[UPT], uint32_t bk) {
@@ -244,10 +272,11 @@ __device__ __forceinline__ void sim_stepwise(const McOption& o, uint32_t unit0, 
 #pragma unroll 2
         for (; j0 < full; j0 += 6, ++blk) {
             Philox6 nx[UPT];
-            step(r, 0);
+            step(r, 0, FLOOR);
             philox_block(nx, blk + 1u);
 #pragma unroll
-            for (int s = 1; s < 6; ++s) step(r, s);
+            for (int s = 1; s < 6; ++s) step(r, s, FLOOR);
+            if (!FLOOR) check();
 #pragma unroll
             for (int k = 0; k < UPT; ++k) r[k] = nx[k];
         }
@@ -255,7 +284,7 @@ __device__ __forceinline__ void sim_stepwise(const McOption& o, uint32_t unit0, 
             const int32_t m = steps - j0;
 #pragma unroll
             for (int s = 0; s < 5; ++s)
-                if (s < m) step(r, s);
+                if (s < m) step(r, s, true);
         }
     } else {
         for (int32_t j0 = 0; j0 < steps; j0 += 6 * SU, blk += SU) {
@@ -268,7 +297,7 @@ __device__ __forceinline__ void sim_stepwise(const McOption& o, uint32_t unit0, 
                 const int32_t m = (steps - j) < 6 ? (steps - j) : 6;
 #pragma unroll
                 for (int s = 0; s < 6; ++s)
-                    if (s < m) step(rb[sb], s);
+                    if (s < m) step(rb[sb], s, true);
             }
         }
     }
@@ -281,6 +310,23 @@ __device__ __forceinline__ void sim_stepwise(const McOption& o, uint32_t unit0, 
             sd[2 * p + 1] = sd2[p].y;
         }
     }
+    return FLOOR || low >= block_min;  // a NaN fails
+}
+
+template <int UPT, bool ANTI, bool MIL, int SU>
+__device__ __forceinline__ void sim_stepwise(const McOption& o, uint32_t unit0, uint32_t stride,
+                                             uint32_t k0, uint32_t k1, Acc& acc) {
+    const uint32_t units = (uint32_t)o.units;
+    float su[UPT], sd[UPT];
+    bool done = false;
+    if constexpr (SU == 1) {
+        const float block_min = o.p[4];  // +inf: no floor-free blocks (stepwise_block_min)
+        if (block_min < 1.0f)
+            done = stepwise_states<UPT, ANTI, MIL, SU, false>(o, unit0, stride, k0, k1, block_min,
+                                                              su, sd);
+    }
+    if (!done)
+        stepwise_states<UPT, ANTI, MIL, SU, true>(o, unit0, stride, k0, k1, 0.0f, su, sd);
     const uint32_t n_pairs = (uint32_t)o.paths >> 1;
 #pragma unroll
     for (int k = 0; k < UPT; ++k) {
@@ -980,11 +1026,21 @@ __device__ __forceinline__ void reduce_tile(Acc acc, TilePartial* __restrict__ o
     __syncthreads();
 }
 
+// The same as a call.  In the Heston grids what surrounds the step loop changes
+// the loop's own schedule: with the reduction and the option search out of
+// line it runs 39.4 ms on 1024 options x 262144 paths x 200 steps, inlined
+// 40.4 (the same instructions, more waits on the special-function queue).
+template <int BLOCK, bool CV>
+__device__ __noinline__ void reduce_tile_call(Acc acc, TilePartial* __restrict__ out, DD* smem) {
+    reduce_tile<BLOCK, CV>(acc, out, smem);
+}
+
 // Option owning `tile`: the last i with tile_begin[i] <= tile (tile_begin is
 // non-decreasing, n + 1 entries, tile_begin[n] = total tiles).  Options of one
 // size, the common batch, have the owner at the proportional place: two loads
-// instead of the search's chain of log2(n).
-__device__ __forceinline__ int32_t find_option(const int64_t* __restrict__ tile_begin, int32_t n,
+// instead of the search's chain of log2(n) (64 options x 262144 paths x 5 Heston
+// steps, with the shorter reduction: 246 -> 226 us).
+__device__ __noinline__ int32_t find_option(const int64_t* __restrict__ tile_begin, int32_t n,
                                                int64_t tile) {
     const int64_t t0 = __ldg(tile_begin), total = __ldg(tile_begin + n) - t0;
     // half a tile in: rounding cannot reach the next option's first tile
@@ -1014,8 +1070,8 @@ __device__ __forceinline__ void sim_family(const McOption& o, uint32_t unit0, ui
 }
 
 // One tile: all UPT * unit_iters units of every thread, then the reduction.
-// `tables` is read by the FP64 families only.
-template <int FAMILY, int BLOCK, int UPT, bool ANTI, int SU = 1>
+// `tables` is read by the FP64 families only; GRID: a single-family grid.
+template <int FAMILY, int BLOCK, int UPT, bool ANTI, int SU = 1, bool GRID = false>
 __device__ __forceinline__ void run_tile(const McOption& o, const McOption* __restrict__ rec,
                                          int64_t tile, TilePartial* partials, DD* smem,
                                          const Fp64Tables* tables) {
@@ -1034,7 +1090,10 @@ __device__ __forceinline__ void run_tile(const McOption& o, const McOption* __re
             sim_family<FAMILY, UPT, ANTI, SU>(o, base + threadIdx.x, (uint32_t)BLOCK, k0, k1, acc);
         }
     }
-    reduce_tile<BLOCK, FAMILY == kFamVr>(acc, partials + tile, smem);
+    if constexpr (GRID && (FAMILY == kFamHeston || FAMILY == kFamHestonLr))
+        reduce_tile_call<BLOCK, false>(acc, partials + tile, smem);
+    else
+        reduce_tile<BLOCK, FAMILY == kFamVr>(acc, partials + tile, smem);
 }
 
 // ----------------------------------------------------------------------------
@@ -1049,11 +1108,16 @@ __device__ __forceinline__ void run_tile(const McOption& o, const McOption* __re
 // independent paths fill the FP64 pipe's latency with 24 warps as well as
 // with 32 (64 registers, a few spills) or 20 (within 2% on the 64-option
 // batches).
-template <int FAMILY, int BLOCK>
-constexpr int kMinCtas = kIsFp64<FAMILY> ? 6 * 128 / BLOCK : 0;
+// Euler at four units per thread is held to 64 registers (eight CTAs of 128):
+// left alone its two loops took 106 and ran 292 us on 48 options x 100001
+// paths x 126 steps, 281 at 64 (282 at 72; Milstein, 80 registers by itself,
+// ran 291 and slower at 72 and 64).
+template <int FAMILY, int BLOCK, int UPT, int SU>
+constexpr int kMinCtas = kIsFp64<FAMILY> ? 6 * 128 / BLOCK
+                       : FAMILY == kFamEuler && UPT == 4 && SU == 1 ? 8 * 128 / BLOCK : 0;
 
 template <int FAMILY, int BLOCK, int UPT, bool ANTI, int SU>
-__global__ void __launch_bounds__(BLOCK, kMinCtas<FAMILY, BLOCK>)
+__global__ void __launch_bounds__(BLOCK, kMinCtas<FAMILY, BLOCK, UPT, SU>)
     mc_simulate_kernel(const McOption* __restrict__ opts, const int64_t* __restrict__ tile_begin,
                        int32_t n, int64_t tile0, int64_t n_tiles, TilePartial* __restrict__ partials) {
     __shared__ DD smem[5 * (BLOCK / 32)];
@@ -1068,7 +1132,7 @@ __global__ void __launch_bounds__(BLOCK, kMinCtas<FAMILY, BLOCK>)
         const int64_t tile = tile0 + t;  // tile_begin holds absolute tile indices
         const int32_t oi = find_option(tile_begin, n, tile);
         const McOption o = opts[oi];
-        run_tile<FAMILY, BLOCK, UPT, ANTI, SU>(o, opts + oi, tile, partials, smem, tables);
+        run_tile<FAMILY, BLOCK, UPT, ANTI, SU, true>(o, opts + oi, tile, partials, smem, tables);
     }
 }
 

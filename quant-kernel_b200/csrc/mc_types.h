@@ -41,6 +41,7 @@ enum : int32_t { kModeSimulate = 0, kModeConstant = 1 };
 //                      p2 = 1e-12 / spot (floor of S/spot)
 //   Milstein (3):      p0 = (r - q) dt - c           p1 = vol sqrt(dt)
 //                      p2 = 1e-12 / spot             p3 = c = vol^2 dt / 2
+//   both one-factor:   p4 = S/spot above which six steps cannot reach p2
 //   Heston (6):        p0 = (r - q) dt   p1 = dt/2   p2 = sqrt(dt)
 //                      p3 = kappa dt     p4 = kappa theta dt
 //                      p5 = sigma sqrt(dt)           p6 = rho
