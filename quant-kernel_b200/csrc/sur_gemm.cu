@@ -162,21 +162,6 @@ __device__ __forceinline__ void store_bf16x32(__nv_bfloat16* dst, const float (&
     }
 }
 
-__device__ __forceinline__ void load_bf16x32(const __nv_bfloat16* src, float (&v)[32]) {
-    const uint4* s = reinterpret_cast<const uint4*>(src);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        uint4 u = s[q];
-        const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            float2 f = __bfloat1622float2(p[j]);
-            v[q * 8 + 2 * j] = f.x;
-            v[q * 8 + 2 * j + 1] = f.y;
-        }
-    }
-}
-
 // Eight epilogue warps: warp w reads TMEM lanes 32 (w % 4) .. + 31 (its tile
 // rows) and the column half w / 4 of the tile (chunks of 32 columns
 // [c_lo, c_hi)); every element's arithmetic is the same as with one warp per
@@ -208,41 +193,12 @@ __device__ __forceinline__ void epilogue(const GemmArgs& a, uint32_t tmem, int m
         for (int c = c_lo; c < c_hi; ++c) {
             tmem_ld32(tbase + c * 32, v);
             const int col0 = n0 + c * 32;
-            float z[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
                 float hz, t;
                 v[j] = silu_from_acc(v[j], 0.5f * __ldg(a.bias + col0 + j), hz, t);
-                z[j] = 2.0f * hz;  // exact: the pre-activation acc + bias
             }
-            if (live) {
-                if (a.z_out) store_bf16x32(a.z_out + static_cast<size_t>(row) * a.N + col0, z);
-                if (a.h_out) store_bf16x32(a.h_out + static_cast<size_t>(row) * a.N + col0, v);
-                if (a.t_out) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        a.t_out[static_cast<size_t>(col0 + j) * a.ldt + row] = __float2bfloat16_rn(v[j]);
-                }
-            }
-        }
-    } else if (EPI == kEpiBwd) {
-#pragma unroll 1
-        for (int c = c_lo; c < c_hi; ++c) {
-            tmem_ld32(tbase + c * 32, v);
-            const int col0 = n0 + c * 32;
-            if (live) {
-                float z[32];
-                load_bf16x32(a.z_in + static_cast<size_t>(row) * a.N + col0, z);
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const float s = sigmoidf_(z[j]);
-                    v[j] = v[j] * s * (1.0f + z[j] * (1.0f - s));
-                }
-                store_bf16x32(a.d_out + static_cast<size_t>(row) * a.N + col0, v);
-#pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    a.dt_out[static_cast<size_t>(col0 + j) * a.ldt + row] = __float2bfloat16_rn(v[j]);
-            }
+            if (live) store_bf16x32(a.h_out + static_cast<size_t>(row) * a.N + col0, v);
         }
     } else {  // kEpiLast: BN == N (the whole hidden row is in this CTA)
         // head dot product as four partial sums, group g over the columns
@@ -274,31 +230,6 @@ __device__ __forceinline__ void epilogue(const GemmArgs& a, uint32_t tmem, int m
         float y = ((part_s[0][r] + part_s[1][r]) + part_s[2][r]) + part_s[3][r];
         y += __ldg(a.b4);
         if (live && half == 0) a.y_out[row] = a.base ? y + __ldg(a.base + row) : y;
-        if (a.target != nullptr) {
-            const float dy = live ? a.loss_scale * (y - a.target[row]) : 0.0f;
-            if (live && half == 0) a.dy_out[row] = dy;
-#pragma unroll 1
-            for (int c = c_lo; c < c_hi; ++c) {
-                tmem_ld32(tbase + c * 32, v);
-                const int col0 = c * 32;
-                float h[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    float hz, t;
-                    h[j] = silu_from_acc(v[j], 0.5f * __ldg(a.bias + col0 + j), hz, t);
-                    const float z = 2.0f * hz, s = fmaf(0.5f, t, 0.5f);
-                    v[j] = dy * __ldg(a.w4 + col0 + j) * s * (1.0f + z * (1.0f - s));
-                }
-                if (live) {
-                    store_bf16x32(a.d_out + static_cast<size_t>(row) * a.N + col0, v);
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        a.dt_out[static_cast<size_t>(col0 + j) * a.ldt + row] = __float2bfloat16_rn(v[j]);
-                        a.t_out[static_cast<size_t>(col0 + j) * a.ldt + row] = __float2bfloat16_rn(h[j]);
-                    }
-                }
-            }
-        }
     }
 }
 
@@ -807,6 +738,471 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     }
 }
 
+// ----------------------------------------------------------------------------
+// Fused training pass: one CTA takes 128 rows of the minibatch through the
+// gather, the three layers, the head, the backward layers and the three weight
+// gradients of its rows (one split-K slab each), in one launch.  The slabs,
+// dZ, H3 and dy go to global memory for the update kernel, which sums them in a
+// fixed order.
+//
+// A step was 14 launches of 6-22 us, each reading back what the one before it
+// had written and its transpose; here the activations stay in shared memory
+// and serve twice: as the K-major A operand of the next layer (row = M), and
+// untransposed as the MN-major operands of the weight gradients (row = K),
+// which the 128-byte-swizzled layout [64-column block][row][64 columns] is as
+// it stands.  Batch 8192 runs 64 CTAs, each a chain of ten short MMA jobs and
+// as many epilogues: latency bounds it, not a pipe.
+//
+// Global arrays of the pass are laid out by chunk, [tile][16-byte chunk of a
+// row][128 rows], so that a warp's stores (one row per lane) are contiguous:
+// as rows they touched 32 lines each, and the stores were half of the kernel.
+//
+// Shared memory: P and Q (64 KiB each) hold H1, H2; then D3 in P and D2, H1
+// (read back from this thread's own global copy), D1 as their readers
+// complete; a 2-slot ring of 32 KiB weight blocks; X (128 x 16) and W1 (256 x
+// 16).  TMEM: accumulator 0 for the layers, accumulator 1 for the weight
+// gradients (256 columns each).  Roles: warp 16 streams weights, warp 17
+// issues MMAs, warps 0-15 gather and run the epilogues (the lane and column
+// split of mlp_infer_kernel).  Job j's completion arrives on full[j],
+// epilogue e's on done[e]; each is used once, and every wait is bounded.
+//
+//   job  MMA                              epilogue
+//   0    X W1^T          -> acc0          0  z1, h1 -> P
+//   1    P W2^T          -> acc0          1  z2, h2 -> Q
+//   2    Q W3^T          -> acc0          2  head, dy, dz3 -> P
+//   3    dW3 rows 0-127  -> acc1          3  slab out
+//   4    P W3            -> acc0
+//   5    dW3 rows 128-   -> acc1          4  (4 and 5 done) dz2 -> Q, h1 -> P
+//   6    Q W2            -> acc0          5  slab out
+//   7    dW2 rows 0-127  -> acc1          6  slab out
+//   8    dW2 rows 128-   -> acc1          7  (6 and 8 done) dz1 -> Q
+//   9    dW1             -> acc0          8  slabs out
+// ----------------------------------------------------------------------------
+constexpr int kTrainEpiWarps = 16;
+constexpr int kTrainThreads = (kTrainEpiWarps + 2) * 32;
+constexpr int kTrainJobs = 10, kTrainDone = 8;
+constexpr size_t kTrainSmem = 2 * kHBytes + kIWSlots * kWBlock + kW1Bytes + kXBytes + 1024;
+
+// MN-major shared-memory descriptors: rows of 128 (32) swizzled bytes along
+// MN, one per k; 8-row groups SBO apart, blocks of 64 (16) columns LBO apart.
+__device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t addr) {
+    return static_cast<uint64_t>((addr >> 4) & 0x3FFFu) |
+           (static_cast<uint64_t>(kABytes >> 4) << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) |
+           (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(2) << 61);
+}
+__device__ __forceinline__ uint64_t desc_mn_sw32(uint32_t addr) {
+    return static_cast<uint64_t>((addr >> 4) & 0x3FFFu) | (static_cast<uint64_t>(1) << 16) |
+           (static_cast<uint64_t>(256 >> 4) << 32) | (static_cast<uint64_t>(1) << 46) |
+           (static_cast<uint64_t>(6) << 61);
+}
+constexpr uint32_t kIdescMn = (1u << 15) | (1u << 16);  // A and B MN-major
+
+// Sixteen values as two 16-byte chunks, `stride` chunks apart.
+__device__ __forceinline__ void store16_bf16(uint4* d, int stride, const float (&v)[16]) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        __nv_bfloat162 p[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p[j] = __floats2bfloat162_rn(v[q * 8 + 2 * j], v[q * 8 + 2 * j + 1]);
+        d[q * stride] = *reinterpret_cast<uint4*>(p);
+    }
+}
+__device__ __forceinline__ void load16_bf16(const uint4* s, int stride, float (&v)[16]) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const uint4 u = s[q * stride];
+        const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float2 f = __bfloat1622float2(p[j]);
+            v[q * 8 + 2 * j] = f.x;
+            v[q * 8 + 2 * j + 1] = f.y;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kTrainThreads, 1)
+    mlp_train_kernel(const __grid_constant__ TrainMaps maps, const TrainArgs a) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                               ~static_cast<uintptr_t>(1023));
+    uint8_t* bufp = smem;
+    uint8_t* bufq = smem + kHBytes;
+    uint8_t* wbuf = smem + 2 * kHBytes;
+    uint8_t* w1s = wbuf + kIWSlots * kWBlock;
+    uint8_t* xs = w1s + kW1Bytes;
+    __shared__ __align__(8) uint64_t w1full, xready, pready, drain;
+    __shared__ __align__(8) uint64_t full[kTrainJobs], done[kTrainDone];
+    __shared__ __align__(8) uint64_t wfull[kIWSlots], wempty[kIWSlots];
+    __shared__ __align__(16) float sb1[kSurHidden], sb2[kSurHidden], sb3[kSurHidden], sw4[kSurHidden];
+    __shared__ float part[4][kBM];
+    __shared__ float starget[kBM];
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile int abort_flag;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tile = blockIdx.x;
+    if (tid < kSurHidden) {
+        sb1[tid] = 0.5f * a.b1[tid];  // halved biases for silu_from_acc (exact)
+        sb2[tid] = 0.5f * a.b2[tid];
+        sb3[tid] = 0.5f * a.b3[tid];
+        sw4[tid] = a.w4[tid];
+    }
+    if (tid == 0) {
+        mbar_init(smem_u32(&w1full), 1);
+        mbar_init(smem_u32(&xready), kTrainEpiWarps);
+        mbar_init(smem_u32(&pready), kTrainEpiWarps);
+        mbar_init(smem_u32(&drain), 1);
+        for (int j = 0; j < kTrainJobs; ++j) mbar_init(smem_u32(&full[j]), 1);
+        for (int e = 0; e < kTrainDone; ++e) mbar_init(smem_u32(&done[e]), kTrainEpiWarps);
+        for (int s = 0; s < kIWSlots; ++s) {
+            mbar_init(smem_u32(&wfull[s]), 1);
+            mbar_init(smem_u32(&wempty[s]), 1);
+        }
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32(&tmem_slot)),
+                     "r"(512u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = tmem_slot;
+    auto fail = [&](int code) {
+        abort_flag = 1;
+        atomicExch(a.err, code);
+    };
+    int last_round[kIWSlots] = {-1, -1};
+    bool w1_issued = false;
+
+    if (warp == kTrainEpiWarps) {
+        if (lane == 0) {
+            mbar_expect_tx(smem_u32(&w1full), kW1Bytes);
+            tma_load_2d(smem_u32(w1s), &maps.w1, 0, 0, smem_u32(&w1full));
+            w1_issued = true;
+            const CUtensorMap* order[4] = {&maps.w2, &maps.w3, &maps.w3t, &maps.w2t};
+            bool ok = true;
+            for (uint32_t wl = 0; ok && wl < 16; ++wl) {
+                const uint32_t s = wl % kIWSlots, round = wl / kIWSlots;
+                if (abort_flag) break;
+                if (round > 0) ok = mbar_wait(smem_u32(&wempty[s]), (round - 1) & 1);
+                if (!ok) {
+                    fail(32);
+                    break;
+                }
+                mbar_expect_tx(smem_u32(&wfull[s]), kWBlock);
+                tma_load_2d(smem_u32(wbuf + s * kWBlock), order[wl >> 2],
+                            static_cast<int>(wl & 3) * kBK, 0, smem_u32(&wfull[s]));
+                last_round[s] = static_cast<int>(round);
+            }
+        }
+    } else if (warp == kTrainEpiWarps + 1) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = idesc_bf16<256>(), idesc_mn = idesc | kIdescMn;
+            constexpr uint32_t idesc_w1 = idesc_bf16<16>() | kIdescMn;
+            const uint32_t acc0 = tmem, acc1 = tmem + 256;
+            uint32_t wc = 0;
+            bool ok = true;
+            auto wait = [&](uint64_t* bar) {
+                ok = ok && !abort_flag && mbar_wait(smem_u32(bar), 0);
+                fence_after();
+            };
+            auto commit = [&](int j) {
+                if (ok) umma_commit(smem_u32(&full[j]));
+            };
+            // a layer: buf [128 x 256] times the next four ring blocks
+            auto layer = [&](const uint8_t* buf) {
+                for (int kb = 0; ok && kb < 4; ++kb) {
+                    const uint32_t s = wc % kIWSlots;
+                    ok = mbar_wait(smem_u32(&wfull[s]), (wc / kIWSlots) & 1);
+                    if (!ok) return;
+                    fence_after();
+                    const uint32_t sa = smem_u32(buf + kb * kABytes), sb = smem_u32(wbuf + s * kWBlock);
+#pragma unroll
+                    for (int kk = 0; kk < kBK / 16; ++kk)
+                        umma_bf16(acc0, desc_sw128(sa + kk * 32), desc_sw128(sb + kk * 32), idesc,
+                                  (kb | kk) != 0 ? 1u : 0u);
+                    umma_commit(smem_u32(&wempty[s]));
+                    ++wc;
+                }
+            };
+            // 128 rows of a weight gradient: D's columns 128 half .. + 127 by
+            // H's 256 columns, over the CTA's 128 batch rows
+            auto grad = [&](const uint8_t* d, int half, const uint8_t* h) {
+                if (!ok) return;
+                const uint32_t da = smem_u32(d + half * 2 * kABytes), hb = smem_u32(h);
+#pragma unroll
+                for (int k = 0; k < kBM / 16; ++k)
+                    umma_bf16(acc1, desc_mn_sw128(da + k * 2048), desc_mn_sw128(hb + k * 2048),
+                              idesc_mn, k != 0 ? 1u : 0u);
+            };
+            wait(&w1full);
+            wait(&xready);
+            if (ok) umma_bf16(acc0, desc_sw32(smem_u32(xs)), desc_sw32(smem_u32(w1s)), idesc, 0u);
+            commit(0);
+            wait(&done[0]);
+            layer(bufp);
+            commit(1);
+            wait(&done[1]);
+            layer(bufq);
+            commit(2);
+            wait(&done[2]);
+            grad(bufp, 0, bufq);
+            commit(3);
+            layer(bufp);
+            commit(4);
+            wait(&done[3]);
+            grad(bufp, 1, bufq);
+            commit(5);
+            wait(&done[4]);
+            layer(bufq);
+            commit(6);
+            wait(&done[5]);
+            grad(bufq, 0, bufp);
+            commit(7);
+            wait(&done[6]);
+            grad(bufq, 1, bufp);
+            commit(8);
+            wait(&done[7]);
+            for (int half = 0; ok && half < 2; ++half) {
+                const uint32_t da = smem_u32(bufq + half * 2 * kABytes), xb = smem_u32(xs);
+#pragma unroll
+                for (int k = 0; k < kBM / 16; ++k)
+                    umma_bf16(acc0 + half * 16, desc_mn_sw128(da + k * 2048),
+                              desc_mn_sw32(xb + k * 512), idesc_w1, k != 0 ? 1u : 0u);
+            }
+            commit(9);
+            if (!ok) fail(34);
+        }
+    } else {
+        const int q = warp & 3, g = warp >> 2;
+        const int r = q * 32 + lane;
+        const size_t row = static_cast<size_t>(tile) * kBM + r;
+        const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
+        const uint32_t acc0 = tmem + lane_off, acc1 = tmem + 256 + lane_off;
+        bool ok = true;
+        // lane 0 polls and broadcasts; then every lane observes the phase itself
+        auto wait = [&](uint64_t* bar) {
+            if (!ok) return;
+            bool got = false;
+            if (lane == 0) got = mbar_wait(smem_u32(bar), 0);
+            got = __shfl_sync(0xFFFFFFFFu, got ? 1 : 0, 0) != 0;
+            if (got) got = __all_sync(0xFFFFFFFFu, mbar_try(smem_u32(bar), 0)) != 0;
+            if (!got && lane == 0) fail(36);
+            ok = got;
+            fence_after();
+        };
+        // shared stores to the tensor core's proxy, TMEM reads before the hand-off
+        auto arrive = [&](uint64_t* bar) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(bar));
+        };
+        auto col = [&](int kb) { return kb * 64 + g * 16; };
+        // this thread's 16 columns of block kb of an accumulator
+        auto acc16 = [&](uint32_t acc, int c, float (&v)[16]) {
+            uint32_t u[16];
+            tmem_ld16_async(acc + c, u);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(u[j]);
+        };
+        // [tile][half][chunk of 4 columns][128 rows]
+        auto slab_out = [&](uint32_t acc, float4* slab, int half) {
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb) {
+                float v[16];
+                acc16(acc, col(kb), v);
+                float4* d = slab + (static_cast<size_t>(tile * 2 + half) * 64 + (col(kb) >> 2)) * kBM + r;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    d[i * kBM] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            }
+        };
+        // this thread's two 8-column chunks of block kb
+        auto chunk = [&](uint4* x, int kb) {
+            return x + (static_cast<size_t>(tile) * 32 + (col(kb) >> 3)) * kBM + r;
+        };
+        // a hidden layer's backward epilogue: acc0 and the stored z -> dz in buf
+        auto backward = [&](uint4* z_in, uint8_t* buf, uint4* d_out) {
+#pragma unroll 1
+            for (int kb = 0; kb < 4; ++kb) {
+                const int c = col(kb);
+                float v[16], z[16];
+                load16_bf16(chunk(z_in, kb), kBM, z);
+                acc16(acc0, c, v);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const float s = sigmoidf_(z[j]);
+                    v[j] = v[j] * s * (1.0f + z[j] * (1.0f - s));
+                }
+                store_h16_sw128(buf, r, c, v);
+                store16_bf16(chunk(d_out, kb), kBM, v);
+            }
+        };
+
+        // gather the tile's rows (first 16 columns, 32-byte swizzle) and targets
+        if (tid < 2 * kBM) {
+            const int i = tid >> 1, ch = tid & 1;
+            const int64_t at = static_cast<int64_t>(*a.step % *a.steps_per_epoch) * a.batch +
+                               static_cast<int64_t>(tile) * kBM + i;
+            const int64_t src = a.perm[at];
+            const uint4 x = *reinterpret_cast<const uint4*>(a.xall + src * a.x_stride + ch * 8);
+            *reinterpret_cast<uint4*>(xs + i * 32 + ((ch ^ ((i >> 2) & 1)) << 4)) = x;
+            if (ch == 0) {
+                const float t = a.tall[src];
+                starget[i] = t;
+                a.target_out[static_cast<size_t>(tile) * kBM + i] = t;
+            }
+        }
+        arrive(&xready);
+
+        // layers 1 and 2 forward
+#pragma unroll 1
+        for (int l = 0; l < 2; ++l) {
+            wait(&full[l]);
+            if (!ok) break;
+            const float* bias = l == 0 ? sb1 : sb2;
+            uint4* z_out = l == 0 ? a.z1 : a.z2;
+            uint8_t* buf = l == 0 ? bufp : bufq;
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb) {
+                const int c = col(kb);
+                float v[16], z[16];
+                acc16(acc0, c, v);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    float hz, t;
+                    v[j] = silu_from_acc(v[j], bias[c + j], hz, t);
+                    z[j] = 2.0f * hz;  // exact: the pre-activation acc + bias
+                }
+                store_h16_sw128(buf, r, c, v);
+                store16_bf16(chunk(z_out, kb), kBM, z);
+                if (l == 0) store16_bf16(chunk(a.h1, kb), kBM, v);
+            }
+            arrive(&done[l]);
+        }
+        // head: partial chains per column group, y, dy; then dz3
+        wait(&full[2]);
+        if (ok) {
+            float p = 0.0f;
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb) {
+                const int c = col(kb);
+                float v[16];
+                acc16(acc0, c, v);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    float hz, t;
+                    const float h = silu_from_acc(v[j], sb3[c + j], hz, t);
+                    p = fmaf(h, sw4[c + j], p);
+                }
+            }
+            part[g][r] = p;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&pready));
+            wait(&pready);
+        }
+        if (ok) {
+            const float y = (((part[0][r] + part[1][r]) + part[2][r]) + part[3][r]) + __ldg(a.b4);
+            const float dy = a.loss_scale * (y - starget[r]);
+            if (g == 0) {
+                a.y_out[row] = y;
+                a.dy_out[row] = dy;
+            }
+#pragma unroll 1
+            for (int kb = 0; kb < 4; ++kb) {
+                const int c = col(kb);
+                float v[16], h[16];
+                acc16(acc0, c, v);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    float hz, t;
+                    h[j] = silu_from_acc(v[j], sb3[c + j], hz, t);
+                    const float z = 2.0f * hz, s = fmaf(0.5f, t, 0.5f);
+                    v[j] = dy * sw4[c + j] * s * (1.0f + z * (1.0f - s));
+                }
+                store_h16_sw128(bufp, r, c, v);
+                store16_bf16(chunk(a.dz3, kb), kBM, v);
+                store16_bf16(chunk(a.h3, kb), kBM, h);
+            }
+            arrive(&done[2]);
+        }
+        wait(&full[3]);
+        if (ok) {
+            slab_out(acc1, a.dw3, 0);
+            arrive(&done[3]);
+        }
+        wait(&full[4]);
+        wait(&full[5]);
+        if (ok) {
+            backward(a.z2, bufq, a.dz2);
+            // this thread's own copy of H1, back into P
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb) {
+                const int c = col(kb);
+                const uint4* src = chunk(a.h1, kb);
+                uint8_t* d = bufp + (c >> 6) * kABytes + r * 128;
+                const int c0 = (c & 63) >> 3;
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    *reinterpret_cast<uint4*>(d + (((c0 + i) ^ (r & 7)) << 4)) = src[i * kBM];
+            }
+            arrive(&done[4]);
+            slab_out(acc1, a.dw3, 1);
+            arrive(&done[5]);
+        }
+        wait(&full[7]);
+        if (ok) {
+            slab_out(acc1, a.dw2, 0);
+            arrive(&done[6]);
+        }
+        wait(&full[6]);
+        wait(&full[8]);
+        if (ok) {
+            backward(a.z1, bufq, a.dz1);
+            arrive(&done[7]);
+            slab_out(acc1, a.dw2, 1);
+        }
+        wait(&full[9]);
+        if (ok && g < 2) {  // group g takes rows 128 g .. of dW1, 16 columns
+            float v[16];
+            acc16(acc0, g * 16, v);
+            float4* d = a.dw1 + static_cast<size_t>(tile * 2 + g) * 4 * kBM + r;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                d[i * kBM] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
+    }
+
+    // Teardown, as in mlp_infer_kernel.
+    fence_before();
+    __syncthreads();
+    if (abort_flag) {
+        if (warp == kTrainEpiWarps && lane == 0) {
+            for (int s = 0; s < kIWSlots; ++s)
+                if (last_round[s] >= 0) mbar_wait(smem_u32(&wfull[s]), last_round[s] & 1);
+            if (w1_issued) mbar_wait(smem_u32(&w1full), 0u);
+        } else if (warp == kTrainEpiWarps + 1 && lane == 0) {
+            umma_commit(smem_u32(&drain));
+            mbar_wait(smem_u32(&drain), 0);
+        }
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u)
+                     : "memory");
+    }
+}
+
 template <int BN, int EPI>
 cudaError_t launch_t(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& a, int splits,
                      cudaStream_t st) {
@@ -838,6 +1234,19 @@ cudaError_t launch_mlp_infer(const CUtensorMap& tx, const CUtensorMap& tw1, cons
     const int64_t tiles = (a.n + kBM - 1) / kBM;
     const int grid = static_cast<int>(tiles < ctas ? tiles : ctas);
     mlp_infer_kernel<<<grid, kInferThreads, kInferSmem, st>>>(tx, tw1, tw2, tw3, a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_mlp_train(const TrainMaps& maps, const TrainArgs& a, cudaStream_t st) {
+    static std::once_flag once;
+    static cudaError_t attr_err = cudaSuccess;
+    std::call_once(once, [] {
+        attr_err = cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(kTrainSmem));
+    });
+    if (attr_err != cudaSuccess) return attr_err;
+    if (a.batch <= 0 || a.batch % kBM != 0) return cudaErrorInvalidValue;
+    mlp_train_kernel<<<a.batch / kBM, kTrainThreads, kTrainSmem, st>>>(maps, a);
     return cudaGetLastError();
 }
 
@@ -901,13 +1310,11 @@ cudaError_t launch_umma_gemm(int epi, int bn, const CUtensorMap& ta, const CUten
         case 128:
             if (epi == kEpiF32) return launch_t<128, kEpiF32>(ta, tb, a, splits, st);
             if (epi == kEpiFwd) return launch_t<128, kEpiFwd>(ta, tb, a, splits, st);
-            if (epi == kEpiBwd) return launch_t<128, kEpiBwd>(ta, tb, a, splits, st);
             break;
         case 256:
             if (epi == kEpiF32) return launch_t<256, kEpiF32>(ta, tb, a, splits, st);
             if (epi == kEpiFwd) return launch_t<256, kEpiFwd>(ta, tb, a, splits, st);
             if (epi == kEpiLast) return launch_t<256, kEpiLast>(ta, tb, a, splits, st);
-            if (epi == kEpiBwd) return launch_t<256, kEpiBwd>(ta, tb, a, splits, st);
             break;
         default:
             break;

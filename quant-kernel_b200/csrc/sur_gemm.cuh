@@ -24,32 +24,22 @@ namespace qkb {
 
 enum : int {
     kEpiF32 = 0,    // C fp32 (split-K partial slab per blockIdx.z)
-    kEpiFwd = 1,    // z = acc + bias; h = silu(z): write Z, H (bf16) and H^T
-    kEpiLast = 2,   // layer 3 + head: y = silu(acc + b3) . w4 + b4; training: dZ3, dZ3^T, H3^T
-    kEpiBwd = 3,    // dz = acc * silu'(z_in): write dZ and dZ^T
+    kEpiFwd = 1,    // h = silu(acc + bias): write H (bf16)
+    kEpiLast = 2,   // layer 3 + head: y = silu(acc + b3) . w4 + b4
 };
 
 struct GemmArgs {
     int M, N, K;             // problem size (K range split over gridDim.z)
     int k_per_split;         // multiple of 64
-    // epilogue operands (bf16 outputs are row-major [M][N]; "t" outputs [N][ldt])
+    // epilogue operands
     float* c_f32;            // kEpiF32: [gridDim.z][M][N]
     const float* bias;       // [N]
-    __nv_bfloat16* z_out;
-    __nv_bfloat16* h_out;
-    __nv_bfloat16* t_out;    // transposed output, row stride ldt
-    int ldt;
-    const __nv_bfloat16* z_in;   // kEpiBwd: pre-activation [M][N]
-    __nv_bfloat16* d_out;        // kEpiLast (training) / kEpiBwd: dZ [M][N]
-    __nv_bfloat16* dt_out;       // dZ^T [N][ldt]
-    const float* w4;             // head weights [N]
-    const float* b4;             // head bias [1]
-    const float* target;         // [M] (training) or null (inference)
-    float* y_out;                // [M]
-    const float* base;           // [M] added to y_out (inference), or null
-    float* dy_out;               // [M] dL/dy (training)
-    float loss_scale;            // dL/dy = loss_scale * (y - target)
-    int* err;                    // error word (0 = ok)
+    __nv_bfloat16* h_out;    // [M][N]
+    const float* w4;         // head weights [N]
+    const float* b4;         // head bias [1]
+    float* y_out;            // [M]
+    const float* base;       // [M] added to y_out, or null
+    int* err;                // error word (0 = ok)
 };
 
 // Fused MLP inference: y[i] = w4 . silu(W3 silu(W2 silu(W1 x_i + b1) + b2) + b3) + b4
@@ -72,6 +62,35 @@ struct InferArgs {
 // ctas: persistent grid size (one CTA per SM).
 cudaError_t launch_mlp_infer(const CUtensorMap& tx, const CUtensorMap& tw1, const CUtensorMap& tw2,
                              const CUtensorMap& tw3, const InferArgs& a, int ctas, cudaStream_t st);
+
+// Fused training pass over one minibatch (mlp_train_kernel in sur_gemm.cu):
+// rows perm[(step % steps_per_epoch) batch + i] of xall, forward, head, loss
+// gradient, backward, and one slab of each weight gradient per 128 rows.
+struct TrainMaps {
+    CUtensorMap w1;            // W1 [256][64], first 16 columns, box 16 x 256
+    CUtensorMap w2, w3;        // [256][256], boxes 64 x 256
+    CUtensorMap w3t, w2t;      // their transposes
+};
+struct TrainArgs {
+    const __nv_bfloat16* xall;  // rows of x_stride bf16, first 16 read
+    int x_stride;
+    const float* tall;
+    const int32_t* perm;
+    const int* step;
+    const int* steps_per_epoch;
+    int batch;                  // multiple of 128
+    float loss_scale;           // dL/dy = loss_scale (y - target)
+    const float *b1, *b2, *b3, *w4, *b4;
+    // bf16 [batch / 128 tiles][32 chunks of 8 columns][128 rows]
+    uint4 *z1, *z2, *h1;        // this pass's scratch
+    uint4 *h3, *dz3, *dz2, *dz1;
+    float *y_out, *dy_out, *target_out;  // [batch]
+    // slabs [tile][2 halves of 128 rows][chunks of 4 columns][128 rows]: 4
+    // chunks (the first 16 columns of W1), 64, 64
+    float4 *dw1, *dw2, *dw3;
+    int* err;                   // error word (0 = ok)
+};
+cudaError_t launch_mlp_train(const TrainMaps& maps, const TrainArgs& a, cudaStream_t st);
 
 // Host side: tensor maps over bf16 row-major [rows][cols] (cols contiguous).
 bool make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,

@@ -1,20 +1,12 @@
 // sur_mlp.cu -- training and inference of the Heston price surrogate.
 //
-// One optimiser step on a minibatch of B rows (B % 128 == 0) is 14 launches,
-// captured once into a CUDA graph and replayed:
-//   gather      minibatch rows (a permutation drawn per epoch) -> X, X^T, target
-//   fwd1/fwd2   tcgen05 GEMM, epilogue z = acc + b, h = silu(z) -> Z, H, H^T
-//   fwd3        tcgen05 GEMM, epilogue: y = silu(acc + b3) . w4 + b4,
-//               dy = 2 (y - t) / B, dZ3 = dy w4 silu'(z3) -> dZ3, dZ3^T, H3^T
-//   loss        db4 = sum dy, loss = mean (y - t)^2          (fixed order)
-//   rowsum      db3 = sum_b dZ3^T, dw4 = H3^T . dy           (fixed order)
-//   bwd2/bwd1   tcgen05 GEMM dH = dZ . W, epilogue dZ = dH silu'(z) -> dZ, dZ^T
-//   dW3/dW2/dW1 tcgen05 GEMM dZ^T . H over the batch, split-K slabs
-//   rowsum      db2, db1
-//   adam        sum slabs (fixed order), Adam with cosine-decayed lr, write the
-//               FP32 master, and the bf16 weights and transposed weights the
-//               next step's GEMMs read
-//   advance     step += 1
+// One optimiser step on a minibatch of B rows (B % 128 == 0) is two launches:
+//   mlp_train_kernel  (sur_gemm.cu) gather, forward, head, loss gradient,
+//                     backward, and each 128 rows' slab of the weight gradients
+//   update_kernel     sums the slabs, the bias and head gradients and the loss in
+//                     a fixed order, Adam with cosine-decayed lr, the FP32
+//                     master, the bf16 weights and transposed weights the next
+//                     step reads; the last block advances the step
 // All reductions run in a fixed order: training is deterministic.
 #include "sur_mlp.h"
 
@@ -24,6 +16,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <numeric>
 #include <random>
 #include <vector>
@@ -74,21 +67,6 @@ __global__ void init_params_kernel(float* P, uint64_t seed) {
         v = z0 * sqrtf(2.0f / kSurHid);
     }
     P[i] = v;
-}
-
-__global__ void gather_kernel(const __nv_bfloat16* __restrict__ xall, const float* __restrict__ tall,
-                              const int32_t* __restrict__ perm, const SurState* __restrict__ st,
-                              __nv_bfloat16* __restrict__ xb, __nv_bfloat16* __restrict__ xtb,
-                              float* __restrict__ tb) {
-    const int B = st->batch;
-    const int i = blockIdx.x;  // row in the batch
-    const int c = threadIdx.x; // feature column, 0..63
-    const int64_t b0 = static_cast<int64_t>(st->step % st->steps_per_epoch) * B;
-    const int64_t src = perm[b0 + i];
-    const __nv_bfloat16 v = xall[src * kSurInPad + c];
-    xb[static_cast<int64_t>(i) * kSurInPad + c] = v;
-    xtb[static_cast<int64_t>(c) * B + i] = v;
-    if (c == 0) tb[i] = tall[src];
 }
 
 // The residual's base: the Black-Scholes call / S at the Heston model's mean
@@ -233,109 +211,276 @@ quote_price_kernel(const double* __restrict__ fix, int64_t n, const float* __res
     if (i < n) out[i] = fix[i] * static_cast<double>(y[i]) - fix[n + i] + fix[2 * n + i];
 }
 
-// out[r] = sum_j X[r][j] * (w ? w[j] : 1), one warp per row, fixed order.
-__global__ void rowsum_kernel(const __nv_bfloat16* __restrict__ X, int rows, int L,
-                              const float* __restrict__ w, float* __restrict__ out) {
-    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= rows) return;
-    float acc = 0.0f;
-    const __nv_bfloat16* x = X + static_cast<int64_t>(row) * L;
-    for (int j = lane; j < L; j += 32) acc = fmaf(__bfloat162float(x[j]), w ? w[j] : 1.0f, acc);
+// ----------------------------------------------------------------------------
+// The update.  Block kinds, by blockIdx.x:
+//   [0, 128)     8 columns of db1, db2, db3 (sums of dZ over the batch) or dw4
+//                (sum of h3 dy), two a warp: 32 residue chains a column (lane =
+//                row mod 32, in row order), merged in a fixed shuffle tree
+//   128          db4 = sum dy and the loss (256 strided chains, a tree)
+//   [129, ...)   four weights a thread: their slabs in order
+// each followed by Adam on what it summed.  Bound by reading the slabs and dZ
+// back from L2 (50 MB at batch 8192).  Every array is read in the layout the
+// training pass writes (16-byte chunks, rows contiguous).
+// ----------------------------------------------------------------------------
+constexpr int kUpdThreads = 128;
+constexpr int kBiasBlocks = 128;
+constexpr int kWeightDepth = 32;
+constexpr size_t kUpdSmem = sizeof(uint4) * kWeightDepth * kUpdThreads;
+constexpr int kW1Quads = kSurHid * 16 / 4, kWQuads = kSurHid * kSurHid / 4;
+
+struct UpdateArgs {
+    const uint4* dz[3];              // dZ1, dZ2, dZ3
+    const uint4* h3;
+    const float *y, *target, *dy;    // [B]
+    const float4 *dw1, *dw2, *dw3;   // slabs
+    int batch;
+    float *P, *M, *V, *G;            // flat layout; G is written without update only
+    __nv_bfloat16 *W1b, *W2b, *W3b, *W2Tb, *W3Tb;
+    float* loss_hist;
+    int loss_cap;
+    int update;                      // 0: gradients only
+    SurState* st;
+    unsigned* blocks_done;
+};
+
+// add(k, value) for k = 0 .. n - 1 in order, value k the 16 bytes at addr(k),
+// through a ring of DEPTH asynchronous copies per thread (slot k of thread t at
+// buf[k % DEPTH][t] of T threads).  As register loads the compiler kept four
+// in flight and the chain waited on L2 at every fourth addition.
+template <int T, int DEPTH, class Addr, class Add>
+__device__ __forceinline__ void stream_sum(uint4* buf, int t, int n, const Addr& addr, const Add& add) {
+    constexpr int kGroup = 16, kAhead = DEPTH / kGroup;
+    auto issue = [&](int g) {
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
-    if (lane == 0) out[row] = acc;
+        for (int i = 0; i < kGroup; ++i) {
+            const int k = g * kGroup + i;
+            if (k < n) {
+                const uint32_t dst =
+                    static_cast<uint32_t>(__cvta_generic_to_shared(buf + (k % DEPTH) * T + t));
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(addr(k)) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int g = 0; g < kAhead; ++g) issue(g);
+    for (int g = 0; g * kGroup < n; ++g) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
+#pragma unroll
+        for (int i = 0; i < kGroup; ++i) {
+            const int k = g * kGroup + i;
+            if (k < n) add(k, buf[(k % DEPTH) * T + t]);
+        }
+        issue(g + kAhead);
+    }
 }
 
-// db4 = sum dy; loss = mean (y - t)^2, written to loss_hist[step].
-__global__ void loss_kernel(const float* __restrict__ y, const float* __restrict__ t,
-                            const float* __restrict__ dy, const SurState* __restrict__ st,
-                            float* __restrict__ db4, float* __restrict__ loss_hist, int loss_cap) {
-    __shared__ float s1[256], s2[256];
-    const int B = st->batch;
-    float a = 0.0f, b = 0.0f;
-    for (int i = threadIdx.x; i < B; i += 256) {
-        a += dy[i];
-        const float d = y[i] - t[i];
-        b = fmaf(d, d, b);
+// Adam with this step's constants.
+struct Adam {
+    float lr, b1, b2, eps, c1, c2;
+    __device__ __forceinline__ explicit Adam(const SurState& st) {
+        const int t = st.step + 1;
+        const float span = static_cast<float>(max(st.total_steps - st.step_begin, 1));
+        const float prog = fminf(static_cast<float>(st.step - st.step_begin) / span, 1.0f);
+        lr = st.lr0 * 0.5f * (1.0f + cosf(3.14159265358979f * prog));
+        b1 = st.beta1;
+        b2 = st.beta2;
+        eps = st.eps;
+        c1 = 1.0f - powf(st.beta1, static_cast<float>(t));
+        c2 = 1.0f - powf(st.beta2, static_cast<float>(t));
     }
-    s1[threadIdx.x] = a;
-    s2[threadIdx.x] = b;
+    __device__ __forceinline__ void operator()(float g, float& p, float& m, float& v) const {
+        m = b1 * m + (1.0f - b1) * g;
+        v = b2 * v + (1.0f - b2) * g * g;
+        const float mh = m / c1;
+        const float vh = v / c2;
+        p -= lr * mh / (sqrtf(vh) + eps);
+    }
+};
+
+__device__ __forceinline__ void update_one(const UpdateArgs& a, int idx, float g) {
+    if (!a.update) {
+        a.G[idx] = g;
+        return;
+    }
+    float p = a.P[idx], m = a.M[idx], v = a.V[idx];
+    Adam(*a.st)(g, p, m, v);
+    a.P[idx] = p;
+    a.M[idx] = m;
+    a.V[idx] = v;
+}
+
+__device__ __forceinline__ void update_columns(const UpdateArgs& a, int block) {
+    const int lane = threadIdx.x & 31, pair = threadIdx.x >> 5;
+    const int which = block >> 5, chunk = block & 31;
+    const uint32_t* x = reinterpret_cast<const uint32_t*>((which < 3 ? a.dz[which] : a.h3) + chunk * 128 + lane) + pair;
+    const float* w = which < 3 ? nullptr : a.dy + lane;
+    const int n = a.batch / 32;
+    // row 32 m + lane is row 32 (m % 4) + lane of tile m / 4
+    auto at = [&](int m) { return x + (static_cast<size_t>(m >> 2) * 32 * 128 + (m & 3) * 32) * 4; };
+    float s0 = 0.0f, s1 = 0.0f;
+    auto add = [&](uint32_t u, float wv) {
+        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u));
+        s0 = fmaf(f.x, wv, s0);
+        s1 = fmaf(f.y, wv, s1);
+    };
+    // 32 loads ahead of the additions (n is a multiple of 4)
+    int m = 0;
+    for (; m + 32 <= n; m += 32) {
+        uint32_t u[32];
+#pragma unroll
+        for (int k = 0; k < 32; ++k) u[k] = __ldg(at(m + k));
+        if (w) {
+            float wv[32];
+#pragma unroll
+            for (int k = 0; k < 32; ++k) wv[k] = __ldg(w + 32 * (m + k));
+#pragma unroll
+            for (int k = 0; k < 32; ++k) add(u[k], wv[k]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 32; ++k) add(u[k], 1.0f);
+        }
+    }
+    for (; m < n; m += 4) {
+        uint32_t u[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) u[k] = __ldg(at(m + k));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) add(u[k], w ? __ldg(w + 32 * (m + k)) : 1.0f);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        s0 += __shfl_down_sync(0xffffffffu, s0, off);
+        s1 += __shfl_down_sync(0xffffffffu, s1, off);
+    }
+    s1 = __shfl_sync(0xffffffffu, s1, 0);
+    if (lane < 2) {
+        const int off = which == 0 ? SurLayout::b1 : which == 1 ? SurLayout::b2
+                      : which == 2 ? SurLayout::b3 : SurLayout::w4;
+        update_one(a, off + chunk * 8 + pair * 2 + lane, lane == 0 ? s0 : s1);
+    }
+}
+
+__device__ __forceinline__ void update_loss(const UpdateArgs& a, float* s1, float* s2) {
+    // chains t and t + 128 of 256
+    const int t = threadIdx.x;
+    float d1[2] = {}, d2[2] = {};
+#pragma unroll 8
+    for (int i = t; i < a.batch; i += 256) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int k = i + h * 128;
+            if (k < a.batch) {
+                d1[h] += a.dy[k];
+                const float d = a.y[k] - a.target[k];
+                d2[h] = fmaf(d, d, d2[h]);
+            }
+        }
+    }
+    s1[t] = d1[0];
+    s2[t] = d2[0];
+    s1[t + 128] = d1[1];
+    s2[t + 128] = d2[1];
     __syncthreads();
     for (int off = 128; off > 0; off >>= 1) {
-        if (threadIdx.x < off) {
-            s1[threadIdx.x] += s1[threadIdx.x + off];
-            s2[threadIdx.x] += s2[threadIdx.x + off];
+        if (t < off) {
+            s1[t] += s1[t + off];
+            s2[t] += s2[t + off];
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        *db4 = s1[0];
-        const int k = st->step;
-        if (k >= 0 && k < loss_cap) loss_hist[k] = s2[0] / static_cast<float>(B);
+    if (t == 0) {
+        const int k = a.st->step;
+        if (k >= 0 && k < a.loss_cap) a.loss_hist[k] = s2[0] / static_cast<float>(a.batch);
+        update_one(a, SurLayout::b4, s1[0]);
     }
 }
 
-struct AdamSeg {
-    int off, n;               // range in the flat layout
-    const float* g;           // gradient (or split-K slabs); null: no gradient
-    int splits;
-    int64_t split_stride;
-    __nv_bfloat16* wb;        // bf16 copy, same layout (optional)
-    __nv_bfloat16* wtb;       // bf16 transpose (optional)
-    int rows, cols;
-};
+__device__ __forceinline__ void update_weights(const UpdateArgs& a, int e, uint4* ring) {
+    if (e >= kW1Quads + 2 * kWQuads) return;
+    // W1's slabs hold the first 16 columns; the padding's gradient is zero and
+    // leaves it zero
+    const int which = e < kW1Quads ? 0 : (e < kW1Quads + kWQuads ? 1 : 2);
+    const int local = which == 0 ? e : (which == 1 ? e - kW1Quads : e - kW1Quads - kWQuads);
+    const float4* slab = (which == 0 ? a.dw1 : (which == 1 ? a.dw2 : a.dw3)) + local;
+    const size_t stride = which == 0 ? kW1Quads : kWQuads;
+    float4 g = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    stream_sum<kUpdThreads, kWeightDepth>(
+        ring, threadIdx.x, a.batch / 128, [&](int k) { return slab + k * stride; },
+        [&](int, const uint4& v) {
+            g.x += __uint_as_float(v.x);
+            g.y += __uint_as_float(v.y);
+            g.z += __uint_as_float(v.z);
+            g.w += __uint_as_float(v.w);
+        });
+    // [half][chunk of 4 columns][row of 128]
+    const int half = local / (which == 0 ? 4 * 128 : 64 * 128);
+    const int row = half * 128 + (local & 127), c = ((local >> 7) & (which == 0 ? 3 : 63)) * 4;
+    const int at = row * (which == 0 ? kSurInPad : kSurHid) + c;
+    const int idx = (which == 0 ? SurLayout::W1 : which == 1 ? SurLayout::W2 : SurLayout::W3) + at;
+    if (!a.update) {
+        *reinterpret_cast<float4*>(a.G + idx) = g;
+        return;
+    }
+    float4 p = *reinterpret_cast<float4*>(a.P + idx);
+    float4 m = *reinterpret_cast<float4*>(a.M + idx);
+    float4 v = *reinterpret_cast<float4*>(a.V + idx);
+    const Adam adam(*a.st);
+    adam(g.x, p.x, m.x, v.x);
+    adam(g.y, p.y, m.y, v.y);
+    adam(g.z, p.z, m.z, v.z);
+    adam(g.w, p.w, m.w, v.w);
+    *reinterpret_cast<float4*>(a.P + idx) = p;
+    *reinterpret_cast<float4*>(a.M + idx) = m;
+    *reinterpret_cast<float4*>(a.V + idx) = v;
+    __nv_bfloat162 b[2] = {__floats2bfloat162_rn(p.x, p.y), __floats2bfloat162_rn(p.z, p.w)};
+    __nv_bfloat16* wb = which == 0 ? a.W1b : which == 1 ? a.W2b : a.W3b;
+    *reinterpret_cast<uint2*>(wb + at) = *reinterpret_cast<uint2*>(b);
+    if (which != 0) {
+        __nv_bfloat16* wt = (which == 1 ? a.W2Tb : a.W3Tb) + c * kSurHid + row;  // rows contiguous in a warp
+        wt[0] = b[0].x;
+        wt[kSurHid] = b[0].y;
+        wt[2 * kSurHid] = b[1].x;
+        wt[3 * kSurHid] = b[1].y;
+    }
+}
 
-struct AdamArgs {
-    AdamSeg seg[8];
-    int nseg;
-    int total;
-    float* P;
-    float* M;
-    float* V;
-    float* G;
-    int update;
-    const SurState* st;
-};
-
-__global__ void adam_kernel(const AdamArgs a) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= a.total) return;
-    int s = 0;
-    while (s + 1 < a.nseg && idx >= a.seg[s + 1].off) ++s;
-    const AdamSeg& sg = a.seg[s];
-    const int local = idx - sg.off;
-    if (local >= sg.n) return;
-    float p = a.P[idx];
-    if (sg.g != nullptr) {
-        float g = 0.0f;
-        for (int k = 0; k < sg.splits; ++k) g += sg.g[k * sg.split_stride + local];
-        a.G[idx] = g;
-        if (a.update) {
-            const SurState& st = *a.st;
-            const int t = st.step + 1;
-            const float span = static_cast<float>(max(st.total_steps - st.step_begin, 1));
-            const float prog = fminf(static_cast<float>(st.step - st.step_begin) / span, 1.0f);
-            const float lr = st.lr0 * 0.5f * (1.0f + cosf(3.14159265358979f * prog));
-            const float m = st.beta1 * a.M[idx] + (1.0f - st.beta1) * g;
-            const float v = st.beta2 * a.V[idx] + (1.0f - st.beta2) * g * g;
-            a.M[idx] = m;
-            a.V[idx] = v;
-            const float mh = m / (1.0f - powf(st.beta1, static_cast<float>(t)));
-            const float vh = v / (1.0f - powf(st.beta2, static_cast<float>(t)));
-            p -= lr * mh / (sqrtf(vh) + st.eps);
-            a.P[idx] = p;
+__global__ void __launch_bounds__(kUpdThreads) update_kernel(const UpdateArgs a) {
+    extern __shared__ uint4 ring[];
+    const int b = blockIdx.x;
+    if (b < kBiasBlocks) {
+        update_columns(a, b);
+    } else if (b == kBiasBlocks) {
+        update_loss(a, reinterpret_cast<float*>(ring), reinterpret_cast<float*>(ring) + 256);
+    } else {
+        update_weights(a, (b - kBiasBlocks - 1) * kUpdThreads + threadIdx.x, ring);
+    }
+    if (!a.update) return;
+    // every block has read the step; the last one advances it
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(a.blocks_done, 1u) == gridDim.x - 1) {
+            *a.blocks_done = 0u;
+            a.st->step += 1;
         }
     }
-    const __nv_bfloat16 pb = __float2bfloat16_rn(p);
-    if (sg.wb) sg.wb[local] = pb;
-    if (sg.wtb) {
-        const int r = local / sg.cols, c = local % sg.cols;
-        sg.wtb[static_cast<int64_t>(c) * sg.rows + r] = pb;
-    }
 }
 
-__global__ void advance_kernel(SurState* st) { st->step += 1; }
+// bf16 weights and transposes from the FP32 master (after init and loads).
+__global__ void refresh_kernel(const float* __restrict__ P, __nv_bfloat16* W1b, __nv_bfloat16* W2b,
+                               __nv_bfloat16* W3b, __nv_bfloat16* W2Tb, __nv_bfloat16* W3Tb) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kSurHid * kSurInPad) W1b[i] = __float2bfloat16_rn(P[SurLayout::W1 + i]);
+    if (i < kSurHid * kSurHid) {
+        const int r = i >> 8, c = i & 255;
+        const __nv_bfloat16 w2 = __float2bfloat16_rn(P[SurLayout::W2 + i]);
+        const __nv_bfloat16 w3 = __float2bfloat16_rn(P[SurLayout::W3 + i]);
+        W2b[i] = w2;
+        W3b[i] = w3;
+        W2Tb[c * kSurHid + r] = w2;
+        W3Tb[c * kSurHid + r] = w3;
+    }
+}
 
 bool tmap(CUtensorMap* m, const void* base, int64_t rows, int64_t cols, int box_rows) {
     return make_tmap_bf16(m, base, static_cast<uint64_t>(rows), static_cast<uint64_t>(cols),
@@ -356,25 +501,27 @@ struct DeviceGuard {
 
 }  // namespace
 
+struct SurModel::StepLaunch {
+    TrainMaps maps;
+    TrainArgs train;
+    UpdateArgs update;
+};
+
 // ----------------------------------------------------------------------------
 SurModel::~SurModel() {
     if (device_ < 0) return;
     DeviceGuard g(device_);
-    if (step_graph_) cudaGraphExecDestroy(step_graph_);
-    float* fl[] = {P_, M_, V_, G_, Tall_, Tb_, y_, dy_, dW1p_, dW2p_, dW3p_, db1_, db2_, db3_, dw4_, db4_, loss_hist_, Py_, Pbase_};
+    float* fl[] = {P_, M_, V_, G_, Tall_, Tb_, y_, dy_, dW1p_, dW2p_, dW3p_, loss_hist_, Py_, Pbase_};
     for (float* p : fl)
         if (p) cudaFree(p);
-    __nv_bfloat16* bl[] = {W1b_, W2b_, W3b_, W2Tb_, W3Tb_, Xall_, Xb_, XTb_, Z1_, H1_, H1T_, Z2_, H2_, H2T_,
-                           dZ3_, dZ3T_, H3T_, dZ2_, dZ2T_, dZ1_, dZ1T_, PX_, PH1_, PH2_};
+    __nv_bfloat16* bl[] = {W1b_, W2b_, W3b_, W2Tb_, W3Tb_, Xall_, Z1_, H1_, Z2_, H3_, dZ3_, dZ2_, dZ1_,
+                           PX_, PH1_, PH2_};
     for (__nv_bfloat16* p : bl)
         if (p) cudaFree(p);
     if (perm_) cudaFree(perm_);
     if (state_) cudaFree(state_);
+    if (blocks_done_) cudaFree(blocks_done_);
     if (d_in_) cudaFree(d_in_);
-    for (cudaEvent_t& e : ev_)
-        if (e) cudaEventDestroy(e);
-    for (cudaStream_t& a : aux_)
-        if (a) cudaStreamDestroy(a);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -382,8 +529,6 @@ cudaError_t SurModel::init(uint64_t seed, const SurBox& box) {
     QK_TRY(cudaGetDevice(&device_));
     box_ = box;
     QK_TRY(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
-    for (cudaStream_t& a : aux_) QK_TRY(cudaStreamCreateWithFlags(&a, cudaStreamNonBlocking));
-    for (cudaEvent_t& e : ev_) QK_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     QK_TRY(dalloc(&P_, SurLayout::total));
     QK_TRY(dalloc(&M_, SurLayout::total));
     QK_TRY(dalloc(&V_, SurLayout::total));
@@ -394,6 +539,8 @@ cudaError_t SurModel::init(uint64_t seed, const SurBox& box) {
     QK_TRY(dalloc(&W2Tb_, kSurHid * kSurHid));
     QK_TRY(dalloc(&W3Tb_, kSurHid * kSurHid));
     QK_TRY(dalloc(&state_, 1));
+    QK_TRY(dalloc(&blocks_done_, 1));
+    QK_TRY(cudaMemsetAsync(blocks_done_, 0, sizeof(unsigned), stream_));
     SurState s{};
     s.beta1 = 0.9f;
     s.beta2 = 0.999f;
@@ -438,31 +585,12 @@ cudaError_t SurModel::features_device(const double* f, int64_t n, __nv_bfloat16*
 }
 
 cudaError_t SurModel::refresh_bf16(cudaStream_t st) {
-    AdamArgs a{};
-    const int hid2 = kSurHid * kSurHid;
-    a.seg[0] = AdamSeg{SurLayout::W1, kSurHid * kSurInPad, nullptr, 0, 0, W1b_, nullptr, kSurHid, kSurInPad};
-    a.seg[1] = AdamSeg{SurLayout::W2, hid2, nullptr, 0, 0, W2b_, W2Tb_, kSurHid, kSurHid};
-    a.seg[2] = AdamSeg{SurLayout::W3, hid2, nullptr, 0, 0, W3b_, W3Tb_, kSurHid, kSurHid};
-    a.nseg = 3;
-    a.total = SurLayout::b3;
-    a.P = P_;
-    a.M = M_;
-    a.V = V_;
-    a.G = G_;
-    a.update = 0;
-    a.st = state_;
-    // segments must be ordered and contiguous for the lookup: W1 | b1 gap | W2 ...
-    // (indices in gaps find the previous segment and return at local >= n)
-    adam_kernel<<<(a.total + 255) / 256, 256, 0, st>>>(a);
+    refresh_kernel<<<kSurHid * kSurHid / 256, 256, 0, st>>>(P_, W1b_, W2b_, W3b_, W2Tb_, W3Tb_);
     return cudaGetLastError();
 }
 
 cudaError_t SurModel::set_dataset(const double* features, const double* target, int64_t n) {
     DeviceGuard g(device_);
-    if (step_graph_) {
-        cudaGraphExecDestroy(step_graph_);
-        step_graph_ = nullptr;
-    }
     std::vector<__nv_bfloat16> rows(static_cast<size_t>(n) * kSurInPad);
     normalise(features, n, rows.data());
     // the network learns target - base
@@ -485,130 +613,101 @@ cudaError_t SurModel::set_dataset(const double* features, const double* target, 
 
 cudaError_t SurModel::ensure_batch_buffers(int B) {
     if (B == batch_) return cudaSuccess;
-    if (step_graph_) {
-        cudaGraphExecDestroy(step_graph_);
-        step_graph_ = nullptr;
-    }
+    batch_ = 0;
     const size_t BH = static_cast<size_t>(B) * kSurHid;
     const int S = B / 128;
-    QK_TRY(dalloc(&Xb_, static_cast<size_t>(B) * kSurInPad));
-    QK_TRY(dalloc(&XTb_, static_cast<size_t>(B) * kSurInPad));
-    QK_TRY(dalloc(&Tb_, B));
-    __nv_bfloat16** act[] = {&Z1_, &H1_, &H1T_, &Z2_, &H2_, &H2T_, &dZ3_, &dZ3T_, &H3T_, &dZ2_, &dZ2T_, &dZ1_, &dZ1T_};
+    __nv_bfloat16** act[] = {&Z1_, &H1_, &Z2_, &H3_, &dZ3_, &dZ2_, &dZ1_};
     for (auto p : act) QK_TRY(dalloc(p, BH));
+    QK_TRY(dalloc(&Tb_, B));
     QK_TRY(dalloc(&y_, B));
     QK_TRY(dalloc(&dy_, B));
-    QK_TRY(dalloc(&dW1p_, static_cast<size_t>(S) * kSurHid * kSurInPad));
+    QK_TRY(dalloc(&dW1p_, static_cast<size_t>(S) * kSurHid * 16));
     QK_TRY(dalloc(&dW2p_, static_cast<size_t>(S) * kSurHid * kSurHid));
     QK_TRY(dalloc(&dW3p_, static_cast<size_t>(S) * kSurHid * kSurHid));
-    float** vec[] = {&db1_, &db2_, &db3_, &dw4_};
-    for (auto p : vec) QK_TRY(dalloc(p, kSurHid));
-    QK_TRY(dalloc(&db4_, 4));
     batch_ = B;
     return cudaSuccess;
 }
 
-cudaError_t SurModel::run_step(cudaStream_t st, bool update) {
-    const int B = batch_;
-    const int S = B / 128;
-    CUtensorMap tXb, tW1, tH1, tW2, tH2, tW3, tdZ3, tW3T, tdZ3T, tH2T, tdZ2, tW2T, tdZ2T, tH1T, tdZ1T, tXTb;
-    bool ok = tmap(&tXb, Xb_, B, kSurInPad, 128) && tmap(&tW1, W1b_, kSurHid, kSurInPad, 128) &&
-              tmap(&tH1, H1_, B, kSurHid, 128) && tmap(&tW2, W2b_, kSurHid, kSurHid, 128) &&
-              tmap(&tH2, H2_, B, kSurHid, 128) && tmap(&tW3, W3b_, kSurHid, kSurHid, 256) &&
-              tmap(&tdZ3, dZ3_, B, kSurHid, 128) && tmap(&tW3T, W3Tb_, kSurHid, kSurHid, 128) &&
-              tmap(&tdZ3T, dZ3T_, kSurHid, B, 128) && tmap(&tH2T, H2T_, kSurHid, B, 128) &&
-              tmap(&tdZ2, dZ2_, B, kSurHid, 128) && tmap(&tW2T, W2Tb_, kSurHid, kSurHid, 128) &&
-              tmap(&tdZ2T, dZ2T_, kSurHid, B, 128) && tmap(&tH1T, H1T_, kSurHid, B, 128) &&
-              tmap(&tdZ1T, dZ1T_, kSurHid, B, 128) && tmap(&tXTb, XTb_, kSurInPad, B, 64);
-    if (!ok) return cudaErrorInvalidValue;
-    int* err = &state_->err;
-
-    gather_kernel<<<B, kSurInPad, 0, st>>>(Xall_, Tall_, perm_, state_, Xb_, XTb_, Tb_);
-    QK_TRY(cudaGetLastError());
-
-    GemmArgs g{};
-    g.err = err;
-    // layer 1 forward
-    g.M = B; g.N = kSurHid; g.K = kSurInPad; g.k_per_split = kSurInPad;
-    g.bias = P_ + SurLayout::b1; g.z_out = Z1_; g.h_out = H1_; g.t_out = H1T_; g.ldt = B;
-    QK_TRY(launch_umma_gemm(kEpiFwd, 128, tXb, tW1, g, 1, st));
-    // layer 2 forward
-    g.K = kSurHid; g.k_per_split = kSurHid;
-    g.bias = P_ + SurLayout::b2; g.z_out = Z2_; g.h_out = H2_; g.t_out = H2T_;
-    QK_TRY(launch_umma_gemm(kEpiFwd, 128, tH1, tW2, g, 1, st));
-    // layer 3 forward + head + loss gradient
-    GemmArgs l{};
-    l.err = err;
-    l.M = B; l.N = kSurHid; l.K = kSurHid; l.k_per_split = kSurHid;
-    l.bias = P_ + SurLayout::b3; l.w4 = P_ + SurLayout::w4; l.b4 = P_ + SurLayout::b4;
-    l.target = Tb_; l.y_out = y_; l.dy_out = dy_; l.loss_scale = 2.0f / static_cast<float>(B);
-    l.d_out = dZ3_; l.dt_out = dZ3T_; l.t_out = H3T_; l.ldt = B;
-    QK_TRY(launch_umma_gemm(kEpiLast, 256, tH2, tW3, l, 1, st));
-    // Side branch 1 (aux_[0]): the loss, db3, dw4 and the dW3 GEMM read only
-    // what layer 3's epilogue wrote; they run beside the backward chain.
-    QK_TRY(cudaEventRecord(ev_[0], st));
-    QK_TRY(cudaStreamWaitEvent(aux_[0], ev_[0], 0));
-    loss_kernel<<<1, 256, 0, aux_[0]>>>(y_, Tb_, dy_, state_, db4_, loss_hist_, loss_cap_);
-    rowsum_kernel<<<kSurHid / 8, 256, 0, aux_[0]>>>(dZ3T_, kSurHid, B, nullptr, db3_);
-    rowsum_kernel<<<kSurHid / 8, 256, 0, aux_[0]>>>(H3T_, kSurHid, B, dy_, dw4_);
-    QK_TRY(cudaGetLastError());
-    GemmArgs w{};
-    w.err = err;
-    w.M = kSurHid; w.N = kSurHid; w.K = B; w.k_per_split = 128; w.c_f32 = dW3p_;
-    QK_TRY(launch_umma_gemm(kEpiF32, 128, tdZ3T, tH2T, w, S, aux_[0]));
-    QK_TRY(cudaEventRecord(ev_[1], aux_[0]));
-    // layer 3 backward to layer 2
-    GemmArgs b{};
-    b.err = err;
-    b.M = B; b.N = kSurHid; b.K = kSurHid; b.k_per_split = kSurHid; b.ldt = B;
-    b.z_in = Z2_; b.d_out = dZ2_; b.dt_out = dZ2T_;
-    QK_TRY(launch_umma_gemm(kEpiBwd, 128, tdZ3, tW3T, b, 1, st));
-    // Side branch 2 (aux_[1]): dW2 and db2 read layer 2's gradient
-    QK_TRY(cudaEventRecord(ev_[2], st));
-    QK_TRY(cudaStreamWaitEvent(aux_[1], ev_[2], 0));
-    GemmArgs w2 = w;
-    w2.c_f32 = dW2p_;
-    QK_TRY(launch_umma_gemm(kEpiF32, 128, tdZ2T, tH1T, w2, S, aux_[1]));
-    rowsum_kernel<<<kSurHid / 8, 256, 0, aux_[1]>>>(dZ2T_, kSurHid, B, nullptr, db2_);
-    QK_TRY(cudaGetLastError());
-    QK_TRY(cudaEventRecord(ev_[3], aux_[1]));
-    // layer 2 backward to layer 1, dW1 (N = 64 padded inputs) and db1
-    b.z_in = Z1_; b.d_out = dZ1_; b.dt_out = dZ1T_;
-    QK_TRY(launch_umma_gemm(kEpiBwd, 128, tdZ2, tW2T, b, 1, st));
-    GemmArgs w1 = w;
-    w1.N = kSurInPad; w1.c_f32 = dW1p_;
-    QK_TRY(launch_umma_gemm(kEpiF32, 64, tdZ1T, tXTb, w1, S, st));
-    rowsum_kernel<<<kSurHid / 8, 256, 0, st>>>(dZ1T_, kSurHid, B, nullptr, db1_);
-    QK_TRY(cudaGetLastError());
-    // join both branches before Adam reads every gradient
-    QK_TRY(cudaStreamWaitEvent(st, ev_[1], 0));
-    QK_TRY(cudaStreamWaitEvent(st, ev_[3], 0));
-
-    AdamArgs a{};
-    const int hid2 = kSurHid * kSurHid;
-    a.seg[0] = AdamSeg{SurLayout::W1, kSurHid * kSurInPad, dW1p_, S, (int64_t)kSurHid * kSurInPad, W1b_, nullptr, kSurHid, kSurInPad};
-    a.seg[1] = AdamSeg{SurLayout::b1, kSurHid, db1_, 1, 0, nullptr, nullptr, 1, kSurHid};
-    a.seg[2] = AdamSeg{SurLayout::W2, hid2, dW2p_, S, hid2, W2b_, W2Tb_, kSurHid, kSurHid};
-    a.seg[3] = AdamSeg{SurLayout::b2, kSurHid, db2_, 1, 0, nullptr, nullptr, 1, kSurHid};
-    a.seg[4] = AdamSeg{SurLayout::W3, hid2, dW3p_, S, hid2, W3b_, W3Tb_, kSurHid, kSurHid};
-    a.seg[5] = AdamSeg{SurLayout::b3, kSurHid, db3_, 1, 0, nullptr, nullptr, 1, kSurHid};
-    a.seg[6] = AdamSeg{SurLayout::w4, kSurHid, dw4_, 1, 0, nullptr, nullptr, 1, kSurHid};
-    a.seg[7] = AdamSeg{SurLayout::b4, 1, db4_, 1, 0, nullptr, nullptr, 1, 1};
-    a.nseg = 8;
-    a.total = SurLayout::b4 + 1;
-    a.P = P_;
-    a.M = M_;
-    a.V = V_;
-    a.G = G_;
-    a.update = update ? 1 : 0;
-    a.st = state_;
-    adam_kernel<<<(a.total + 255) / 256, 256, 0, st>>>(a);
-    QK_TRY(cudaGetLastError());
-    if (update) {
-        advance_kernel<<<1, 1, 0, st>>>(state_);
-        QK_TRY(cudaGetLastError());
-    }
+// What every step of a call launches: the step's kernels read the step
+// counter and the schedule from state_.
+cudaError_t SurModel::prepare_steps(bool update, StepLaunch* s) {
+    TrainMaps& m = s->maps;
+    if (!(make_tmap_bf16_k16(&m.w1, W1b_, kSurHid, kSurInPad, 256) &&
+          tmap(&m.w2, W2b_, kSurHid, kSurHid, 256) && tmap(&m.w3, W3b_, kSurHid, kSurHid, 256) &&
+          tmap(&m.w3t, W3Tb_, kSurHid, kSurHid, 256) && tmap(&m.w2t, W2Tb_, kSurHid, kSurHid, 256)))
+        return cudaErrorInvalidValue;
+    TrainArgs& t = s->train;
+    t = TrainArgs{};
+    t.xall = Xall_;
+    t.x_stride = kSurInPad;
+    t.tall = Tall_;
+    t.perm = perm_;
+    t.step = &state_->step;
+    t.steps_per_epoch = &state_->steps_per_epoch;
+    t.batch = batch_;
+    t.loss_scale = 2.0f / static_cast<float>(batch_);
+    t.b1 = P_ + SurLayout::b1;
+    t.b2 = P_ + SurLayout::b2;
+    t.b3 = P_ + SurLayout::b3;
+    t.w4 = P_ + SurLayout::w4;
+    t.b4 = P_ + SurLayout::b4;
+    t.z1 = reinterpret_cast<uint4*>(Z1_);
+    t.z2 = reinterpret_cast<uint4*>(Z2_);
+    t.h1 = reinterpret_cast<uint4*>(H1_);
+    t.h3 = reinterpret_cast<uint4*>(H3_);
+    t.dz3 = reinterpret_cast<uint4*>(dZ3_);
+    t.dz2 = reinterpret_cast<uint4*>(dZ2_);
+    t.dz1 = reinterpret_cast<uint4*>(dZ1_);
+    t.y_out = y_;
+    t.dy_out = dy_;
+    t.target_out = Tb_;
+    t.dw1 = reinterpret_cast<float4*>(dW1p_);
+    t.dw2 = reinterpret_cast<float4*>(dW2p_);
+    t.dw3 = reinterpret_cast<float4*>(dW3p_);
+    t.err = &state_->err;
+    UpdateArgs& u = s->update;
+    u = UpdateArgs{};
+    u.dz[0] = reinterpret_cast<const uint4*>(dZ1_);
+    u.dz[1] = reinterpret_cast<const uint4*>(dZ2_);
+    u.dz[2] = reinterpret_cast<const uint4*>(dZ3_);
+    u.h3 = reinterpret_cast<const uint4*>(H3_);
+    u.y = y_;
+    u.target = Tb_;
+    u.dy = dy_;
+    u.dw1 = reinterpret_cast<const float4*>(dW1p_);
+    u.dw2 = reinterpret_cast<const float4*>(dW2p_);
+    u.dw3 = reinterpret_cast<const float4*>(dW3p_);
+    u.batch = batch_;
+    u.P = P_;
+    u.M = M_;
+    u.V = V_;
+    u.G = G_;
+    u.W1b = W1b_;
+    u.W2b = W2b_;
+    u.W3b = W3b_;
+    u.W2Tb = W2Tb_;
+    u.W3Tb = W3Tb_;
+    u.loss_hist = loss_hist_;
+    u.loss_cap = loss_cap_;
+    u.update = update ? 1 : 0;
+    u.st = state_;
+    u.blocks_done = blocks_done_;
     return cudaSuccess;
+}
+
+cudaError_t SurModel::run_step(const StepLaunch& s, cudaStream_t st) {
+    static std::once_flag once;
+    static cudaError_t attr_err = cudaSuccess;
+    std::call_once(once, [] {
+        attr_err = cudaFuncSetAttribute(update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(kUpdSmem));
+    });
+    QK_TRY(attr_err);
+    QK_TRY(launch_mlp_train(s.maps, s.train, st));
+    constexpr int kQuads = kW1Quads + 2 * kWQuads;
+    update_kernel<<<kBiasBlocks + 1 + (kQuads + kUpdThreads - 1) / kUpdThreads, kUpdThreads, kUpdSmem, st>>>(
+        s.update);
+    return cudaGetLastError();
 }
 
 cudaError_t SurModel::train(int epochs, int batch, float lr0, uint64_t shuffle_seed,
@@ -622,12 +721,12 @@ cudaError_t SurModel::train(int epochs, int batch, float lr0, uint64_t shuffle_s
     QK_TRY(cudaMemcpy(&s, state_, sizeof s, cudaMemcpyDeviceToHost));
     const int step0 = s.step;
     if (loss_cap_ < step0 + total) {
-        QK_TRY(dalloc(&loss_hist_, static_cast<size_t>(step0 + total)));
-        loss_cap_ = step0 + total;
-        if (step_graph_) {
-            cudaGraphExecDestroy(step_graph_);
-            step_graph_ = nullptr;
-        }
+        // half as much again, so that a caller training epoch by epoch does
+        // not reallocate on every call
+        const int cap = step0 + total + (step0 + total) / 2;
+        loss_cap_ = 0;
+        QK_TRY(dalloc(&loss_hist_, static_cast<size_t>(cap)));
+        loss_cap_ = cap;
     }
     s.total_steps = step0 + total;
     s.step_begin = step0;
@@ -638,33 +737,27 @@ cudaError_t SurModel::train(int epochs, int batch, float lr0, uint64_t shuffle_s
     // steps_per_epoch and batch change the gather: keep the step counter and
     // make epoch boundaries relative to it
     QK_TRY(cudaMemcpy(state_, &s, sizeof s, cudaMemcpyHostToDevice));
-    if (!step_graph_) {
-        cudaGraph_t graph;
-        QK_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-        cudaError_t le = run_step(stream_, true);
-        cudaError_t ce = cudaStreamEndCapture(stream_, &graph);
-        if (le != cudaSuccess) return le;
-        QK_TRY(ce);
-        ce = cudaGraphInstantiate(&step_graph_, graph, 0);
-        cudaGraphDestroy(graph);
-        QK_TRY(ce);
-    }
+    StepLaunch step;
+    QK_TRY(prepare_steps(true, &step));
     std::mt19937_64 rng(shuffle_seed);
     std::vector<int32_t> perm(static_cast<size_t>(n_data_));
     std::iota(perm.begin(), perm.end(), 0);
+    // the gather reads perm[(step % spe) * batch + i]: the permutation goes up
+    // rotated, in two pieces, so that the epoch starts at its beginning whatever
+    // step0 % spe is.  The copies run on the stream, after the epoch before, and
+    // have read perm when they return: the next shuffle overlaps this epoch.
+    const int64_t head = static_cast<int64_t>(spe - step0 % spe) * batch;
+    const int64_t all = static_cast<int64_t>(spe) * batch;
+    auto upload = [&](int64_t to, int64_t from, int64_t count) -> cudaError_t {
+        if (count == 0) return cudaSuccess;
+        return cudaMemcpyAsync(perm_ + to, perm.data() + from, static_cast<size_t>(count) * sizeof(int32_t),
+                               cudaMemcpyHostToDevice, stream_);
+    };
     for (int e = 0; e < epochs; ++e) {
         std::shuffle(perm.begin(), perm.end(), rng);
-        // the gather reads perm[(step % spe) * batch + i]: rotate so the epoch
-        // starts at the permutation's beginning whatever step0 % spe is
-        const int rot = (step0 + e * spe) % spe;
-        std::vector<int32_t> rotated(perm.size());
-        for (int j = 0; j < spe; ++j)
-            std::copy(perm.begin() + static_cast<int64_t>(j) * batch, perm.begin() + static_cast<int64_t>(j + 1) * batch,
-                      rotated.begin() + static_cast<int64_t>((j + rot) % spe) * batch);
-        QK_TRY(cudaStreamSynchronize(stream_));
-        QK_TRY(cudaMemcpy(perm_, rotated.data(), static_cast<size_t>(spe) * batch * sizeof(int32_t),
-                          cudaMemcpyHostToDevice));
-        for (int j = 0; j < spe; ++j) QK_TRY(cudaGraphLaunch(step_graph_, stream_));
+        QK_TRY(upload(all - head, 0, head));
+        QK_TRY(upload(0, head, all - head));
+        for (int j = 0; j < spe; ++j) QK_TRY(run_step(step, stream_));
     }
     QK_TRY(cudaStreamSynchronize(stream_));
     std::vector<float> hist(static_cast<size_t>(total));
@@ -900,7 +993,9 @@ cudaError_t SurModel::gradients(const double* features, const double* target, in
     s.batch = n;
     s.steps_per_epoch = 1;
     QK_TRY(cudaMemcpy(state_, &s, sizeof s, cudaMemcpyHostToDevice));
-    QK_TRY(run_step(stream_, false));
+    StepLaunch step;
+    QK_TRY(prepare_steps(false, &step));
+    QK_TRY(run_step(step, stream_));
     QK_TRY(cudaStreamSynchronize(stream_));
     std::vector<float> G(SurLayout::total);
     QK_TRY(cudaMemcpy(G.data(), G_, G.size() * sizeof(float), cudaMemcpyDeviceToHost));

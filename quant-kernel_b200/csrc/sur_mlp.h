@@ -108,16 +108,13 @@ private:
     template <class Fill, class Enqueue, class Drain>
     cudaError_t run_chunked(int64_t n, size_t in_row, size_t out_row, const Fill& fill,
                             const Enqueue& enqueue, const Drain& drain);
-    cudaError_t run_step(cudaStream_t st, bool update);
+    struct StepLaunch;  // the arguments of a step's two kernels
+    cudaError_t prepare_steps(bool update, StepLaunch* s);
+    cudaError_t run_step(const StepLaunch& s, cudaStream_t st);
     cudaError_t refresh_bf16(cudaStream_t st);
 
     int device_ = -1;
     cudaStream_t stream_ = nullptr;
-    // the training step's side branches (loss and bias sums with the dW3
-    // GEMM; the dW2 GEMM with db2) run on these beside the backward chain,
-    // forked and joined by events (inside the captured step graph too)
-    cudaStream_t aux_[2] = {nullptr, nullptr};
-    cudaEvent_t ev_[4] = {nullptr, nullptr, nullptr, nullptr};
     SurBox box_{};
     int32_t base_kind_ = kSurBaseBsmMeanVar;
     // parameters, Adam moments, gradient
@@ -134,18 +131,14 @@ private:
     int64_t n_data_ = 0;
     // training batch buffers
     int batch_ = 0;
-    __nv_bfloat16 *Xb_ = nullptr, *XTb_ = nullptr;
     float* Tb_ = nullptr;
-    __nv_bfloat16 *Z1_ = nullptr, *H1_ = nullptr, *H1T_ = nullptr;
-    __nv_bfloat16 *Z2_ = nullptr, *H2_ = nullptr, *H2T_ = nullptr;
-    __nv_bfloat16 *dZ3_ = nullptr, *dZ3T_ = nullptr, *H3T_ = nullptr;
-    __nv_bfloat16 *dZ2_ = nullptr, *dZ2T_ = nullptr, *dZ1_ = nullptr, *dZ1T_ = nullptr;
+    __nv_bfloat16 *Z1_ = nullptr, *H1_ = nullptr, *Z2_ = nullptr, *H3_ = nullptr;
+    __nv_bfloat16 *dZ3_ = nullptr, *dZ2_ = nullptr, *dZ1_ = nullptr;
     float *y_ = nullptr, *dy_ = nullptr;
     float *dW1p_ = nullptr, *dW2p_ = nullptr, *dW3p_ = nullptr;
-    float *db1_ = nullptr, *db2_ = nullptr, *db3_ = nullptr, *dw4_ = nullptr, *db4_ = nullptr;
+    unsigned* blocks_done_ = nullptr;  // update_kernel's block counter
     float* loss_hist_ = nullptr;
     int loss_cap_ = 0;
-    cudaGraphExec_t step_graph_ = nullptr;
     // inference buffers
     int64_t pred_rows_ = 0;
     int sm_count_ = 0;
