@@ -751,7 +751,8 @@ __global__ void __launch_bounds__(kInferThreads, 1)
 // untransposed as the MN-major operands of the weight gradients (row = K),
 // which the 128-byte-swizzled layout [64-column block][row][64 columns] is as
 // it stands.  Batch 8192 runs 64 CTAs, each a chain of ten short MMA jobs and
-// as many epilogues: latency bounds it, not a pipe.
+// as many epilogues: latency bounds it, not a pipe (45 us, and 16 us for the
+// update; the 14 launches took 129 us a step, the same losses and weights).
 //
 // Global arrays of the pass are laid out by chunk, [tile][16-byte chunk of a
 // row][128 rows], so that a warp's stores (one row per lane) are contiguous:
@@ -760,27 +761,31 @@ __global__ void __launch_bounds__(kInferThreads, 1)
 // Shared memory: P and Q (64 KiB each) hold H1, H2; then D3 in P and D2, H1
 // (read back from this thread's own global copy), D1 as their readers
 // complete; a 2-slot ring of 32 KiB weight blocks; X (128 x 16) and W1 (256 x
-// 16).  TMEM: accumulator 0 for the layers, accumulator 1 for the weight
-// gradients (256 columns each).  Roles: warp 16 streams weights, warp 17
+// 16).  TMEM: two accumulators of 256 columns.
+// Roles: warp 16 streams weights, warp 17
 // issues MMAs, warps 0-15 gather and run the epilogues (the lane and column
 // split of mlp_infer_kernel).  Job j's completion arrives on full[j],
-// epilogue e's on done[e]; each is used once, and every wait is bounded.
+// hand-overs to the MMA warp on blk and done; each barrier is used once, and
+// every wait is bounded.
 //
-//   job  MMA                              epilogue
-//   0    X W1^T          -> acc0          0  z1, h1 -> P
-//   1    P W2^T          -> acc0          1  z2, h2 -> Q
-//   2    Q W3^T          -> acc0          2  head, dy, dz3 -> P
-//   3    dW3 rows 0-127  -> acc1          3  slab out
-//   4    P W3            -> acc0
-//   5    dW3 rows 128-   -> acc1          4  (4 and 5 done) dz2 -> Q, h1 -> P
-//   6    Q W2            -> acc0          5  slab out
-//   7    dW2 rows 0-127  -> acc1          6  slab out
-//   8    dW2 rows 128-   -> acc1          7  (6 and 8 done) dz1 -> Q
-//   9    dW1             -> acc0          8  slabs out
+//   job  MMA                              epilogue after it
+//   0    X W1^T          -> acc0          z1, h1 -> P
+//   1    P W2^T          -> acc1          z2, h2 -> Q
+//   2    Q W3^T          -> acc0          head, dy, dz3 -> P
+//   3    P W3            -> acc1
+//   4    dW3 rows 0-127  -> acc0          slab out
+//   5    dW3 rows 128-   -> acc0          h1 -> P, slab out, then (job 3) dz2 -> Q
+//   6    Q W2            -> acc0
+//   7    dW2 rows 0-127  -> acc1          slab out
+//   8    dW2 rows 128-   -> acc1          (with job 6) dz1 -> Q, slab out
+//   9    dW1             -> acc0          slab out
+//
+// A layer's MMAs start per 64-column block as the epilogue before it writes the
+// block (blk), into the accumulator that epilogue is not reading.
 // ----------------------------------------------------------------------------
 constexpr int kTrainEpiWarps = 16;
 constexpr int kTrainThreads = (kTrainEpiWarps + 2) * 32;
-constexpr int kTrainJobs = 10, kTrainDone = 8;
+constexpr int kTrainJobs = 10, kTrainDone = 3, kTrainBlocked = 4;
 constexpr size_t kTrainSmem = 2 * kHBytes + kIWSlots * kWBlock + kW1Bytes + kXBytes + 1024;
 
 // MN-major shared-memory descriptors: rows of 128 (32) swizzled bytes along
@@ -832,7 +837,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     uint8_t* w1s = wbuf + kIWSlots * kWBlock;
     uint8_t* xs = w1s + kW1Bytes;
     __shared__ __align__(8) uint64_t w1full, xready, pready, drain;
-    __shared__ __align__(8) uint64_t full[kTrainJobs], done[kTrainDone];
+    __shared__ __align__(8) uint64_t full[kTrainJobs], done[kTrainDone], blk[kTrainBlocked][4];
     __shared__ __align__(8) uint64_t wfull[kIWSlots], wempty[kIWSlots];
     __shared__ __align__(16) float sb1[kSurHidden], sb2[kSurHidden], sb3[kSurHidden], sw4[kSurHidden];
     __shared__ float part[4][kBM];
@@ -855,6 +860,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
         mbar_init(smem_u32(&drain), 1);
         for (int j = 0; j < kTrainJobs; ++j) mbar_init(smem_u32(&full[j]), 1);
         for (int e = 0; e < kTrainDone; ++e) mbar_init(smem_u32(&done[e]), kTrainEpiWarps);
+        for (int e = 0; e < kTrainBlocked * 4; ++e) mbar_init(smem_u32(&blk[e >> 2][e & 3]), kTrainEpiWarps);
         for (int s = 0; s < kIWSlots; ++s) {
             mbar_init(smem_u32(&wfull[s]), 1);
             mbar_init(smem_u32(&wempty[s]), 1);
@@ -915,17 +921,19 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
             auto commit = [&](int j) {
                 if (ok) umma_commit(smem_u32(&full[j]));
             };
-            // a layer: buf [128 x 256] times the next four ring blocks
-            auto layer = [&](const uint8_t* buf) {
+            // a layer: buf [128 x 256] times the next four ring blocks, each
+            // block as epilogue e hands it over
+            auto layer = [&](const uint8_t* buf, uint32_t acc, int e) {
                 for (int kb = 0; ok && kb < 4; ++kb) {
                     const uint32_t s = wc % kIWSlots;
-                    ok = mbar_wait(smem_u32(&wfull[s]), (wc / kIWSlots) & 1);
+                    wait(&blk[e][kb]);
+                    if (ok) ok = mbar_wait(smem_u32(&wfull[s]), (wc / kIWSlots) & 1);
                     if (!ok) return;
                     fence_after();
                     const uint32_t sa = smem_u32(buf + kb * kABytes), sb = smem_u32(wbuf + s * kWBlock);
 #pragma unroll
                     for (int kk = 0; kk < kBK / 16; ++kk)
-                        umma_bf16(acc0, desc_sw128(sa + kk * 32), desc_sw128(sb + kk * 32), idesc,
+                        umma_bf16(acc, desc_sw128(sa + kk * 32), desc_sw128(sb + kk * 32), idesc,
                                   (kb | kk) != 0 ? 1u : 0u);
                     umma_commit(smem_u32(&wempty[s]));
                     ++wc;
@@ -933,42 +941,37 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
             };
             // 128 rows of a weight gradient: D's columns 128 half .. + 127 by
             // H's 256 columns, over the CTA's 128 batch rows
-            auto grad = [&](const uint8_t* d, int half, const uint8_t* h) {
+            auto grad = [&](const uint8_t* d, int half, const uint8_t* h, uint32_t acc) {
                 if (!ok) return;
                 const uint32_t da = smem_u32(d + half * 2 * kABytes), hb = smem_u32(h);
 #pragma unroll
                 for (int k = 0; k < kBM / 16; ++k)
-                    umma_bf16(acc1, desc_mn_sw128(da + k * 2048), desc_mn_sw128(hb + k * 2048),
+                    umma_bf16(acc, desc_mn_sw128(da + k * 2048), desc_mn_sw128(hb + k * 2048),
                               idesc_mn, k != 0 ? 1u : 0u);
             };
             wait(&w1full);
             wait(&xready);
             if (ok) umma_bf16(acc0, desc_sw32(smem_u32(xs)), desc_sw32(smem_u32(w1s)), idesc, 0u);
             commit(0);
-            wait(&done[0]);
-            layer(bufp);
+            layer(bufp, acc1, 0);
             commit(1);
-            wait(&done[1]);
-            layer(bufq);
+            layer(bufq, acc0, 1);
             commit(2);
-            wait(&done[2]);
-            grad(bufp, 0, bufq);
+            layer(bufp, acc1, 2);
             commit(3);
-            layer(bufp);
+            grad(bufp, 0, bufq, acc0);
             commit(4);
-            wait(&done[3]);
-            grad(bufp, 1, bufq);
+            wait(&done[0]);
+            grad(bufp, 1, bufq, acc0);
             commit(5);
-            wait(&done[4]);
-            layer(bufq);
+            layer(bufq, acc0, 3);
             commit(6);
-            wait(&done[5]);
-            grad(bufq, 0, bufp);
+            grad(bufq, 0, bufp, acc1);
             commit(7);
-            wait(&done[6]);
-            grad(bufq, 1, bufp);
+            wait(&done[1]);
+            grad(bufq, 1, bufp, acc1);
             commit(8);
-            wait(&done[7]);
+            wait(&done[2]);
             for (int half = 0; ok && half < 2; ++half) {
                 const uint32_t da = smem_u32(bufq + half * 2 * kABytes), xb = smem_u32(xs);
 #pragma unroll
@@ -1029,20 +1032,28 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
         auto chunk = [&](uint4* x, int kb) {
             return x + (static_cast<size_t>(tile) * 32 + (col(kb) >> 3)) * kBM + r;
         };
-        // a hidden layer's backward epilogue: acc0 and the stored z -> dz in buf
-        auto backward = [&](uint4* z_in, uint8_t* buf, uint4* d_out) {
-#pragma unroll 1
+        // a hidden layer's backward epilogue: acc and the stored z -> dz in
+        // buf, handed over per block where `bars` is not null
+        auto backward = [&](uint32_t acc, uint4* z_in, uint8_t* buf, uint4* d_out, uint64_t* bars) {
+            uint4 raw[4][2];  // every block's z in flight at once
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb) {
+                raw[kb][0] = chunk(z_in, kb)[0];
+                raw[kb][1] = chunk(z_in, kb)[kBM];
+            }
+#pragma unroll
             for (int kb = 0; kb < 4; ++kb) {
                 const int c = col(kb);
                 float v[16], z[16];
-                load16_bf16(chunk(z_in, kb), kBM, z);
-                acc16(acc0, c, v);
+                load16_bf16(raw[kb], 1, z);
+                acc16(acc, c, v);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                     const float s = sigmoidf_(z[j]);
                     v[j] = v[j] * s * (1.0f + z[j] * (1.0f - s));
                 }
                 store_h16_sw128(buf, r, c, v);
+                if (bars) arrive(bars + kb);
                 store16_bf16(chunk(d_out, kb), kBM, v);
             }
         };
@@ -1075,7 +1086,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
             for (int kb = 0; kb < 4; ++kb) {
                 const int c = col(kb);
                 float v[16], z[16];
-                acc16(acc0, c, v);
+                acc16(l == 0 ? acc0 : acc1, c, v);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                     float hz, t;
@@ -1083,10 +1094,10 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
                     z[j] = 2.0f * hz;  // exact: the pre-activation acc + bias
                 }
                 store_h16_sw128(buf, r, c, v);
+                arrive(&blk[l][kb]);
                 store16_bf16(chunk(z_out, kb), kBM, z);
                 if (l == 0) store16_bf16(chunk(a.h1, kb), kBM, v);
             }
-            arrive(&done[l]);
         }
         // head: partial chains per column group, y, dy; then dz3
         wait(&full[2]);
@@ -1129,45 +1140,47 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
                     v[j] = dy * sw4[c + j] * s * (1.0f + z * (1.0f - s));
                 }
                 store_h16_sw128(bufp, r, c, v);
+                arrive(&blk[2][kb]);
                 store16_bf16(chunk(a.dz3, kb), kBM, v);
                 store16_bf16(chunk(a.h3, kb), kBM, h);
             }
-            arrive(&done[2]);
-        }
-        wait(&full[3]);
-        if (ok) {
-            slab_out(acc1, a.dw3, 0);
-            arrive(&done[3]);
         }
         wait(&full[4]);
-        wait(&full[5]);
         if (ok) {
-            backward(a.z2, bufq, a.dz2);
+            slab_out(acc0, a.dw3, 0);
+            arrive(&done[0]);
+        }
+        wait(&full[3]);
+        wait(&full[5]);  // every reader of P and Q is done
+        if (ok) {
             // this thread's own copy of H1, back into P
+            uint4 h[4][2];
 #pragma unroll
             for (int kb = 0; kb < 4; ++kb) {
-                const int c = col(kb);
-                const uint4* src = chunk(a.h1, kb);
+                h[kb][0] = chunk(a.h1, kb)[0];
+                h[kb][1] = chunk(a.h1, kb)[kBM];
+            }
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb) {
+                const int c = col(kb), c0 = (c & 63) >> 3;
                 uint8_t* d = bufp + (c >> 6) * kABytes + r * 128;
-                const int c0 = (c & 63) >> 3;
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
-                    *reinterpret_cast<uint4*>(d + (((c0 + i) ^ (r & 7)) << 4)) = src[i * kBM];
+                    *reinterpret_cast<uint4*>(d + (((c0 + i) ^ (r & 7)) << 4)) = h[kb][i];
             }
-            arrive(&done[4]);
-            slab_out(acc1, a.dw3, 1);
-            arrive(&done[5]);
+            slab_out(acc0, a.dw3, 1);
+            backward(acc1, a.z2, bufq, a.dz2, blk[3]);
         }
         wait(&full[7]);
         if (ok) {
             slab_out(acc1, a.dw2, 0);
-            arrive(&done[6]);
+            arrive(&done[1]);
         }
         wait(&full[6]);
         wait(&full[8]);
         if (ok) {
-            backward(a.z1, bufq, a.dz1);
-            arrive(&done[7]);
+            backward(acc0, a.z1, bufq, a.dz1, nullptr);
+            arrive(&done[2]);
             slab_out(acc1, a.dw2, 1);
         }
         wait(&full[9]);
