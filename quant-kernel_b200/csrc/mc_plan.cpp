@@ -35,6 +35,12 @@ constexpr double kEps = 1e-12;
 constexpr int64_t kMaxTilesPerOption = 4096;
 constexpr int64_t kTerminalItersPerThread = 4;
 constexpr int64_t kMinTerminalTiles = 32;
+// Two CTAs on each of 148 SMs.  One Heston option at 100 steps: 10 tiles of two
+// pairs a thread 40.3 us a call, of one 35.8; 160 tiles 46.0 and 44.7; at 500
+// two pairs win, 62.9 against 65.8 (Euler, four units a thread: 39.8 and 32.6,
+// 45.3 and 41.3, 60.2 and 70.7 with one).
+constexpr int64_t kSmallBatchTiles = 296;
+constexpr int32_t kHostResultOptions = 64;
 
 double nan_value() { return std::numeric_limits<double>::quiet_NaN(); }
 
@@ -416,20 +422,11 @@ cudaError_t Plan::release() {
     drop_graph();
     if (device_ >= 0) {
         DeviceGuard g(device_);
-        d_opts_.release();
-        d_tile_begin_.release();
+        d_in_.release();
         d_partials_.release();
-        d_price_.release();
-        d_se_.release();
-        d_counter_.release();
-        d_out_index_.release();
-        h_out_index_.release();
-        d_groups_.release();
-        h_groups_.release();
-        h_opts_.release();
-        h_tile_begin_.release();
-        h_price_.release();
-        h_se_.release();
+        d_res_.release();
+        h_in_.release();
+        h_res_.release();
         if (ev0_) cudaEventDestroy(ev0_);
         if (ev1_) cudaEventDestroy(ev1_);
         if (stream_) cudaStreamDestroy(stream_);
@@ -502,7 +499,8 @@ cudaError_t Plan::build(const BatchInput& in, int32_t flags, std::string* err) {
     const std::string key = device_name(device_) + "|" + (persistent_ ? "persistent" : std::to_string(family_)) +
                             "|" + (anti_ ? "anti" : "plain");
     LaunchConfig tuned;
-    if (tuned_config(key, &tuned)) {
+    const bool tuned_shape = tuned_config(key, &tuned);
+    if (tuned_shape) {
         cfg_.block = tuned.block;
         // a multi-family plan takes the tuned mode unless the caller asked
         // for the persistent kernel explicitly
@@ -511,6 +509,13 @@ cudaError_t Plan::build(const BatchInput& in, int32_t flags, std::string* err) {
         if (persistent_ && cfg_.upt > 0) cfg_.upt = kUptPersistent;
         cfg_.su = (!persistent_ && step_unroll2_compiled(family_, cfg_.upt)) ? tuned.su : 1;
     }
+    // A batch too small to fill the chip runs its paths on more threads
+    if (!persistent_ && !tuned_shape && !(flags & (kFlagStepUnroll2 | kFlagAutotune)))
+        cfg_.upt = small_batch_upt(cfg_, family_);
+    // Two 8-byte stores an option over PCIe against a copy's launch: a small
+    // batch's results go straight to the pinned buffer (one quote, with a
+    // single upload in place of three operations: 45 -> 25 us in the library)
+    host_results_ = (flags & kFlagOneShot) && in.n <= kHostResultOptions;
     // QK_PLAN_STEP_UNROLL2: two step blocks per loop iteration where compiled
     if ((flags & kFlagStepUnroll2) && !persistent_ && step_unroll2_compiled(family_, cfg_.upt))
         cfg_.su = 2;
@@ -537,6 +542,23 @@ static int family_rank(int fam) {
         case kFamVr: return 3;
         default: return 4;  // terminal
     }
+}
+
+// Units per thread for a stepwise single-family batch: the family's own while
+// that makes at least kSmallBatchTiles tiles, else halved (and halved again),
+// which spreads the same paths over more warps.  A path's normals and
+// arithmetic do not change, and tile sums are double-double.
+int Plan::small_batch_upt(const LaunchConfig& cfg, int family) const {
+    if (!family_is_stepwise(family)) return cfg.upt;
+    int upt = cfg.upt;
+    for (; upt > 1; upt /= 2) {
+        int64_t tiles = 0;
+        for (const McOption& o : opts_) {
+            if (o.mode == kModeSimulate) tiles += (o.units + cfg.block * upt - 1) / (cfg.block * upt);
+            if (tiles >= kSmallBatchTiles) return upt;
+        }
+    }
+    return upt;
 }
 
 cudaError_t Plan::layout_tiles(const LaunchConfig& cfg) {
@@ -591,36 +613,35 @@ cudaError_t Plan::layout_tiles(const LaunchConfig& cfg) {
     }
 
     cudaError_t e;
-    const size_t opt_bytes = sizeof(McOption) * (size_t)std::max(n, 1);
+    auto align = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t tb_bytes = sizeof(int64_t) * ((size_t)n + 1);
-    if ((e = d_opts_.ensure(opt_bytes)) != cudaSuccess) return e;
-    if ((e = d_tile_begin_.ensure(tb_bytes)) != cudaSuccess) return e;
-    if ((e = d_partials_.ensure(sizeof(TilePartial) * (size_t)std::max<int64_t>(total, 1))) != cudaSuccess) return e;
-    if ((e = d_price_.ensure(sizeof(double) * (size_t)std::max(n, 1))) != cudaSuccess) return e;
-    if ((e = d_se_.ensure(sizeof(double) * (size_t)std::max(n, 1))) != cudaSuccess) return e;
-    if ((e = d_counter_.ensure(sizeof(unsigned long long))) != cudaSuccess) return e;
-    if ((e = h_opts_.ensure(opt_bytes)) != cudaSuccess) return e;
-    if ((e = h_tile_begin_.ensure(tb_bytes)) != cudaSuccess) return e;
-    const size_t ix_bytes = sizeof(int32_t) * (size_t)std::max(n, 1);
+    in_.tile_begin = align(sizeof(McOption) * (size_t)std::max(n, 1));
+    in_.counter = align(in_.tile_begin + tb_bytes);
+    in_.bytes = in_.counter + sizeof(unsigned long long);
     if (persistent_) {
-        if ((e = d_out_index_.ensure(ix_bytes)) != cudaSuccess) return e;
-        if ((e = h_out_index_.ensure(ix_bytes)) != cudaSuccess) return e;
-        if ((e = d_groups_.ensure(sizeof(GroupTable))) != cudaSuccess) return e;
-        if ((e = h_groups_.ensure(sizeof(GroupTable))) != cudaSuccess) return e;
+        in_.groups = align(in_.bytes);
+        in_.out_index = align(in_.groups + sizeof(GroupTable));
+        in_.bytes = in_.out_index + sizeof(int32_t) * (size_t)n;
     }
-    // The previous upload from these staging buffers may still be in flight.
-    if ((e = cudaStreamSynchronize(stream_)) != cudaSuccess) return e;
-    McOption* h_rec = static_cast<McOption*>(h_opts_.p);
+    const size_t res_bytes = 2 * sizeof(double) * (size_t)std::max(n, 1);
+    if ((e = d_in_.ensure(in_.bytes)) != cudaSuccess) return e;
+    if ((e = d_partials_.ensure(sizeof(TilePartial) * (size_t)std::max<int64_t>(total, 1))) != cudaSuccess) return e;
+    if ((e = d_res_.ensure(res_bytes)) != cudaSuccess) return e;
+    // The previous upload from this staging buffer may still be in flight.
+    if (upload_pending_ && (e = cudaStreamSynchronize(stream_)) != cudaSuccess) return e;
+    upload_pending_ = false;
+    if ((e = h_in_.ensure(in_.bytes)) != cudaSuccess) return e;
+    if ((e = h_res_.ensure(res_bytes)) != cudaSuccess) return e;
+    char* h = static_cast<char*>(h_in_.p);
+    McOption* h_rec = reinterpret_cast<McOption*>(h);
     for (int32_t k = 0; k < n; ++k) h_rec[k] = opts_[(size_t)order_[(size_t)k]];
-    std::memcpy(h_tile_begin_.p, begin.data(), tb_bytes);
+    std::memcpy(h + in_.tile_begin, begin.data(), tb_bytes);
+    std::memset(h + in_.counter, 0, sizeof(unsigned long long));
     if (persistent_) {
-        std::memcpy(h_out_index_.p, order_.data(), sizeof(int32_t) * (size_t)n);
-        if ((e = cudaMemcpyAsync(d_out_index_.p, h_out_index_.p, sizeof(int32_t) * (size_t)n,
-                                 cudaMemcpyHostToDevice, stream_)) != cudaSuccess)
-            return e;
+        std::memcpy(h + in_.out_index, order_.data(), sizeof(int32_t) * (size_t)n);
         // the persistent kernel's group table (at most 2 groups per family:
         // antithetic and plain; constant records carry no tiles)
-        GroupTable* gt = static_cast<GroupTable*>(h_groups_.p);
+        GroupTable* gt = reinterpret_cast<GroupTable*>(h + in_.groups);
         std::memset(gt, 0, sizeof(GroupTable));
         if (groups_.size() > (size_t)kMaxGroups) return cudaErrorInvalidConfiguration;
         gt->count = (int32_t)groups_.size();
@@ -630,14 +651,9 @@ cudaError_t Plan::layout_tiles(const LaunchConfig& cfg) {
             gt->opt_hi[k] = groups_[k].opt_hi;
             gt->tile_hi[k] = groups_[k].tile_hi;
         }
-        if ((e = cudaMemcpyAsync(d_groups_.p, h_groups_.p, sizeof(GroupTable),
-                                 cudaMemcpyHostToDevice, stream_)) != cudaSuccess)
-            return e;
     }
-    if ((e = cudaMemcpyAsync(d_opts_.p, h_opts_.p, sizeof(McOption) * (size_t)n, cudaMemcpyHostToDevice, stream_)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(d_tile_begin_.p, h_tile_begin_.p, tb_bytes, cudaMemcpyHostToDevice, stream_)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(d_counter_.p, 0, sizeof(unsigned long long), stream_)) != cudaSuccess) return e;
-    counter_ready_ = true;
+    upload_pending_ = true;
+    if ((e = cudaMemcpyAsync(d_in_.p, h_in_.p, in_.bytes, cudaMemcpyHostToDevice, stream_)) != cudaSuccess) return e;
     if (persistent_ && cfg.upt == kUptPersistent) {
         max_ctas_ = max_resident_ctas(-1, cfg.block, 0, device_);
         if (max_ctas_ <= 0) return cudaErrorInvalidConfiguration;
@@ -651,19 +667,19 @@ cudaError_t Plan::layout_tiles(const LaunchConfig& cfg) {
 cudaError_t Plan::launch_all(cudaStream_t st, bool timing) {
     if (cudaError_t fe = injected_fault(kFaultLaunch)) return fe;
     SimArgs a;
-    a.opts = static_cast<const McOption*>(d_opts_.p);
-    a.tile_begin = static_cast<const int64_t*>(d_tile_begin_.p);
+    a.opts = d_records();
+    a.tile_begin = d_tile_begin();
     a.n = n_;
     a.n_tiles = n_tiles_;
     a.partials = static_cast<TilePartial*>(d_partials_.p);
     a.max_ctas = max_ctas_;
-    unsigned long long* counter = static_cast<unsigned long long*>(d_counter_.p);
+    unsigned long long* counter = d_at<unsigned long long>(in_.counter);
     cudaError_t e = cudaSuccess;
     if (timing && (e = cudaEventRecord(ev0_, st)) != cudaSuccess) return e;
     const bool use_counter = persistent_ && cfg_.upt == kUptPersistent;
     if (n_tiles_ > 0) {
         if (use_counter) {
-            e = launch_persistent(cfg_.block, a, static_cast<const GroupTable*>(d_groups_.p),
+            e = launch_persistent(cfg_.block, a, d_at<const GroupTable>(in_.groups),
                                   counter, st);
         } else if (persistent_) {
             // one grid per (family, antithetic) group, back to back
@@ -686,8 +702,8 @@ cudaError_t Plan::launch_all(cudaStream_t st, bool timing) {
     if (timing && (e = cudaEventRecord(ev1_, st)) != cudaSuccess) return e;
     // persistent plans hold the records in work order; the finalize kernel
     // scatters results back to the caller's order
-    const int32_t* out_index = persistent_ ? static_cast<const int32_t*>(d_out_index_.p) : nullptr;
-    return launch_finalize(a.opts, n_, a.partials, d_price(), d_se(), out_index,
+    double* out = static_cast<double*>(host_results_ ? h_res_.p : d_res_.p);
+    return launch_finalize(a.opts, n_, a.partials, out, out + n_, d_out_index(),
                            use_counter ? counter : nullptr, st);
 }
 
@@ -753,8 +769,8 @@ cudaError_t Plan::order_after_upload(cudaStream_t st) {
 cudaError_t Plan::launch_tiles(cudaStream_t st, int64_t lo, int64_t hi, bool timing) {
     if (cudaError_t fe = injected_fault(kFaultLaunch)) return fe;
     SimArgs a;
-    a.opts = static_cast<const McOption*>(d_opts_.p);
-    a.tile_begin = static_cast<const int64_t*>(d_tile_begin_.p);
+    a.opts = d_records();
+    a.tile_begin = d_tile_begin();
     a.n = n_;
     a.partials = static_cast<TilePartial*>(d_partials_.p);
     a.max_ctas = std::numeric_limits<int32_t>::max();
@@ -785,10 +801,8 @@ cudaError_t Plan::launch_tiles(cudaStream_t st, int64_t lo, int64_t hi, bool tim
 }
 
 cudaError_t Plan::launch_finalize_all(cudaStream_t st) {
-    const int32_t* out_index = persistent_ ? static_cast<const int32_t*>(d_out_index_.p) : nullptr;
-    return launch_finalize(static_cast<const McOption*>(d_opts_.p), n_,
-                           static_cast<const TilePartial*>(d_partials_.p), d_price(), d_se(),
-                           out_index, nullptr, st);
+    return launch_finalize(d_records(), n_, static_cast<const TilePartial*>(d_partials_.p), d_price(),
+                           d_se(), d_out_index(), nullptr, st);
 }
 
 cudaError_t Plan::capture_graph() {
@@ -835,13 +849,14 @@ cudaError_t Plan::results(double* out_price, double* out_se) {
     cudaStream_t st = last_stream_ ? last_stream_ : stream_;
     const size_t bytes = sizeof(double) * (size_t)n_;
     cudaError_t e;
-    if ((e = h_price_.ensure(bytes)) != cudaSuccess) return e;
-    if (out_se && (e = h_se_.ensure(bytes)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(h_price_.p, d_price_.p, bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
-    if (out_se && (e = cudaMemcpyAsync(h_se_.p, d_se_.p, bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+    if (!host_results_ && (e = cudaMemcpyAsync(h_res_.p, d_res_.p, out_se ? 2 * bytes : bytes,
+                                               cudaMemcpyDeviceToHost, st)) != cudaSuccess)
+        return e;
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
-    std::memcpy(out_price, h_price_.p, bytes);
-    if (out_se) std::memcpy(out_se, h_se_.p, bytes);
+    upload_pending_ = false;  // the executes waited for it
+    const double* res = static_cast<const double*>(h_res_.p);
+    std::memcpy(out_price, res, bytes);
+    if (out_se) std::memcpy(out_se, res + n_, bytes);
     if (flags_ & kFlagTiming) {
         float ms = 0.0f;
         if (cudaEventElapsedTime(&ms, ev0_, ev1_) == cudaSuccess) last_ms_ = ms;

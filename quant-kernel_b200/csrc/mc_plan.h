@@ -36,6 +36,8 @@ enum : int32_t {
     kFlagAutotune = 0x10,
     kFlagFamilyGrids = 0x20,
     kFlagStepUnroll2 = 0x40,
+    // internal: built, executed and read once (the one-shot batch calls)
+    kFlagOneShot = 0x10000,
 };
 
 // Grow-only device / pinned host allocations.
@@ -94,8 +96,8 @@ public:
     int step_unroll() const { return cfg_.upt > 0 ? cfg_.su : 1; }
     int ctas() const { return max_ctas_; }
     bool persistent() const { return persistent_; }
-    double* d_price() const { return static_cast<double*>(d_price_.p); }
-    double* d_se() const { return static_cast<double*>(d_se_.p); }
+    double* d_price() const { return static_cast<double*>(d_res_.p); }
+    double* d_se() const { return d_price() + n_; }
     int device() const { return device_; }
     TilePartial* d_partials() const { return static_cast<TilePartial*>(d_partials_.p); }
     cudaStream_t stream() const { return stream_; }
@@ -116,6 +118,7 @@ public:
 
 private:
     cudaError_t ensure_stream();
+    int small_batch_upt(const LaunchConfig& cfg, int family) const;
     cudaError_t layout_tiles(const LaunchConfig& cfg);  // tile geometry + upload
     cudaError_t launch_all(cudaStream_t st, bool timing);
     cudaError_t autotune();
@@ -135,7 +138,8 @@ private:
     LaunchConfig cfg_;
     int max_ctas_ = 0;
     double last_ms_ = 0.0;
-    bool counter_ready_ = false;
+    bool upload_pending_ = false;  // an upload from h_in_ that nothing has waited for
+    bool host_results_ = false;    // finalize writes h_res_ itself
 
     std::vector<McOption> opts_;       // host copy (units/tiles filled per layout)
     std::vector<int32_t> order_;       // device record k is option order_[k]
@@ -148,9 +152,22 @@ private:
     std::vector<Group> groups_;        // filled for multi-family plans
     std::vector<int64_t> shard_bounds_;  // cached partition (shard_world_ ranks)
     int shard_world_ = 0;
-    DevBuf d_opts_, d_tile_begin_, d_partials_, d_price_, d_se_, d_counter_, d_out_index_,
-        d_groups_;
-    PinnedBuf h_opts_, h_tile_begin_, h_price_, h_se_, h_out_index_, h_groups_;
+    // One upload: records, tile offsets, work counter (zero) and, for multi-
+    // family plans, the group table and the caller's order, at fixed offsets.
+    struct InLayout {
+        size_t tile_begin, counter, groups, out_index, bytes;
+    };
+    InLayout in_{};
+    template <class T>
+    T* d_at(size_t off) const { return reinterpret_cast<T*>(static_cast<char*>(d_in_.p) + off); }
+    const McOption* d_records() const { return d_at<const McOption>(0); }
+    const int64_t* d_tile_begin() const { return d_at<const int64_t>(in_.tile_begin); }
+    const int32_t* d_out_index() const {
+        return persistent_ ? d_at<const int32_t>(in_.out_index) : nullptr;
+    }
+    // results: n prices, then n standard errors
+    DevBuf d_in_, d_partials_, d_res_;
+    PinnedBuf h_in_, h_res_;
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t graph_exec_ = nullptr;

@@ -54,7 +54,7 @@ int32_t run_batch(const qkb::BatchInput& in, int32_t flags, double* out_prices, 
     if (e != cudaSuccess) return fail_cuda(e, where);
     qkb::Plan* plan = qkb::thread_scratch_plan(dev);
     std::string err;
-    if ((e = plan->build(in, flags, &err)) != cudaSuccess) return fail_cuda(e, where);
+    if ((e = plan->build(in, flags | qkb::kFlagOneShot, &err)) != cudaSuccess) return fail_cuda(e, where);
     if ((e = plan->execute(nullptr)) != cudaSuccess) return fail_cuda(e, where);
     if ((e = plan->results(out_prices, out_se)) != cudaSuccess) return fail_cuda(e, where);
     return QK_OK;

@@ -17,10 +17,7 @@ import ctypes as ct
 import numpy as np
 
 from ._abi import QK_OK
-from .engine import QuantKernel
-
-PD = ct.POINTER(ct.c_double)
-PI32 = ct.POINTER(ct.c_int32)
+from .engine import QuantKernel, _ptr
 
 FEATURES = ("S/K", "T", "r", "q", "v0", "kappa", "theta", "sigma", "rho")
 N_PARAMS = 134401
@@ -30,10 +27,6 @@ N_PARAMS = 134401
 # kappa in [0.5, 5], vol of vol in [0.1, 1], rho in [-0.9, 0].
 HESTON_BOX_LO = np.array([100.0 / 130.0, 0.25, 0.0, 0.0, 0.01, 0.5, 0.01, 0.1, -0.9])
 HESTON_BOX_HI = np.array([100.0 / 70.0, 2.0, 0.05, 0.0, 0.09, 5.0, 0.09, 1.0, 0.0])
-
-
-def _pd(a):
-    return a.ctypes.data_as(PD)
 
 
 def features_of(spot, strike, t, r, q, v0, kappa, theta, sigma, rho):
@@ -64,7 +57,7 @@ class HestonSurrogate:
         self.box_lo = np.ascontiguousarray(box_lo, np.float64)
         self.box_hi = np.ascontiguousarray(box_hi, np.float64)
         self._h = ct.c_void_p()
-        self._check(self.lib.qk_sur_heston_create(_pd(self.box_lo), _pd(self.box_hi), int(seed),
+        self._check(self.lib.qk_sur_heston_create(_ptr(self.box_lo), _ptr(self.box_hi), int(seed),
                                                   ct.byref(self._h)), "create")
 
     def _check(self, rc, what):
@@ -75,18 +68,18 @@ class HestonSurrogate:
         f = np.ascontiguousarray(features, np.float64)
         t = np.ascontiguousarray(target, np.float64)
         assert f.ndim == 2 and f.shape[1] == 9 and t.shape == (f.shape[0],)
-        self._check(self.lib.qk_sur_heston_set_dataset(self._h, _pd(f), _pd(t), f.shape[0]), "set_dataset")
+        self._check(self.lib.qk_sur_heston_set_dataset(self._h, _ptr(f), _ptr(t), f.shape[0]), "set_dataset")
 
     def train(self, epochs, batch=8192, lr=1e-3, shuffle_seed=0):
         losses = np.empty(epochs)
         self._check(self.lib.qk_sur_heston_train(self._h, int(epochs), int(batch), float(lr),
-                                                 int(shuffle_seed), _pd(losses)), "train")
+                                                 int(shuffle_seed), _ptr(losses)), "train")
         return losses
 
     def predict(self, features):
         f = np.ascontiguousarray(features, np.float64)
         out = np.empty(f.shape[0])
-        self._check(self.lib.qk_sur_heston_predict(self._h, _pd(f), f.shape[0], _pd(out)), "predict")
+        self._check(self.lib.qk_sur_heston_predict(self._h, _ptr(f), f.shape[0], _ptr(out)), "predict")
         return out
 
     def predict_device(self, x_rows_ptr, base_ptr, n, y_ptr, stream=0, layered=False):
@@ -113,7 +106,7 @@ class HestonSurrogate:
         f = np.ascontiguousarray(features, np.float64)
         out = np.empty((f.shape[0], 64), np.uint16)
         base = np.empty(f.shape[0], np.float32)
-        self._check(self.lib.qk_sur_heston_features(self._h, _pd(f), f.shape[0],
+        self._check(self.lib.qk_sur_heston_features(self._h, _ptr(f), f.shape[0],
                                                     out.ctypes.data_as(ct.c_void_p),
                                                     base.ctypes.data_as(ct.c_void_p)), "features")
         return out, base
@@ -127,19 +120,19 @@ class HestonSurrogate:
         t = np.ascontiguousarray(target, np.float64)
         g = np.empty(N_PARAMS)
         loss = ct.c_double()
-        self._check(self.lib.qk_sur_heston_gradients(self._h, _pd(f), _pd(t), f.shape[0], _pd(g),
+        self._check(self.lib.qk_sur_heston_gradients(self._h, _ptr(f), _ptr(t), f.shape[0], _ptr(g),
                                                      ct.byref(loss)), "gradients")
         return loss.value, g
 
     def parameters(self):
         p = np.empty(N_PARAMS)
-        self._check(self.lib.qk_sur_heston_parameters(self._h, _pd(p)), "parameters")
+        self._check(self.lib.qk_sur_heston_parameters(self._h, _ptr(p)), "parameters")
         return p
 
     def set_parameters(self, p):
         p = np.ascontiguousarray(p, np.float64)
         assert p.shape == (N_PARAMS,)
-        self._check(self.lib.qk_sur_heston_set_parameters(self._h, _pd(p)), "set_parameters")
+        self._check(self.lib.qk_sur_heston_set_parameters(self._h, _ptr(p)), "set_parameters")
 
     def save(self, path):
         self._check(self.lib.qk_sur_heston_save(self._h, str(path).encode()), "save")
@@ -156,8 +149,8 @@ class HestonSurrogate:
         out = np.empty(n)
         src = np.empty(n, np.int32)
         self._check(self.lib.qk_sur_heston_price_batch(
-            self._h, *[_pd(a) for a in arrs], ot.ctypes.data_as(PI32), n, int(fallback_paths),
-            int(fallback_steps), int(fallback_seed), _pd(out), src.ctypes.data_as(PI32)), "price_batch")
+            self._h, *[_ptr(a) for a in arrs], _ptr(ot), n, int(fallback_paths),
+            int(fallback_steps), int(fallback_seed), _ptr(out), _ptr(src)), "price_batch")
         return out, src
 
     def close(self):

@@ -1,0 +1,47 @@
+"""One-shot batches around the sizes where the plan changes: fewer units per
+thread while the tiles do not fill the chip, results written straight to the
+pinned buffer up to 64 options.  An option's price and standard error must not
+depend on the batch it is in (double-double sums: 1e-14 allows their final
+rounding only), and read-only or sliced columns must serve like owned ones.
+"""
+
+import numpy as np
+import pytest
+
+from quantkernel_b200 import workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def _batch(kind, n, paths):
+    if kind == "heston":
+        return workloads.heston(n, paths, 20, seed=4)
+    b = workloads.bsm_terminal(n, paths, seed=4)
+    if kind != "antithetic_variates":
+        b["steps"] = np.full(n, 20, np.int32)
+    return b
+
+
+@pytest.mark.parametrize("paths", (999, 4097))
+@pytest.mark.parametrize("kind", ("heston", "euler_maruyama", "milstein", "antithetic_variates"))
+def test_price_does_not_depend_on_the_batch(qk, kind, paths):
+    fn = getattr(qk, "heston_monte_carlo_price_se_batch" if kind == "heston" else kind + "_price_se_batch")
+    full = _batch(kind, 700, paths)
+    want = fn(**full)
+    for n in (1, 2, 36, 63, 64, 65, 150):
+        got = fn(**{k: v[:n] for k, v in full.items()})
+        for g, w in zip(got, want):
+            np.testing.assert_allclose(g, w[:n], rtol=1e-14, atol=0)
+
+
+def test_read_only_and_strided_columns(qk):
+    b = _batch("heston", 12, 1001)
+    want = qk.heston_monte_carlo_price_batch(**b)
+    odd = {}
+    for i, (k, v) in enumerate(b.items()):
+        if i % 2:
+            v = np.repeat(v, 2)[::2]
+        v = v.copy() if i % 3 else v
+        v.flags.writeable = bool(i % 3)
+        odd[k] = v
+    assert np.array_equal(qk.heston_monte_carlo_price_batch(**odd), want)
