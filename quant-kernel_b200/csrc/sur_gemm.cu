@@ -41,6 +41,27 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
+// One lane of a converged warp.  tcgen05 and TMA instructions take their
+// operands from uniform registers: under this predicate the compiler knows
+// that one lane is active.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+    return e != 0;
+}
+
+// Whether the phase has completed, without waiting.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Bounded wait: false after kSpinLimit polls (each poll may suspend briefly).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     for (uint32_t i = 0; i < kSpinLimit; ++i)
@@ -354,46 +375,53 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 // ----------------------------------------------------------------------------
 // Fused MLP inference.  One persistent CTA per SM walks its 128-row tiles two
 // at a time, ping-pong: tile slot s (0, 1) owns TMEM accumulator s (256 fp32
-// columns) and a 64 KiB shared buffer that holds the slot's input rows, then
-// layer 1's and layer 2's activations.  While the epilogue warps work on one
-// slot's layer, the tensor core computes the other slot's, so neither waits
-// for the other's tail.  Four warp roles:
+// columns), a 64 KiB shared buffer of activations and a 4 KiB one of input
+// rows.  While the epilogue warps work on one slot's layer, the tensor core
+// computes the other slot's.  Four warp roles:
 //   warp 16 (one lane)  weight producer: W1's first 16 columns once (8 KiB,
 //                       resident), then the 32 KiB k-blocks of W2 and W3 in
 //                       the order the MMA issuer takes them (per tile pair:
 //                       W2[0..3] for A, for B, W3[0..3] for A, for B) through
 //                       a 2-slot ring;
-//   warp 17 (one lane)  MMA issuer: per tile pair, layer by layer, tile A's
-//                       then tile B's: layer 1 (one K = 16 MMA: the 9
-//                       features and their zero padding; the rows' columns
-//                       16..63 are zeros too and would add exact zeros) once
-//                       the slot's input rows have landed and its previous
-//                       tile's head has read the accumulator, layers 2 and 3
-//                       once the epilogue has written the slot's previous
-//                       layer;
+//   warp 17 (one lane)  MMA issuer: per tile pair A, B: layer 2 of A, of B,
+//                       layer 3 of A, of B, each once the epilogue has written
+//                       the slot's previous layer.  Layer 1 (one K = 16 MMA:
+//                       the 9 features and their zero padding; the rows'
+//                       columns 16..63 are zeros too and would add exact
+//                       zeros) of the next A goes in among the k-blocks of B's
+//                       layer 3, of the next B among those of A's layer 2, as
+//                       soon as the head has read the slot's accumulator;
 //   warp 18 (one lane)  input loader: a slot's next input rows (their first
-//                       16 columns, 32-byte swizzled: 4 KiB) once the MMAs
-//                       of its previous tile's layer 3 (the last reader of
-//                       the slot's buffer) have completed;
-//   warps 0-15          epilogue, in the MMA issuer's order: warp w reads TMEM
-//                       lanes 32 (w % 4) .. + 31 (its tile rows) and, in each
-//                       64-column block kb, columns 64 kb + 16 (w / 4) .. + 15;
-//                       bias + SiLU, BF16 into the slot's buffer in the
-//                       128-byte-swizzled K-major layout the next layer's MMA
-//                       reads as its A operand; the head sums partial chains
-//                       and writes the prices.
+//                       16 columns, 32-byte swizzled) once its previous tile's
+//                       layer 1 has read the buffer;
+//   warps 0-15          epilogue: layer 2 of A, of B, the head of A, layer 1
+//                       of the next A, the head of B, layer 1 of the next B;
+//                       warp w reads TMEM lanes 32 (w % 4) .. + 31 (its tile
+//                       rows) and, in each 64-column block kb, columns 64 kb +
+//                       16 (w / 4) .. + 15; bias + SiLU, BF16 into the slot's
+//                       buffer in the 128-byte-swizzled K-major layout the
+//                       next layer's MMA reads as its A operand; the head sums
+//                       partial chains and writes the prices.
 // Every hand-off is an mbarrier with a bounded wait (no CTA-wide barrier
 // inside the loop), so a timeout anywhere ends every role with an error code.
-// Barriers per slot: xfull (input rows landed), accfull (a layer's MMAs
-// complete: three phases per tile), hdone (all 16 epilogue warps finished a
-// layer of the slot: three phases per tile), pready (the head's partial sums,
-// one phase per tile).  Hazards, each closed by the chain: an accumulator is
-// rewritten only after hdone reports the epilogue read it; a buffer is
-// rewritten by the epilogue only after accfull reports that the MMAs which
-// read it completed, and by the input loader only after the slot's layer-3
-// accfull; the head's partial sums are double-buffered by slot.
+// Barriers per slot: xfull (input rows landed), xfree (layer 1 has read them),
+// accfull (a layer's MMAs complete: three phases per tile), hdone (all 16
+// epilogue warps finished a layer of the slot: three phases per tile), pready
+// (the head's partial sums, one phase per tile).  Hazards, each closed by the
+// chain: an accumulator is rewritten only after hdone reports the epilogue
+// read it; a buffer of activations is rewritten by the epilogue only after
+// accfull reports that the MMAs which read it completed; the head's partial
+// sums are double-buffered by slot.
 // The arithmetic and summation order are those of the layer-by-layer GEMMs
 // (kEpiFwd, kEpiLast), so the results are the same bits.
+//
+// Bound by the chain of a slot (epilogue, hand-off, MMAs) and the ring, whose
+// two blocks take 1.8k cycles to come round: 10.5k cycles a tile, 6.3k of them
+// in the epilogue, whose tanh needs 6.1k.  With layer 1 after both heads and
+// the issuing lane chosen by its number, a million rows took 355 us, now 335
+// (100,000: 42.1 with their features, now 40.4).  Pairs of CTAs that share the
+// weight blocks (cta_group::2) took 395: beside the faster MMAs the epilogue
+// slows from 2.1k to 3k cycles a layer.
 // ----------------------------------------------------------------------------
 constexpr int kIWSlots = 2;
 constexpr uint32_t kWBlock = 256 * kBK * 2;        // 32 KiB: 256 rows x 64 bf16
@@ -403,7 +431,7 @@ constexpr int kTileSlots = 2;
 // rows of 32 bytes, and W1's first 16 columns held resident for the launch.
 constexpr uint32_t kXBytes = kBM * 16 * 2;         // 4 KiB: 128 rows x 16 bf16
 constexpr uint32_t kW1Bytes = 256 * 16 * 2;        // 8 KiB: 256 rows x 16 bf16
-constexpr size_t kInferSmem = kTileSlots * kHBytes + kIWSlots * kWBlock + kW1Bytes + 1024;
+constexpr size_t kInferSmem = kTileSlots * (kHBytes + kXBytes) + kIWSlots * kWBlock + kW1Bytes + 1024;
 constexpr int kInferEpiWarps = 16;                 // 4 per TMEM lane quarter
 constexpr int kInferThreads = (kInferEpiWarps + 3) * 32;
 constexpr int kProducerWarp = kInferEpiWarps, kMmaWarp = kInferEpiWarps + 1,
@@ -447,11 +475,12 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
-    uint8_t* hbufs = smem;  // [kTileSlots][kHBytes]: a slot's input rows, then its activations
+    uint8_t* hbufs = smem;  // [kTileSlots][kHBytes]: a slot's activations
     uint8_t* wbuf = smem + kTileSlots * kHBytes;
     uint8_t* w1s = wbuf + kIWSlots * kWBlock;  // W1 [256][16], resident
+    uint8_t* xbufs = w1s + kW1Bytes;           // [kTileSlots][kXBytes]: a slot's input rows
     __shared__ __align__(8) uint64_t w1full;
-    __shared__ __align__(8) uint64_t xfull[kTileSlots], slotfree[kTileSlots], accfull[kTileSlots];
+    __shared__ __align__(8) uint64_t xfull[kTileSlots], xfree[kTileSlots], accfull[kTileSlots];
     __shared__ __align__(8) uint64_t hdone[kTileSlots], pready[kTileSlots];
     __shared__ __align__(8) uint64_t wfull[kIWSlots], wempty[kIWSlots], drain;
     __shared__ __align__(16) float sb1[kSurHidden], sb2[kSurHidden], sb3[kSurHidden], sw4[kSurHidden];
@@ -475,7 +504,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     if (tid == 0) {
         for (int s = 0; s < kTileSlots; ++s) {
             mbar_init(smem_u32(&xfull[s]), 1);
-            mbar_init(smem_u32(&slotfree[s]), 1);
+            mbar_init(smem_u32(&xfree[s]), 1);
             mbar_init(smem_u32(&accfull[s]), 1);
             mbar_init(smem_u32(&hdone[s]), kInferEpiWarps);
             mbar_init(smem_u32(&pready[s]), kInferEpiWarps);
@@ -509,9 +538,11 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     int last_round[kIWSlots] = {-1, -1};
     int64_t x_last[kTileSlots] = {-1, -1};
     bool w1_issued = false;
+    bool leader = false;  // this warp's elected lane
 
     if (warp == kProducerWarp) {
-        if (lane == 0) {
+        if (elect_one()) {
+            leader = true;
             uint32_t wl = 0;
             auto load_w = [&](const CUtensorMap* m, int kx) -> bool {
                 const uint32_t s = wl % kIWSlots, round = wl / kIWSlots;
@@ -543,26 +574,28 @@ __global__ void __launch_bounds__(kInferThreads, 1)
             }
         }
     } else if (warp == kXWarp) {
-        if (lane == 0) {
+        if (elect_one()) {
+            leader = true;
             for (int64_t i = 0; i < my_tiles; ++i) {
                 if (abort_flag) break;
                 const int s = static_cast<int>(i & 1);
                 const int64_t u = i >> 1;
-                // the slot's previous tile's layer-3 MMAs, the last readers of
-                // its buffer, have completed (one slotfree phase per tile)
-                if (u > 0 && !mbar_wait(smem_u32(&slotfree[s]), static_cast<uint32_t>((u - 1) & 1))) {
+                // layer 1 of the slot's previous tile, the buffer's reader, has
+                // completed (one xfree phase per tile)
+                if (u > 0 && !mbar_wait(smem_u32(&xfree[s]), static_cast<uint32_t>((u - 1) & 1))) {
                     fail(21);
                     break;
                 }
                 mbar_expect_tx(smem_u32(&xfull[s]), kXBytes);
                 const int64_t t = blockIdx.x + i * gridDim.x;
-                tma_load_2d(smem_u32(hbufs + s * kHBytes), &tx, 0, static_cast<int>(t * kBM),
+                tma_load_2d(smem_u32(xbufs + s * kXBytes), &tx, 0, static_cast<int>(t * kBM),
                             smem_u32(&xfull[s]));
                 x_last[s] = u;
             }
         }
     } else if (warp == kMmaWarp) {
-        if (lane == 0) {
+        if (elect_one()) {
+            leader = true;
             constexpr uint32_t idesc = idesc_bf16<256>();
             uint32_t wc = 0;
             // one k-block of W from the ring into accumulator acc
@@ -582,36 +615,49 @@ __global__ void __launch_bounds__(kInferThreads, 1)
             bool ok = my_tiles == 0 || mbar_wait(smem_u32(&w1full), 0u);
             if (!ok) fail(25);
             const uint64_t dw1 = desc_sw32(smem_u32(w1s));
-            for (int64_t i0 = 0; ok && i0 < my_tiles; i0 += 2) {
-                if (abort_flag) break;
-                const int nt = (my_tiles - i0) >= 2 ? 2 : 1;
-                const int64_t u = i0 >> 1;
-                for (int l = 0; ok && l < 3; ++l) {
-                    for (int s = 0; ok && s < nt; ++s) {
-                        const uint32_t acc = tmem + s * 256;
-                        const uint8_t* hb = hbufs + s * kHBytes;
-                        if (l == 0) {
-                            // the slot's input rows, and its previous tile's
-                            // head done reading the accumulator
-                            ok = mbar_wait(smem_u32(&xfull[s]), static_cast<uint32_t>(u & 1));
-                            if (ok && u > 0)
-                                ok = mbar_wait(smem_u32(&hdone[s]), static_cast<uint32_t>((3 * u - 1) & 1));
-                            fence_after();
-                            // K = 16: the input rows and the resident W1 slice
-                            if (ok) umma_bf16(acc, desc_sw32(smem_u32(hb)), dw1, idesc, 0u);
-                        } else {
-                            // layer l's activations written (and its
-                            // accumulator read) by every epilogue warp
-                            ok = mbar_wait(smem_u32(&hdone[s]), static_cast<uint32_t>((3 * u + l - 1) & 1));
-                            fence_after();
-                            for (int kb = 0; ok && kb < 4; ++kb)
-                                ok = mma_kblock(acc, smem_u32(hb + kb * kABytes), kb == 0);
-                        }
-                        if (!ok) break;
-                        umma_commit(smem_u32(&accfull[s]));
-                        if (l == 2) umma_commit(smem_u32(&slotfree[s]));
-                    }
+            // layer 1 of tile i, one K = 16 MMA, once its input rows have landed
+            // and the head of the slot's previous tile has read the accumulator;
+            // where wait is false only if both have happened
+            auto layer1 = [&](int64_t i, bool wait) -> bool {
+                const int s = static_cast<int>(i & 1);
+                const int64_t u = i >> 1;
+                const uint32_t xp = static_cast<uint32_t>(u & 1), hp = static_cast<uint32_t>((3 * u - 1) & 1);
+                if (wait) {
+                    ok = ok && mbar_wait(smem_u32(&xfull[s]), xp) && (u == 0 || mbar_wait(smem_u32(&hdone[s]), hp));
+                    if (!ok) return false;
+                } else if (!mbar_test(smem_u32(&xfull[s]), xp) || (u > 0 && !mbar_test(smem_u32(&hdone[s]), hp))) {
+                    return false;
                 }
+                fence_after();
+                umma_bf16(tmem + s * 256, desc_sw32(smem_u32(xbufs + s * kXBytes)), dw1, idesc, 0u);
+                umma_commit(smem_u32(&xfree[s]));
+                umma_commit(smem_u32(&accfull[s]));
+                return true;
+            };
+            // layer l (1, 2) of tile i, once every epilogue warp has written its
+            // activations and read its accumulator; layer 1 of tile `next` goes
+            // in between as soon as it can
+            auto layer = [&](int64_t i, int l, int64_t next) {
+                const int s = static_cast<int>(i & 1);
+                bool pending = next < my_tiles;
+                if (pending) pending = !layer1(next, false);
+                ok = ok && mbar_wait(smem_u32(&hdone[s]), static_cast<uint32_t>((3 * (i >> 1) + l - 1) & 1));
+                fence_after();
+                for (int kb = 0; ok && kb < 4; ++kb) {
+                    if (pending) pending = !layer1(next, false);
+                    ok = mma_kblock(tmem + s * 256, smem_u32(hbufs + s * kHBytes + kb * kABytes), kb == 0);
+                }
+                if (ok) umma_commit(smem_u32(&accfull[s]));
+                if (ok && pending) layer1(next, true);
+            };
+            if (ok && my_tiles > 0 && !layer1(0, true)) fail(24);
+            for (int64_t i = 0; ok && i < my_tiles; i += 2) {
+                if (abort_flag) break;
+                const bool two = i + 1 < my_tiles;
+                layer(i, 1, i + 1);
+                if (two) layer(i + 1, 1, my_tiles);
+                layer(i, 2, my_tiles);
+                if (two) layer(i + 1, 2, i + 2);
                 if (!ok) fail(24);
             }
         }
@@ -632,79 +678,99 @@ __global__ void __launch_bounds__(kInferThreads, 1)
         const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
         const float b4 = __ldg(a.b4);
         bool ok = true;
-        for (int64_t i0 = 0; ok && i0 < my_tiles; i0 += 2) {
-            const int nt = (my_tiles - i0) >= 2 ? 2 : 1;
-            const int64_t u = i0 >> 1;
-            for (int l = 0; ok && l < 3; ++l) {
-                for (int s = 0; ok && s < nt; ++s) {
-                    const uint32_t acc = tmem + s * 256 + lane_off;
-                    ok = warp_wait(smem_u32(&accfull[s]), static_cast<uint32_t>((3 * u + l) & 1));
-                    fence_after();
-                    if (!ok) {
-                        if (lane == 0) fail(26);
-                        break;
+        // layer 1 of the first two tiles, then pair by pair: layer 2 of A and
+        // of B, the head of A, layer 1 of the next A, the head of B, layer 1 of
+        // the next B (bit pairs of `kLayers`, bits of `kSlots`, lowest first)
+        constexpr uint32_t kLayers = 1u | 1u << 2 | 2u << 4 | 0u << 6 | 2u << 8 | 0u << 10;
+        constexpr uint32_t kSlots = 0u | 1u << 1 | 0u << 2 | 0u << 3 | 1u << 4 | 1u << 5;
+        for (int64_t i0 = -2; ok && i0 < my_tiles; i0 += 2) {
+            for (int e = 0; ok && e < 6; ++e) {
+                const int l = (kLayers >> (2 * e)) & 3, s = (kSlots >> e) & 1;
+                const int64_t i = i0 + s + (l == 0 ? 2 : 0);
+                if (i < 0 || i >= my_tiles) continue;
+                const int64_t u = i >> 1;
+                const uint32_t acc = tmem + s * 256 + lane_off;
+                ok = warp_wait(smem_u32(&accfull[s]), static_cast<uint32_t>((3 * u + l) & 1));
+                fence_after();
+                if (!ok) {
+                    if (lane == 0) fail(26);
+                    break;
+                }
+                if (l < 2) {
+                    const float* bias = l == 0 ? sb1 : sb2;
+                    uint8_t* hbuf = hbufs + s * kHBytes;
+#pragma unroll
+                    for (int kb = 0; kb < 4; ++kb) {
+                        const int col0 = kb * 64 + g * 16;
+                        uint32_t uu[16];
+                        tmem_ld16_async(acc + col0, uu);
+                        tmem_wait_ld();
+                        float v[16];
+#pragma unroll
+                        for (int j = 0; j < 16; j += 4) {
+                            const float4 b = *reinterpret_cast<const float4*>(bias + col0 + j);
+                            const float2 h0 = silu2_from_acc(
+                                make_float2(__uint_as_float(uu[j]), __uint_as_float(uu[j + 1])),
+                                make_float2(b.x, b.y));
+                            const float2 h1 = silu2_from_acc(
+                                make_float2(__uint_as_float(uu[j + 2]), __uint_as_float(uu[j + 3])),
+                                make_float2(b.z, b.w));
+                            v[j] = h0.x;
+                            v[j + 1] = h0.y;
+                            v[j + 2] = h1.x;
+                            v[j + 3] = h1.y;
+                        }
+                        store_h16_sw128(hbuf, r, col0, v);
                     }
-                    if (l < 2) {
-                        const float* bias = l == 0 ? sb1 : sb2;
-                        uint8_t* hbuf = hbufs + s * kHBytes;
+                    // the shared stores to the tensor core's (async) proxy,
+                    // the TMEM reads before the hand-off
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&hdone[s]));
+                } else {
+                    // head: this warp's chain over columns 64 kb + 16 g + j
+                    float p = 0.0f;
 #pragma unroll
-                        for (int kb = 0; kb < 4; ++kb) {
-                            const int col0 = kb * 64 + g * 16;
-                            uint32_t uu[16];
-                            tmem_ld16_async(acc + col0, uu);
-                            tmem_wait_ld();
-                            float v[16];
+                    for (int kb = 0; kb < 4; ++kb) {
+                        const int col0 = kb * 64 + g * 16;
+                        uint32_t uu[16];
+                        tmem_ld16_async(acc + col0, uu);
+                        tmem_wait_ld();
 #pragma unroll
-                            for (int j = 0; j < 16; j += 2) {
-                                const float2 h = silu2_from_acc(
-                                    make_float2(__uint_as_float(uu[j]), __uint_as_float(uu[j + 1])),
-                                    *reinterpret_cast<const float2*>(bias + col0 + j));
-                                v[j] = h.x;
-                                v[j + 1] = h.y;
-                            }
-                            store_h16_sw128(hbuf, r, col0, v);
+                        for (int j = 0; j < 16; j += 4) {
+                            const float4 b = *reinterpret_cast<const float4*>(sb3 + col0 + j);
+                            const float4 w = *reinterpret_cast<const float4*>(sw4 + col0 + j);
+                            const float2 h0 = silu2_from_acc(
+                                make_float2(__uint_as_float(uu[j]), __uint_as_float(uu[j + 1])),
+                                make_float2(b.x, b.y));
+                            const float2 h1 = silu2_from_acc(
+                                make_float2(__uint_as_float(uu[j + 2]), __uint_as_float(uu[j + 3])),
+                                make_float2(b.z, b.w));
+                            p = fmaf(h0.x, w.x, p);
+                            p = fmaf(h0.y, w.y, p);
+                            p = fmaf(h1.x, w.z, p);
+                            p = fmaf(h1.y, w.w, p);
                         }
-                        // the shared stores to the tensor core's (async) proxy,
-                        // the TMEM reads before the hand-off
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&hdone[s]));
-                    } else {
-                        // head: this warp's chain over columns 64 kb + 16 g + j
-                        float p = 0.0f;
-#pragma unroll
-                        for (int kb = 0; kb < 4; ++kb) {
-                            const int col0 = kb * 64 + g * 16;
-                            uint32_t uu[16];
-                            tmem_ld16_async(acc + col0, uu);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                float hz, t;
-                                const float h = silu_from_acc(__uint_as_float(uu[j]), sb3[col0 + j], hz, t);
-                                p = fmaf(h, sw4[col0 + j], p);
-                            }
+                    }
+                    // the accumulator is read: the slot's next tile may start
+                    // its layer 1
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&hdone[s]));
+                    part[s][g][r] = p;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&pready[s]));
+                    if (g == 0) {
+                        ok = warp_wait(smem_u32(&pready[s]), static_cast<uint32_t>(u & 1));
+                        if (!ok) {
+                            if (lane == 0) fail(27);
+                            break;
                         }
-                        // the accumulator is read: the slot's next tile may
-                        // start its layer 1
-                        fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&hdone[s]));
-                        part[s][g][r] = p;
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(smem_u32(&pready[s]));
-                        if (g == 0) {
-                            ok = warp_wait(smem_u32(&pready[s]), static_cast<uint32_t>(u & 1));
-                            if (!ok) {
-                                if (lane == 0) fail(27);
-                                break;
-                            }
-                            const float y =
-                                (((part[s][0][r] + part[s][1][r]) + part[s][2][r]) + part[s][3][r]) + b4;
-                            const int64_t row = (blockIdx.x + (i0 + s) * gridDim.x) * kBM + r;
-                            if (row < a.n) a.y[row] = a.base ? y + __ldg(a.base + row) : y;
-                        }
+                        const float y =
+                            (((part[s][0][r] + part[s][1][r]) + part[s][2][r]) + part[s][3][r]) + b4;
+                        const int64_t row = (blockIdx.x + i * gridDim.x) * kBM + r;
+                        if (row < a.n) a.y[row] = a.base ? y + __ldg(a.base + row) : y;
                     }
                 }
             }
@@ -717,14 +783,14 @@ __global__ void __launch_bounds__(kInferThreads, 1)
     fence_before();
     __syncthreads();
     if (abort_flag) {
-        if (warp == kProducerWarp && lane == 0) {
+        if (warp == kProducerWarp && leader) {
             for (int s = 0; s < kIWSlots; ++s)
                 if (last_round[s] >= 0) mbar_wait(smem_u32(&wfull[s]), last_round[s] & 1);
             if (w1_issued) mbar_wait(smem_u32(&w1full), 0u);
-        } else if (warp == kXWarp && lane == 0) {
+        } else if (warp == kXWarp && leader) {
             for (int s = 0; s < kTileSlots; ++s)
                 if (x_last[s] >= 0) mbar_wait(smem_u32(&xfull[s]), static_cast<uint32_t>(x_last[s] & 1));
-        } else if (warp == kMmaWarp && lane == 0) {
+        } else if (warp == kMmaWarp && leader) {
             umma_commit(smem_u32(&drain));
             mbar_wait(smem_u32(&drain), 0);
         }
@@ -885,9 +951,11 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     };
     int last_round[kIWSlots] = {-1, -1};
     bool w1_issued = false;
+    bool elected = false;
 
     if (warp == kTrainEpiWarps) {
-        if (lane == 0) {
+        if (elect_one()) {
+            elected = true;
             mbar_expect_tx(smem_u32(&w1full), kW1Bytes);
             tma_load_2d(smem_u32(w1s), &maps.w1, 0, 0, smem_u32(&w1full));
             w1_issued = true;
@@ -908,7 +976,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
             }
         }
     } else if (warp == kTrainEpiWarps + 1) {
-        if (lane == 0) {
+        if (elect_one()) {
+            elected = true;
             constexpr uint32_t idesc = idesc_bf16<256>(), idesc_mn = idesc | kIdescMn;
             constexpr uint32_t idesc_w1 = idesc_bf16<16>() | kIdescMn;
             const uint32_t acc0 = tmem, acc1 = tmem + 256;
@@ -1198,11 +1267,11 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     fence_before();
     __syncthreads();
     if (abort_flag) {
-        if (warp == kTrainEpiWarps && lane == 0) {
+        if (warp == kTrainEpiWarps && elected) {
             for (int s = 0; s < kIWSlots; ++s)
                 if (last_round[s] >= 0) mbar_wait(smem_u32(&wfull[s]), last_round[s] & 1);
             if (w1_issued) mbar_wait(smem_u32(&w1full), 0u);
-        } else if (warp == kTrainEpiWarps + 1 && lane == 0) {
+        } else if (warp == kTrainEpiWarps + 1 && elected) {
             umma_commit(smem_u32(&drain));
             mbar_wait(smem_u32(&drain), 0);
         }
