@@ -913,12 +913,6 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tile = blockIdx.x;
-    if (tid < kSurHidden) {
-        sb1[tid] = 0.5f * a.b1[tid];  // halved biases for silu_from_acc (exact)
-        sb2[tid] = 0.5f * a.b2[tid];
-        sb3[tid] = 0.5f * a.b3[tid];
-        sw4[tid] = a.w4[tid];
-    }
     if (tid == 0) {
         mbar_init(smem_u32(&w1full), 1);
         mbar_init(smem_u32(&xready), kTrainEpiWarps);
@@ -940,6 +934,15 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
                      "r"(512u)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    // what the previous kernel of the stream wrote is read from here on
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+    if (tid < kSurHidden) {
+        sb1[tid] = 0.5f * a.b1[tid];  // halved biases for silu_from_acc (exact)
+        sb2[tid] = 0.5f * a.b2[tid];
+        sb3[tid] = 0.5f * a.b3[tid];
+        sw4[tid] = a.w4[tid];
     }
     fence_before();
     __syncthreads();
@@ -1328,8 +1331,7 @@ cudaError_t launch_mlp_train(const TrainMaps& maps, const TrainArgs& a, cudaStre
     });
     if (attr_err != cudaSuccess) return attr_err;
     if (a.batch <= 0 || a.batch % kBM != 0) return cudaErrorInvalidValue;
-    mlp_train_kernel<<<a.batch / kBM, kTrainThreads, kTrainSmem, st>>>(maps, a);
-    return cudaGetLastError();
+    return launch_dependent(mlp_train_kernel, a.batch / kBM, kTrainThreads, kTrainSmem, st, maps, a);
 }
 
 bool make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,

@@ -60,6 +60,27 @@ struct InferArgs {
 // (make_tmap_bf16_k16: the 9 features and their zero padding; boxes 16 x 128
 // and 16 x 256, 32-byte swizzle); tw2, tw3: [256][256] (boxes 64 x 256).
 // ctas: persistent grid size (one CTA per SM).
+// Launches a kernel that may start while the previous one of the stream still
+// runs: it calls griddepcontrol.wait before it touches what that one writes.
+// A training step is two short kernels; with the set-up of each under the tail
+// of the other, an epoch of 182 steps of 384 rows takes 8.63 ms instead of
+// 9.25, one of 32 steps of 8192 rows 2.65 instead of 2.71.
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st,
+                             const A&... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 cudaError_t launch_mlp_infer(const CUtensorMap& tx, const CUtensorMap& tw1, const CUtensorMap& tw2,
                              const CUtensorMap& tw3, const InferArgs& a, int ctas, cudaStream_t st);
 

@@ -447,6 +447,9 @@ __device__ __forceinline__ void update_weights(const UpdateArgs& a, int e, uint4
 __global__ void __launch_bounds__(kUpdThreads) update_kernel(const UpdateArgs a) {
     extern __shared__ uint4 ring[];
     const int b = blockIdx.x;
+    // what the training pass wrote is read from here on
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
     if (b < kBiasBlocks) {
         update_columns(a, b);
     } else if (b == kBiasBlocks) {
@@ -705,9 +708,8 @@ cudaError_t SurModel::run_step(const StepLaunch& s, cudaStream_t st) {
     QK_TRY(attr_err);
     QK_TRY(launch_mlp_train(s.maps, s.train, st));
     constexpr int kQuads = kW1Quads + 2 * kWQuads;
-    update_kernel<<<kBiasBlocks + 1 + (kQuads + kUpdThreads - 1) / kUpdThreads, kUpdThreads, kUpdSmem, st>>>(
-        s.update);
-    return cudaGetLastError();
+    return launch_dependent(update_kernel, kBiasBlocks + 1 + (kQuads + kUpdThreads - 1) / kUpdThreads, kUpdThreads,
+                            kUpdSmem, st, s.update);
 }
 
 cudaError_t SurModel::train(int epochs, int batch, float lr0, uint64_t shuffle_seed,
