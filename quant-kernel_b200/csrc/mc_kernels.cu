@@ -1262,6 +1262,7 @@ __global__ void __launch_bounds__(256)
                        const TilePartial* __restrict__ partials, double* __restrict__ out_price,
                        double* __restrict__ out_se, const int32_t* __restrict__ out_index,
                        unsigned long long* __restrict__ work_counter) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the simulation's slots, if still running
     if (work_counter != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *work_counter = 0ull;
     const int32_t warp = (int32_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
@@ -1446,13 +1447,21 @@ cudaError_t launch_persistent(int block, const SimArgs& a, const GroupTable* gro
 
 cudaError_t launch_finalize(const McOption* opts, int32_t n, const TilePartial* partials,
                             double* out_price, double* out_se, const int32_t* out_index,
-                            unsigned long long* work_counter, cudaStream_t st) {
+                            unsigned long long* work_counter, bool dependent, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     const int64_t threads = (int64_t)n * 32;
     const unsigned grid = (unsigned)((threads + 255) / 256);
-    mc_finalize_kernel<<<grid, 256, 0, st>>>(opts, n, partials, out_price, out_se, out_index,
-                                             work_counter);
-    return cudaGetLastError();
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = dependent ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, mc_finalize_kernel, opts, n, partials, out_price, out_se, out_index,
+                              work_counter);
 }
 
 int max_resident_ctas(int family_or_persistent, int block, int upt, int device) {

@@ -93,9 +93,12 @@ cudaError_t launch_simulate(int family, bool anti, int block, int upt, int su, c
 cudaError_t launch_persistent(int block, const SimArgs& a, const GroupTable* groups,
                               unsigned long long* work_counter, cudaStream_t st);
 // out_index (nullable): record k's results go to slot out_index[k].
+// dependent: the launch is prepared while the simulation runs (the kernel waits
+// for it before it reads anything).  One quote 32.8 us with a plain launch,
+// 30.6 so; for calls on a plan's own stream, so that captures keep plain nodes.
 cudaError_t launch_finalize(const McOption* opts, int32_t n, const TilePartial* partials,
                             double* out_price, double* out_se, const int32_t* out_index,
-                            unsigned long long* work_counter, cudaStream_t st);
+                            unsigned long long* work_counter, bool dependent, cudaStream_t st);
 // Resident CTAs on `device` for a family kernel (family >= 0) or the
 // persistent kernel (family < 0); 0 on error.
 int max_resident_ctas(int family_or_persistent, int block, int upt, int device);

@@ -158,7 +158,7 @@ NoAllocStatus noalloc_heston_batch(const BatchInput& in, double* out_prices, dou
         e = injected_fault(kFaultLaunch);
         if (e == cudaSuccess) e = launch_simulate(kFamHeston, true, kBlock, kUpt, 1, a, st);
     }
-    if (e == cudaSuccess) e = launch_finalize(d_rec, in.n, d_part, d_price, d_se, nullptr, nullptr, st);
+    if (e == cudaSuccess) e = launch_finalize(d_rec, in.n, d_part, d_price, d_se, nullptr, nullptr, false, st);
     if (e == cudaSuccess) e = injected_fault(kFaultCopy);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(out_prices, d_price, sizeof(double) * in.n, cudaMemcpyDeviceToHost, st);

@@ -515,7 +515,8 @@ cudaError_t Plan::build(const BatchInput& in, int32_t flags, std::string* err) {
     // Two 8-byte stores an option over PCIe against a copy's launch: a small
     // batch's results go straight to the pinned buffer (one quote, with a
     // single upload in place of three operations: 45 -> 25 us in the library)
-    host_results_ = (flags & kFlagOneShot) && in.n <= kHostResultOptions;
+    one_shot_ = (flags & kFlagOneShot) != 0;
+    host_results_ = one_shot_ && in.n <= kHostResultOptions;
     // QK_PLAN_STEP_UNROLL2: two step blocks per loop iteration where compiled
     if ((flags & kFlagStepUnroll2) && !persistent_ && step_unroll2_compiled(family_, cfg_.upt))
         cfg_.su = 2;
@@ -704,7 +705,7 @@ cudaError_t Plan::launch_all(cudaStream_t st, bool timing) {
     // scatters results back to the caller's order
     double* out = static_cast<double*>(host_results_ ? h_res_.p : d_res_.p);
     return launch_finalize(a.opts, n_, a.partials, out, out + n_, d_out_index(),
-                           use_counter ? counter : nullptr, st);
+                           use_counter ? counter : nullptr, one_shot_ && !timing, st);
 }
 
 void partition_by_cost(const double* cost, int64_t n, int world, int64_t* bounds) {
@@ -802,7 +803,7 @@ cudaError_t Plan::launch_tiles(cudaStream_t st, int64_t lo, int64_t hi, bool tim
 
 cudaError_t Plan::launch_finalize_all(cudaStream_t st) {
     return launch_finalize(d_records(), n_, static_cast<const TilePartial*>(d_partials_.p), d_price(),
-                           d_se(), d_out_index(), nullptr, st);
+                           d_se(), d_out_index(), nullptr, false, st);
 }
 
 cudaError_t Plan::capture_graph() {

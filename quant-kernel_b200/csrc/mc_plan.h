@@ -139,6 +139,7 @@ private:
     int max_ctas_ = 0;
     double last_ms_ = 0.0;
     bool upload_pending_ = false;  // an upload from h_in_ that nothing has waited for
+    bool one_shot_ = false;        // a batch call's plan: own stream, no capture
     bool host_results_ = false;    // finalize writes h_res_ itself
 
     std::vector<McOption> opts_;       // host copy (units/tiles filled per layout)
