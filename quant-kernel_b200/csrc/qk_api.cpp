@@ -795,7 +795,7 @@ int32_t qk_mcm_plan_create(const int32_t* model, const double* spot, const doubl
     if (rc != QK_OK) return rc;
     qk_mc_plan* p = new qk_mc_plan();
     std::string err;
-    cudaError_t e = p->plan.build(in, flags, &err);
+    cudaError_t e = p->plan.build(in, flags & ~static_cast<int32_t>(qkb::kFlagOneShot), &err);
     if (e != cudaSuccess) {
         delete p;
         return fail_cuda(e, "qk_mcm_plan_create");

@@ -45,3 +45,25 @@ def test_read_only_and_strided_columns(qk):
         v.flags.writeable = bool(i % 3)
         odd[k] = v
     assert np.array_equal(qk.heston_monte_carlo_price_batch(**odd), want)
+
+
+class _Device:
+    def __init__(self, ptr, n):
+        self.__cuda_array_interface__ = dict(shape=(n,), typestr="<f8", data=(ptr, False), version=3)
+
+
+def test_unknown_plan_flags_keep_device_results(qk):
+    """A plan built with a flag bit that means nothing to callers is read and
+    run again like any other: its results stay on the device too."""
+    import torch
+
+    b = workloads.mixed(8, seed=3, log2_paths=(10, 11), log2_steps=(3, 4))
+    plan = qk.plan(**b, flags=0x10000)
+    want = qk.plan(**b)
+    for p in (want, plan, plan):
+        p.execute()
+    w, g = want.results(), plan.results()
+    for a, c in zip(g, w):
+        assert np.array_equal(a, c)
+    for ptr, a in zip(plan.device_results(), w):
+        assert np.array_equal(torch.as_tensor(_Device(ptr, 8), device="cuda").cpu().numpy(), a)
