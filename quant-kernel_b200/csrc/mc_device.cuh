@@ -24,11 +24,6 @@ __device__ __forceinline__ float ptx_lg2(float x) {
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float ptx_ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 __device__ __forceinline__ float ptx_sqrt(float x) {
     float y;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -51,16 +46,11 @@ __device__ __forceinline__ float ptx_max_nan(float a, float b) {
     asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
     return y;
 }
-// Three-operand min and max (sm_100), NaN-propagating: one instruction adds two
-// values to a running extreme.
+// Three-operand min (sm_100), NaN-propagating: one instruction adds two values
+// to a running minimum.
 __device__ __forceinline__ float ptx_min3_nan(float a, float b, float c) {
     float y;
     asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
-    return y;
-}
-__device__ __forceinline__ float ptx_max3_nan(float a, float b, float c) {
-    float y;
-    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
     return y;
 }
 __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
