@@ -76,6 +76,15 @@ PIPES = {"issue": float(ISSUE_PER_CLK), "xu": float(XU_PER_CLK), "fp64": float(F
 PROBE_KINDS = (("issue", 1), ("xu", 0), ("fp64", 3), ("ffma2_lanes", 2), ("xu_in_heston_mix", 4))
 
 
+
+def plan_upload_bytes(n: int) -> int:
+    """Bytes a single-family batch of n options sends: 128-byte records, tile
+    offsets (each padded to 256 bytes) and the work counter, one buffer."""
+    def pad(x):
+        return (x + 255) // 256 * 256
+    return pad(128 * n) + pad(8 * (n + 1)) + 8
+
+
 def measure_pipes(qk, device):
     """Measure the pipe widths on `device` with the library's probe (FP32 FMA
     lanes = the issue width, MUFU lanes, FP64 FMA lanes, packed-FMA lanes, and
@@ -666,7 +675,7 @@ def main_gpu(args):
         else:
             extras["secondary_error"] = f"{type(exc).__name__}: {exc}"[:300]
 
-    h2d = n_opt * 128 + (n_opt + 1) * 8  # packed option records + tile offsets
+    h2d = plan_upload_bytes(n_opt)
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": total_ms / args.steps, "higher_is_better": True,
@@ -1117,7 +1126,7 @@ def bsm_terminal_leg(qk, reps=20, f_mhz=1965.0, cpu=True):
     res = {"workload": "64 BSM calls/puts x 131072 paths (terminal GBM, antithetic pairs)",
            "dtype": "f64", "ms": ms, "paths_per_s": paths / (ms / 1e3), "e2e_ms": 1e3 * e2e,
            "e2e_paths_per_s": paths / e2e, "api": "qk_mcm_antithetic_variates_price_batch",
-           "h2d_bytes": n * 128 + (n + 1) * 8, "d2h_bytes": n * 8,
+           "h2d_bytes": plan_upload_bytes(n), "d2h_bytes": n * 8,
            "roofline": {"bound": "fp64", "unit": "GFLOP/s",
                         "achieved": pairs * FP64_PER_PAIR / (kern_ms / 1e3) / 1e9,
                         "peak": fp64_peak / 1e9,
@@ -1273,11 +1282,11 @@ def heston_cf_leg(qk, reps=5, n=65536, cpu=True):
     e2e = e2e_time(qk.heston_price_cf_batch, workloads.heston_cf(n))
     res = {"workload": f"{n} Heston calls/puts, CF with 1024 steps, limit 120",
            "e2e_ms": 1e3 * e2e, "e2e_options_per_s": n / e2e,
-           "h2d_bytes": n * 128, "d2h_bytes": n * 8}
+           "h2d_bytes": n * 96, "d2h_bytes": n * 8}
     e2e = e2e_time(qk.cos_method_fang_oosterlee_heston_price_batch, _cos_batch(n))
     cos = {"workload": f"{n} Heston calls/puts, COS with 256 terms, width 10",
            "e2e_ms": 1e3 * e2e, "e2e_options_per_s": n / e2e,
-           "h2d_bytes": n * 128, "d2h_bytes": n * 8}
+           "h2d_bytes": n * 96, "d2h_bytes": n * 8}
     if cpu:
         res["cpu_baseline"] = cpu_rate()
         cos["cpu_baseline"] = cpu_rate(method="cos")
