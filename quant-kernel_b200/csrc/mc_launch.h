@@ -34,8 +34,8 @@ constexpr int kUptVr = 1;
 
 // The one family -> units-per-thread map: the persistent kernel's family
 // bodies, the tiling of every mixed plan and the default single-family
-// tiling all take it, so a mixed launch and the per-method calls tile each
-// option alike and give the same bits.
+// tiling take it (stepwise_batch_upt lowers the last for small batches and
+// long one-factor paths; the sums give the same bits).
 constexpr int family_upt(int family) {
     return family == kFamTerminal ? kUptTerminal
          : family == kFamVr ? kUptVr

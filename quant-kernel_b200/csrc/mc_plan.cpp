@@ -40,6 +40,16 @@ constexpr int64_t kMinTerminalTiles = 32;
 // two pairs win, 62.9 against 65.8 (Euler, four units a thread: 39.8 and 32.6,
 // 45.3 and 41.3, 60.2 and 70.7 with one).
 constexpr int64_t kSmallBatchTiles = 296;
+// Two units a thread instead of four for long one-factor paths: no spills under
+// Euler's register bound, 66 registers instead of 80 for Milstein, a shorter
+// last wave; but a tile's fixed cost weighs on half the paths.
+// Four and two, us a call of 48 options: Euler at 126 steps 147 and 139 with
+// 2400 tiles (of four), 463 and 449 with 9600, 928 and 899 with 20016; Milstein
+// 95 and 90 with 1200, 260 and 255 with 4800, 478 and 480 with 9600 (719 and
+// 715 at 200 steps); at 24 steps and 4800 tiles four wins (Euler 88.1 and 89.6,
+// Milstein 89.5 and 92.9).
+constexpr int64_t kLongPathSteps = 72;
+constexpr int64_t kMilsteinTiles = 6000, kMilsteinSteps = 180;
 constexpr int32_t kHostResultOptions = 64;
 
 double nan_value() { return std::numeric_limits<double>::quiet_NaN(); }
@@ -509,9 +519,10 @@ cudaError_t Plan::build(const BatchInput& in, int32_t flags, std::string* err) {
         if (persistent_ && cfg_.upt > 0) cfg_.upt = kUptPersistent;
         cfg_.su = (!persistent_ && step_unroll2_compiled(family_, cfg_.upt)) ? tuned.su : 1;
     }
-    // A batch too small to fill the chip runs its paths on more threads
+    // Long one-factor paths, and a batch too small to fill the chip, run on
+    // more threads
     if (!persistent_ && !tuned_shape && !(flags & (kFlagStepUnroll2 | kFlagAutotune)))
-        cfg_.upt = small_batch_upt(cfg_, family_);
+        cfg_.upt = stepwise_batch_upt(cfg_, family_);
     // Two 8-byte stores an option over PCIe against a copy's launch: a small
     // batch's results go straight to the pinned buffer (one quote, with a
     // single upload in place of three operations: 45 -> 25 us in the library)
@@ -545,13 +556,26 @@ static int family_rank(int fam) {
     }
 }
 
-// Units per thread for a stepwise single-family batch: the family's own while
-// that makes at least kSmallBatchTiles tiles, else halved (and halved again),
-// which spreads the same paths over more warps.  A path's normals and
-// arithmetic do not change, and tile sums are double-double.
-int Plan::small_batch_upt(const LaunchConfig& cfg, int family) const {
+// Units per thread for a stepwise single-family batch: the family's own, or two
+// for long one-factor paths, while that makes at least kSmallBatchTiles tiles,
+// else halved (and halved again), which spreads the same paths over more warps.
+// A path's normals and arithmetic do not change, and tile sums are
+// double-double.
+int Plan::stepwise_batch_upt(const LaunchConfig& cfg, int family) const {
     if (!family_is_stepwise(family)) return cfg.upt;
     int upt = cfg.upt;
+    if (upt == kUptStepwise) {  // a one-factor family
+        int64_t tiles = 0;
+        double steps = 0.0;
+        for (const McOption& o : opts_) {
+            if (o.mode != kModeSimulate) continue;
+            const int64_t k = (o.units + cfg.block * upt - 1) / (cfg.block * upt);
+            tiles += k;
+            steps += (double)k * (double)o.steps;
+        }
+        const bool milstein = family == kFamMilstein && tiles >= kMilsteinTiles;
+        if (steps >= (double)((milstein ? kMilsteinSteps : kLongPathSteps) * tiles)) upt = 2;
+    }
     for (; upt > 1; upt /= 2) {
         int64_t tiles = 0;
         for (const McOption& o : opts_) {

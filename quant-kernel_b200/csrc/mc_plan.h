@@ -118,7 +118,7 @@ public:
 
 private:
     cudaError_t ensure_stream();
-    int small_batch_upt(const LaunchConfig& cfg, int family) const;
+    int stepwise_batch_upt(const LaunchConfig& cfg, int family) const;
     cudaError_t layout_tiles(const LaunchConfig& cfg);  // tile geometry + upload
     cudaError_t launch_all(cudaStream_t st, bool timing);
     cudaError_t autotune();

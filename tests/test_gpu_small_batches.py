@@ -34,6 +34,21 @@ def test_price_does_not_depend_on_the_batch(qk, kind, paths):
             np.testing.assert_allclose(g, w[:n], rtol=1e-14, atol=0)
 
 
+@pytest.mark.parametrize("steps", (71, 72))
+@pytest.mark.parametrize("paths", (1024 * 124 - 3, 1024 * 125 + 1))
+@pytest.mark.parametrize("kind", ("euler_maruyama", "milstein", "local_vol_monte_carlo"))
+def test_long_one_factor_paths(qk, kind, paths, steps):
+    """Two or four units a thread, on either side of 72 steps and of 6000 tiles:
+    options of a batch of 48 against the same options priced alone."""
+    b = workloads.bsm_terminal(48, paths, seed=9)
+    b["steps"] = np.full(48, steps, np.int32)
+    fn = getattr(qk, kind + "_price_se_batch")
+    full = fn(**b)
+    for i in (0, 31, 47):
+        for g, w in zip(fn(**{k: v[i:i + 1] for k, v in b.items()}), full):
+            np.testing.assert_allclose(g, w[i:i + 1], rtol=1e-14, atol=0)
+
+
 def test_read_only_and_strided_columns(qk):
     b = _batch("heston", 12, 1001)
     want = qk.heston_monte_carlo_price_batch(**b)
