@@ -391,9 +391,18 @@ __global__ void __launch_bounds__(128, 3)
     HestonFast f2, f1;
     Sums s;
     bool nan_phi = false;
-    if (o.limit >= 1.0 && panels < (1 << 24) && fast_constants(o, o.limit, f2, f1)) {
+    const double drift = (o.r - o.q) * o.t;
+    bool bounded = o.limit >= 1.0 && panels < (1 << 24) && fast_constants(o, o.limit, f2, f1);
+    if (bounded) {
+        // log phi(-i): below log(1e-14) = -32.24 the price is NaN, near exp's
+        // range phi(-i) and the quotient by it overflow.  The bounded route forms
+        // neither: both ends are the general form's.
+        const double log_phi = fp64_log(o.spot, tab) + drift;
+        bounded = log_phi >= -32.2 && log_phi <= 700.0;
+    }
+    if (bounded) {
         // of log(S/K), not log S - log K: u magnifies the difference's rounding
-        f2.phase = f1.phase = log(o.spot / o.strike) + (o.r - o.q) * o.t;
+        f2.phase = f1.phase = log(o.spot / o.strike) + drift;
         const double half = 0.5 * width;
         s = tree_sum<WARPS>(
             [&](int v) {
