@@ -92,13 +92,15 @@ int32_t geti(const int32_t* a, int32_t i, int32_t dflt) { return a ? a[i] : dflt
 // The state S/spot above which a block of six one-factor steps cannot reach the
 // floor fl, from a bound on a step's factor: 1 + m0 + b z [+ c z^2] >= g for
 // |z| <= 5.769, above the sqrt(2 24 ln 2) = 5.768 of a 23-bit Box-Muller
-// radius, with room for FP32 rounding.  +inf (no floor-free blocks) where no
-// whole block runs or the bound leaves less than a hundredth of the spot.
+// radius, with room for FP32 rounding.  A factor that only grows counts as 1:
+// the floor may be met at any step of the block, not only its last.  +inf (no
+// floor-free blocks) where no whole block runs or the bound leaves less than a
+// hundredth of the spot.
 float stepwise_block_min(double m0, double b, double fl, double c, int32_t steps) {
     double inc = m0 - 5.769 * b;
     // c z^2 >= 0, and the quadratic's vertex
     if (c > 0.0) inc = std::max(inc, m0 - b * b / (4.0 * c));
-    const double g = 0.9999 + inc;
+    const double g = std::min(0.9999 + inc, 1.0);
     const double limit = 1.001 * fl / (g * g * g * g * g * g);
     return steps >= 6 && g > 0.05 && limit <= 0.01 ? (float)limit
                                                     : std::numeric_limits<float>::infinity();
