@@ -208,7 +208,10 @@ __global__ void __launch_bounds__(kFeatRows)
 quote_price_kernel(const double* __restrict__ fix, int64_t n, const float* __restrict__ y,
                    double* __restrict__ out) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * kFeatRows + threadIdx.x;
-    if (i < n) out[i] = fix[i] * static_cast<double>(y[i]) - fix[n + i] + fix[2 * n + i];
+    if (i >= n) return;
+    const double spot = fix[i];  // 0: not the network's
+    const double call = spot != 0.0 ? spot * static_cast<double>(y[i]) : 0.0;
+    out[i] = call - fix[n + i] + fix[2 * n + i];
 }
 
 // ----------------------------------------------------------------------------
