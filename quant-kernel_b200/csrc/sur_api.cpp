@@ -232,37 +232,24 @@ int32_t qk_sur_heston_price_batch(qk_sur_model* model, const double* spot, const
     if (n <= 0) return qkb::fail_size(n);
     // entry checks, routing, features, the network and put-call parity all
     // run on the GPU; only the options outside the box come back to the host
-    std::vector<int32_t> own_route;
-    if (!out_source) {
-        own_route.resize(static_cast<size_t>(n));
-        out_source = own_route.data();
-    }
     const double* const cols[10] = {spot, strike, t, r, q, v0, kappa, theta, sigma, rho};
-    int32_t rc = sur_status(model->m.price_quotes(cols, option_type, n, out_prices, out_source),
+    qkb::SurOutside far;
+    int32_t rc = sur_status(model->m.price_quotes(cols, option_type, n, out_prices, out_source, &far),
                             "qk_sur_heston_price_batch");
     if (rc != QK_OK) return rc;
-    std::vector<int32_t> mc_idx;
-    for (int32_t i = 0; i < n; ++i)
-        if (out_source[i] == 1) mc_idx.push_back(i);
-    if (!mc_idx.empty()) {
-        const size_t m = mc_idx.size();
-        std::vector<double> a[10];
-        for (auto& v : a) v.resize(m);
-        std::vector<int32_t> ot(m), pp(m, fallback_paths), st(m, fallback_steps);
+    if (!far.index.empty()) {
+        const size_t m = far.index.size();
+        const std::vector<double>* a = far.cols;
+        std::vector<int32_t> pp(m, fallback_paths), st(m, fallback_steps);
         std::vector<uint64_t> sd(m);
-        for (size_t k = 0; k < m; ++k) {
-            const int32_t i = mc_idx[k];
-            for (int c = 0; c < 10; ++c) a[c][k] = cols[c][i];
-            ot[k] = option_type[i];
-            sd[k] = fallback_seed + static_cast<uint64_t>(i);
-        }
+        for (size_t k = 0; k < m; ++k) sd[k] = fallback_seed + static_cast<uint64_t>(far.index[k]);
         std::vector<double> out(m);
         rc = qk_mcm_heston_monte_carlo_price_batch(
             a[0].data(), a[1].data(), a[2].data(), a[3].data(), a[4].data(), a[5].data(), a[6].data(),
-            a[7].data(), a[8].data(), a[9].data(), ot.data(), pp.data(), st.data(), sd.data(),
-            static_cast<int32_t>(m), out.data());
+            a[7].data(), a[8].data(), a[9].data(), far.option_type.data(), pp.data(), st.data(),
+            sd.data(), static_cast<int32_t>(m), out.data());
         if (rc != QK_OK) return rc;
-        for (size_t k = 0; k < m; ++k) out_prices[mc_idx[k]] = out[k];
+        for (size_t k = 0; k < m; ++k) out_prices[far.index[k]] = out[k];
     }
     return QK_OK;
 }

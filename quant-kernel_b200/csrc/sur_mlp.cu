@@ -952,7 +952,7 @@ cudaError_t SurModel::predict(const double* features, int64_t n, double* out) {
 }
 
 cudaError_t SurModel::price_quotes(const double* const (&cols)[10], const int32_t* option_type,
-                                   int64_t n, double* out, int32_t* route) {
+                                   int64_t n, double* out, int32_t* route, SurOutside* outside) {
     DeviceGuard g(device_);
     const size_t in_row = 10 * sizeof(double) + sizeof(int32_t);
     const size_t out_row = sizeof(double) + sizeof(int32_t);
@@ -977,9 +977,15 @@ cudaError_t SurModel::price_quotes(const double* const (&cols)[10], const int32_
             return cudaGetLastError();
         },
         [&](const char* h, int64_t off, int64_t m) {
+            const int32_t* to = reinterpret_cast<const int32_t*>(h + sizeof(double) * static_cast<size_t>(m));
+            for (int64_t i = 0; i < m; ++i) {
+                if (to[i] != 1) continue;
+                outside->index.push_back(static_cast<int32_t>(off + i));
+                outside->option_type.push_back(option_type[off + i]);
+                for (int c = 0; c < 10; ++c) outside->cols[c].push_back(cols[c][off + i]);
+            }
             std::memcpy(out + off, h, sizeof(double) * static_cast<size_t>(m));
-            std::memcpy(route + off, h + sizeof(double) * static_cast<size_t>(m),
-                        sizeof(int32_t) * static_cast<size_t>(m));
+            if (route) std::memcpy(route + off, to, sizeof(int32_t) * static_cast<size_t>(m));
         });
 }
 

@@ -11,6 +11,7 @@
 #include <cstdint>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <vector>
 
 namespace qkb {
 
@@ -54,6 +55,12 @@ struct SurBox {
     double hi[kSurIn];
 };
 
+// Options that the network does not price: their places and inputs.
+struct SurOutside {
+    std::vector<int32_t> index, option_type;
+    std::vector<double> cols[10];
+};
+
 class SurModel {
 public:
     SurModel() = default;
@@ -79,10 +86,12 @@ public:
     // price / spot of calls for raw features, host in and out.
     cudaError_t predict(const double* features, int64_t n, double* out);
     // The host pricing call: columns spot, strike, t, r, q, v0, kappa, theta,
-    // sigma, rho and option_type, n each.  route[i]: 0 priced by the network,
-    // 1 outside the box (out[i] is NaN), 2 decided by the entry checks.
+    // sigma, rho and option_type, n each.  route[i] (route may be null): 0 priced
+    // by the network, 1 outside the box (out[i] is NaN), 2 decided by the entry
+    // checks.  The options outside are copied to `outside` before anything is
+    // written: out and route may be the caller's input columns.
     cudaError_t price_quotes(const double* const (&cols)[10], const int32_t* option_type, int64_t n,
-                             double* out, int32_t* route);
+                             double* out, int32_t* route, SurOutside* outside);
     // Device-resident inference on normalised bf16 rows [n][64] plus the
     // rows' base (required when base_kind() != kSurBaseNone): the fused kernel
     // (all three layers per 128-row tile in one persistent launch), or with

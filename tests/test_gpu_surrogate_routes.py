@@ -1,6 +1,9 @@
 """The surrogate's host pricing call where its routes meet: options that the
-entry checks decide do not depend on the network.
+entry checks decide do not depend on the network, and outputs may share memory
+with the inputs they replace.
 """
+
+import ctypes as ct
 
 import numpy as np
 import pytest
@@ -33,4 +36,24 @@ def test_decided_options_do_not_depend_on_the_network(qk, value):
     decided = kind != 0
     assert np.array_equal(got[decided], want[decided], equal_nan=True)
     assert np.all(np.isfinite(got[kind == 1])) and np.all(np.isfinite(got[kind == 2]))
+    sur.close()
+
+
+@pytest.mark.parametrize("n", (40, 65536 + 21))
+@pytest.mark.parametrize("column", (0, 1, 6, 9))
+def test_outputs_in_the_inputs_memory(qk, n, column):
+    """out_prices over one of the ten columns, out_source over option_type."""
+    sur = HestonSurrogate(qk, seed=3)
+    b, ot, kind = _quotes(n)
+    want, src = sur.price_batch(**b, option_type=ot, fallback_paths=500, fallback_steps=8, fallback_seed=5)
+    cols = [np.ascontiguousarray(b[k], np.float64) for k in ("spot", "strike", "t", "r", "q", "v0", "kappa",
+                                                             "theta", "sigma", "rho")]
+    pd, pi = ct.POINTER(ct.c_double), ct.POINTER(ct.c_int32)
+    typ = ot.copy()
+    rc = sur.lib.qk_sur_heston_price_batch(
+        sur._h, *[c.ctypes.data_as(pd) for c in cols], typ.ctypes.data_as(pi), n, 500, 8, 5,
+        cols[column].ctypes.data_as(pd), typ.ctypes.data_as(pi))
+    assert rc == 0
+    assert np.array_equal(cols[column], want, equal_nan=True)
+    assert np.array_equal(typ, src)
     sur.close()
