@@ -565,13 +565,18 @@ static int family_rank(int fam) {
 // double-double.
 int Plan::stepwise_batch_upt(const LaunchConfig& cfg, int family) const {
     if (!family_is_stepwise(family)) return cfg.upt;
+    // units reach 2^31 - 1
+    auto tiles_of = [&](const McOption& o, int upt) {
+        const int64_t per = (int64_t)cfg.block * upt;
+        return (o.units + per - 1) / per;
+    };
     int upt = cfg.upt;
     if (upt == kUptStepwise) {  // a one-factor family
         int64_t tiles = 0;
         double steps = 0.0;
         for (const McOption& o : opts_) {
             if (o.mode != kModeSimulate) continue;
-            const int64_t k = (o.units + cfg.block * upt - 1) / (cfg.block * upt);
+            const int64_t k = tiles_of(o, upt);
             tiles += k;
             steps += (double)k * (double)o.steps;
         }
@@ -581,7 +586,7 @@ int Plan::stepwise_batch_upt(const LaunchConfig& cfg, int family) const {
     for (; upt > 1; upt /= 2) {
         int64_t tiles = 0;
         for (const McOption& o : opts_) {
-            if (o.mode == kModeSimulate) tiles += (o.units + cfg.block * upt - 1) / (cfg.block * upt);
+            if (o.mode == kModeSimulate) tiles += tiles_of(o, upt);
             if (tiles >= kSmallBatchTiles) return upt;
         }
     }
