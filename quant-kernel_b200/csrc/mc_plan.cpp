@@ -655,7 +655,7 @@ cudaError_t Plan::layout_tiles(const LaunchConfig& cfg) {
         in_.out_index = align(in_.groups + sizeof(GroupTable));
         in_.bytes = in_.out_index + sizeof(int32_t) * (size_t)n;
     }
-    const size_t res_bytes = 2 * sizeof(double) * (size_t)std::max(n, 1);
+    const size_t res_bytes = sizeof(double) * (se_at() + (size_t)std::max(n, 1));
     if ((e = d_in_.ensure(in_.bytes)) != cudaSuccess) return e;
     if ((e = d_partials_.ensure(sizeof(TilePartial) * (size_t)std::max<int64_t>(total, 1))) != cudaSuccess) return e;
     if ((e = d_res_.ensure(res_bytes)) != cudaSuccess) return e;
@@ -735,7 +735,7 @@ cudaError_t Plan::launch_all(cudaStream_t st, bool timing) {
     // persistent plans hold the records in work order; the finalize kernel
     // scatters results back to the caller's order
     double* out = static_cast<double*>(host_results_ ? h_res_.p : d_res_.p);
-    return launch_finalize(a.opts, n_, a.partials, out, out + n_, d_out_index(),
+    return launch_finalize(a.opts, n_, a.partials, out, out + se_at(), d_out_index(),
                            use_counter ? counter : nullptr, one_shot_ && !timing, st);
 }
 
@@ -881,14 +881,15 @@ cudaError_t Plan::results(double* out_price, double* out_se) {
     cudaStream_t st = last_stream_ ? last_stream_ : stream_;
     const size_t bytes = sizeof(double) * (size_t)n_;
     cudaError_t e;
-    if (!host_results_ && (e = cudaMemcpyAsync(h_res_.p, d_res_.p, out_se ? 2 * bytes : bytes,
+    if (!host_results_ && (e = cudaMemcpyAsync(h_res_.p, d_res_.p,
+                                               out_se ? sizeof(double) * se_at() + bytes : bytes,
                                                cudaMemcpyDeviceToHost, st)) != cudaSuccess)
         return e;
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
     upload_pending_ = false;  // the executes waited for it
     const double* res = static_cast<const double*>(h_res_.p);
     std::memcpy(out_price, res, bytes);
-    if (out_se) std::memcpy(out_se, res + n_, bytes);
+    if (out_se) std::memcpy(out_se, res + se_at(), bytes);
     if (flags_ & kFlagTiming) {
         float ms = 0.0f;
         if (cudaEventElapsedTime(&ms, ev0_, ev1_) == cudaSuccess) last_ms_ = ms;

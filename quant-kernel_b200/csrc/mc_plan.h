@@ -97,7 +97,7 @@ public:
     int ctas() const { return max_ctas_; }
     bool persistent() const { return persistent_; }
     double* d_price() const { return static_cast<double*>(d_res_.p); }
-    double* d_se() const { return d_price() + n_; }
+    double* d_se() const { return d_price() + se_at(); }
     int device() const { return device_; }
     TilePartial* d_partials() const { return static_cast<TilePartial*>(d_partials_.p); }
     cudaStream_t stream() const { return stream_; }
@@ -166,7 +166,9 @@ private:
     const int32_t* d_out_index() const {
         return persistent_ ? d_at<const int32_t>(in_.out_index) : nullptr;
     }
-    // results: n prices, then n standard errors
+    // results: n prices, then n standard errors from the next 256-byte boundary
+    // (callers get both device pointers, aligned like allocations)
+    size_t se_at() const { return ((size_t)n_ + 31) & ~(size_t)31; }
     DevBuf d_in_, d_partials_, d_res_;
     PinnedBuf h_in_, h_res_;
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
