@@ -20,6 +20,7 @@ int armed_sites() {
     if (std::strstr(v, "launch")) sites |= kFaultLaunch;
     if (std::strstr(v, "copy")) sites |= kFaultCopy;
     if (std::strstr(v, "collective")) sites |= kFaultCollective;
+    if (std::strstr(v, "timeout")) sites |= kFaultTimeout;
     return sites;
 }
 
@@ -31,6 +32,7 @@ cudaError_t injected_fault(FaultSite site) {
     switch (site) {
         case kFaultAlloc: return cudaErrorMemoryAllocation;
         case kFaultLaunch: return cudaErrorLaunchFailure;
+        case kFaultTimeout: return cudaErrorLaunchTimeout;
         default: return cudaErrorUnknown;
     }
 }

@@ -7,6 +7,8 @@
 //   copy    host<->device copies report cudaErrorUnknown before copying
 //   collective  the sharded execute reports cudaErrorUnknown instead of
 //               issuing its NCCL exchange (after its own simulate kernels)
+//   timeout the surrogate's tensor-core kernels find their error word set, as a
+//               wait that ran out would leave it; the kernels run as usual
 // The variable is read at every site, so a process can arm and disarm it.
 // An injected failure is reported like a real one (QK_ERR_RUNTIME_INIT and a
 // "cuda error: ..." message) with "[injected]" appended to the message.
@@ -19,7 +21,9 @@
 
 namespace qkb {
 
-enum FaultSite : int { kFaultAlloc = 1, kFaultLaunch = 2, kFaultCopy = 4, kFaultCollective = 8 };
+enum FaultSite : int {
+    kFaultAlloc = 1, kFaultLaunch = 2, kFaultCopy = 4, kFaultCollective = 8, kFaultTimeout = 16
+};
 
 // cudaSuccess, or the injected error for `site` when QK_B200_FAULT arms it.
 cudaError_t injected_fault(FaultSite site);

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "qk_error.h"
+#include "qk_fault.h"
 #include "sur_gemm.cuh"
 
 extern "C" {
@@ -58,8 +59,13 @@ struct qk_sur_model {
 
 namespace {
 
-int32_t sur_status(cudaError_t e, const char* where) {
+int32_t sur_status(cudaError_t e, const char* where, qk_sur_model* model = nullptr) {
     if (e == cudaSuccess) return QK_OK;
+    if (const int code = model ? model->m.take_pipeline_code() : 0) {
+        qkb::set_error_fmt("tensor-core pipeline timed out (code %d) in %s%s", code, where,
+                           qkb::take_injected_flag() ? " [injected]" : "");
+        return QK_ERR_RUNTIME_INIT;
+    }
     if (e == cudaErrorInvalidValue) {
         qkb::set_error_fmt("invalid argument in %s", where);
         return QK_ERR_INVALID_INPUT;
@@ -118,13 +124,9 @@ int32_t qk_sur_heston_train(qk_sur_model* model, int32_t epochs, int32_t batch, 
     std::vector<float> el(static_cast<size_t>(epochs));
     float last = 0.0f;
     cudaError_t e = model->m.train(epochs, batch, static_cast<float>(lr), shuffle_seed, &last, el.data());
-    if (e == cudaSuccess && model->m.device_error() != 0) {
-        qkb::set_error_fmt("tensor-core pipeline timed out (code %d)", model->m.device_error());
-        return QK_ERR_RUNTIME_INIT;
-    }
     if (e == cudaSuccess && out_epoch_loss)
         for (int i = 0; i < epochs; ++i) out_epoch_loss[i] = el[static_cast<size_t>(i)];
-    return sur_status(e, "qk_sur_heston_train");
+    return sur_status(e, "qk_sur_heston_train", model);
 }
 
 int32_t qk_sur_heston_predict(qk_sur_model* model, const double* features, int64_t n, double* out) {
@@ -132,7 +134,7 @@ int32_t qk_sur_heston_predict(qk_sur_model* model, const double* features, int64
     if (!features) return qkb::fail_null("features");
     if (!out) return qkb::fail_null("out");
     if (n <= 0) return qkb::fail_size(n);
-    return sur_status(model->m.predict(features, n, out), "qk_sur_heston_predict");
+    return sur_status(model->m.predict(features, n, out), "qk_sur_heston_predict", model);
 }
 
 int32_t qk_sur_heston_predict_device(qk_sur_model* model, const void* x_rows, const float* base,
@@ -189,7 +191,7 @@ int32_t qk_sur_heston_gradients(qk_sur_model* model, const double* features, con
     if (!target) return qkb::fail_null("target");
     if (!grads) return qkb::fail_null("grads");
     if (n <= 0 || n % 128 != 0) return qkb::fail_size(n);
-    return sur_status(model->m.gradients(features, target, n, grads, loss), "qk_sur_heston_gradients");
+    return sur_status(model->m.gradients(features, target, n, grads, loss), "qk_sur_heston_gradients", model);
 }
 
 int32_t qk_sur_heston_parameters(qk_sur_model* model, double* out) {
@@ -235,7 +237,7 @@ int32_t qk_sur_heston_price_batch(qk_sur_model* model, const double* spot, const
     const double* const cols[10] = {spot, strike, t, r, q, v0, kappa, theta, sigma, rho};
     qkb::SurOutside far;
     int32_t rc = sur_status(model->m.price_quotes(cols, option_type, n, out_prices, out_source, &far),
-                            "qk_sur_heston_price_batch");
+                            "qk_sur_heston_price_batch", model);
     if (rc != QK_OK) return rc;
     if (!far.index.empty()) {
         const size_t m = far.index.size();

@@ -23,6 +23,7 @@
 
 #include "mc_device.cuh"
 #include "mc_plan.h"
+#include "qk_fault.h"
 #include "sur_gemm.cuh"
 
 namespace qkb {
@@ -30,6 +31,7 @@ namespace qkb {
 namespace {
 
 constexpr int kPredChunk = 65536;
+constexpr size_t kOutHead = 4 * sizeof(int);  // a chunk's error word before its results
 
 #define QK_TRY(x)                                \
     do {                                         \
@@ -203,12 +205,13 @@ quote_features_kernel(const double* __restrict__ in, int64_t n, SurBox box, int3
 }
 
 // The call from price / S, puts by put-call parity, straight into the pinned
-// slot (coalesced).
+// slot (coalesced), with the network's error word.
 __global__ void __launch_bounds__(kFeatRows)
 quote_price_kernel(const double* __restrict__ fix, int64_t n, const float* __restrict__ y,
-                   double* __restrict__ out) {
+                   double* __restrict__ out, const int* __restrict__ err, int* __restrict__ out_err) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * kFeatRows + threadIdx.x;
     if (i >= n) return;
+    if (i == 0) *out_err = *err;
     const double spot = fix[i];  // 0: not the network's
     const double call = spot != 0.0 ? spot * static_cast<double>(y[i]) : 0.0;
     out[i] = call - fix[n + i] + fix[2 * n + i];
@@ -305,6 +308,7 @@ __device__ __forceinline__ void update_one(const UpdateArgs& a, int idx, float g
         a.G[idx] = g;
         return;
     }
+    if (a.st->err != 0) return;  // a failed pass: its sums are not gradients
     float p = a.P[idx], m = a.M[idx], v = a.V[idx];
     Adam(*a.st)(g, p, m, v);
     a.P[idx] = p;
@@ -424,6 +428,7 @@ __device__ __forceinline__ void update_weights(const UpdateArgs& a, int e, uint4
         *reinterpret_cast<float4*>(a.G + idx) = g;
         return;
     }
+    if (a.st->err != 0) return;
     float4 p = *reinterpret_cast<float4*>(a.P + idx);
     float4 m = *reinterpret_cast<float4*>(a.M + idx);
     float4 v = *reinterpret_cast<float4*>(a.V + idx);
@@ -467,7 +472,7 @@ __global__ void __launch_bounds__(kUpdThreads) update_kernel(const UpdateArgs a)
         __threadfence();
         if (atomicAdd(a.blocks_done, 1u) == gridDim.x - 1) {
             *a.blocks_done = 0u;
-            a.st->step += 1;
+            if (a.st->err == 0) a.st->step += 1;
         }
     }
 }
@@ -517,13 +522,14 @@ struct SurModel::StepLaunch {
 SurModel::~SurModel() {
     if (device_ < 0) return;
     DeviceGuard g(device_);
-    float* fl[] = {P_, M_, V_, G_, Tall_, Tb_, y_, dy_, dW1p_, dW2p_, dW3p_, loss_hist_, Py_, Pbase_};
+    float* fl[] = {P_, M_, V_, G_, Tall_, Tb_, y_, dy_, dW1p_, dW2p_, dW3p_, loss_hist_, Pbase_};
     for (float* p : fl)
         if (p) cudaFree(p);
     __nv_bfloat16* bl[] = {W1b_, W2b_, W3b_, W2Tb_, W3Tb_, Xall_, Z1_, H1_, Z2_, H3_, dZ3_, dZ2_, dZ1_,
                            PX_, PH1_, PH2_};
     for (__nv_bfloat16* p : bl)
         if (p) cudaFree(p);
+    if (Perr_) cudaFree(Perr_);
     if (perm_) cudaFree(perm_);
     if (state_) cudaFree(state_);
     if (blocks_done_) cudaFree(blocks_done_);
@@ -742,6 +748,7 @@ cudaError_t SurModel::train(int epochs, int batch, float lr0, uint64_t shuffle_s
     // steps_per_epoch and batch change the gather: keep the step counter and
     // make epoch boundaries relative to it
     QK_TRY(cudaMemcpy(state_, &s, sizeof s, cudaMemcpyHostToDevice));
+    QK_TRY(arm_timeout(&state_->err));
     StepLaunch step;
     QK_TRY(prepare_steps(true, &step));
     std::mt19937_64 rng(shuffle_seed);
@@ -765,6 +772,11 @@ cudaError_t SurModel::train(int epochs, int batch, float lr0, uint64_t shuffle_s
         for (int j = 0; j < spe; ++j) QK_TRY(run_step(step, stream_));
     }
     QK_TRY(cudaStreamSynchronize(stream_));
+    QK_TRY(cudaMemcpy(&s, state_, sizeof s, cudaMemcpyDeviceToHost));
+    if (s.err != 0) {
+        pipeline_code_ = s.err;
+        return cudaErrorLaunchTimeout;
+    }
     std::vector<float> hist(static_cast<size_t>(total));
     QK_TRY(cudaMemcpy(hist.data(), loss_hist_ + step0, hist.size() * sizeof(float), cudaMemcpyDeviceToHost));
     if (out_loss_last) *out_loss_last = hist.back();
@@ -782,7 +794,9 @@ cudaError_t SurModel::ensure_predict_buffers(int64_t rows, size_t in_row) {
     if (rows > pred_rows_) {
         pred_rows_ = 0;
         QK_TRY(dalloc(&PX_, static_cast<size_t>(rows) * kSurInPad));
-        QK_TRY(dalloc(&Py_, static_cast<size_t>(rows)));
+        QK_TRY(dalloc(&Perr_, static_cast<size_t>(rows) + 4));
+        QK_TRY(cudaMemsetAsync(Perr_, 0, kOutHead, stream_));
+        Py_ = reinterpret_cast<float*>(Perr_ + 4);
         QK_TRY(dalloc(&Pbase_, static_cast<size_t>(rows)));
         pred_rows_ = rows;
     }
@@ -807,6 +821,11 @@ cudaError_t SurModel::ensure_layered_buffers(int64_t rows) {
 
 cudaError_t SurModel::predict_device(const __nv_bfloat16* x, const float* base, int64_t n, float* y,
                                      cudaStream_t st, bool layered) {
+    return network(x, base, n, y, &state_->err, st, layered);
+}
+
+cudaError_t SurModel::network(const __nv_bfloat16* x, const float* base, int64_t n, float* y, int* err,
+                              cudaStream_t st, bool layered) {
     DeviceGuard g(device_);
     if (base_kind_ != kSurBaseNone && base == nullptr) return cudaErrorInvalidValue;
     if (!layered) {
@@ -826,7 +845,7 @@ cudaError_t SurModel::predict_device(const __nv_bfloat16* x, const float* base, 
         ia.b4 = P_ + SurLayout::b4;
         ia.base = base_kind_ != kSurBaseNone ? base : nullptr;
         ia.y = y;
-        ia.err = &state_->err;
+        ia.err = err;
         return launch_mlp_infer(tx, tw1, tw2, tw3, ia, sm_count_, st);
     }
     QK_TRY(ensure_layered_buffers(std::min<int64_t>(n, kPredChunk)));
@@ -838,14 +857,14 @@ cudaError_t SurModel::predict_device(const __nv_bfloat16* x, const float* base, 
                   tmap(&th2, PH2_, m, kSurHid, 128) && tmap(&tw3, W3b_, kSurHid, kSurHid, 256);
         if (!ok) return cudaErrorInvalidValue;
         GemmArgs f{};
-        f.err = &state_->err;
+        f.err = err;
         f.M = static_cast<int>(m); f.N = kSurHid; f.K = kSurInPad; f.k_per_split = kSurInPad;
         f.bias = P_ + SurLayout::b1; f.h_out = PH1_;
         QK_TRY(launch_umma_gemm(kEpiFwd, 128, tx, tw1, f, 1, st));
         f.K = kSurHid; f.k_per_split = kSurHid; f.bias = P_ + SurLayout::b2; f.h_out = PH2_;
         QK_TRY(launch_umma_gemm(kEpiFwd, 128, th1, tw2, f, 1, st));
         GemmArgs l{};
-        l.err = &state_->err;
+        l.err = err;
         l.M = static_cast<int>(m); l.N = kSurHid; l.K = kSurHid; l.k_per_split = kSurHid;
         l.bias = P_ + SurLayout::b3; l.w4 = P_ + SurLayout::w4; l.b4 = P_ + SurLayout::b4;
         l.y_out = y + off;
@@ -891,8 +910,9 @@ HostStage& thread_host_stage(int device) {
 // chunk's inputs are copied into its slot while the GPU works on the chunk
 // before it, and a chunk's results leave its slot when the slot comes up
 // again.  fill(h_in, off, m) copies inputs in, enqueue(h_in, h_out, m) queues
-// the chunk's work on stream_, its results ending in h_out, drain(h_out, off,
-// m) copies them to the caller.
+// the chunk's work on stream_, its results ending in h_out after kOutHead bytes
+// that start with the error word, drain(results, off, m) copies them to the
+// caller.  A chunk whose word is set has no results: the call fails.
 template <class Fill, class Enqueue, class Drain>
 cudaError_t SurModel::run_chunked(int64_t n, size_t in_row, size_t out_row, const Fill& fill,
                                   const Enqueue& enqueue, const Drain& drain) {
@@ -900,15 +920,24 @@ cudaError_t SurModel::run_chunked(int64_t n, size_t in_row, size_t out_row, cons
     QK_TRY(ensure_predict_buffers(chunk, in_row));
     HostStage& stage = thread_host_stage(device_);
     for (int s = 0; s < (n > chunk ? 2 : 1); ++s)
-        QK_TRY(stage.ensure(s, in_row * static_cast<size_t>(chunk), out_row * static_cast<size_t>(chunk)));
+        QK_TRY(stage.ensure(s, in_row * static_cast<size_t>(chunk),
+                            kOutHead + out_row * static_cast<size_t>(chunk)));
     struct Pending {
         int64_t off = 0, m = 0;
     } pending[2];
     cudaError_t e = cudaSuccess;
-    auto finish = [&](int s) {
+    auto finish = [&](int s) -> cudaError_t {
         if (pending[s].m == 0) return cudaSuccess;
-        const cudaError_t es = cudaEventSynchronize(stage.done[s]);
-        if (es == cudaSuccess) drain(static_cast<const char*>(stage.out[s].p), pending[s].off, pending[s].m);
+        cudaError_t es = cudaEventSynchronize(stage.done[s]);
+        if (es == cudaSuccess) {
+            const char* h = static_cast<const char*>(stage.out[s].p);
+            if (const int code = *reinterpret_cast<const int*>(h)) {
+                pipeline_code_ = code;
+                es = cudaErrorLaunchTimeout;
+            } else {
+                drain(h + kOutHead, pending[s].off, pending[s].m);
+            }
+        }
         pending[s].m = 0;
         return es;
     };
@@ -926,7 +955,10 @@ cudaError_t SurModel::run_chunked(int64_t n, size_t in_row, size_t out_row, cons
         const cudaError_t es = finish(s);
         if (e == cudaSuccess) e = es;
     }
-    if (e != cudaSuccess) cudaStreamSynchronize(stream_);  // nothing of the call stays in flight
+    if (e != cudaSuccess) {
+        cudaStreamSynchronize(stream_);  // nothing of the call stays in flight
+        cudaMemsetAsync(Perr_, 0, kOutHead, stream_);
+    }
     return e;
 }
 
@@ -941,9 +973,10 @@ cudaError_t SurModel::predict(const double* features, int64_t n, double* out) {
         [&](char* h_in, char* h_out, int64_t m) -> cudaError_t {
             QK_TRY(cudaMemcpyAsync(d_in_, h_in, row * static_cast<size_t>(m), cudaMemcpyHostToDevice, stream_));
             QK_TRY(features_device(d_in_, m, PX_, Pbase_, stream_));
-            QK_TRY(predict_device(PX_, Pbase_, m, Py_, stream_));
-            return cudaMemcpyAsync(h_out, Py_, sizeof(float) * static_cast<size_t>(m), cudaMemcpyDeviceToHost,
-                                   stream_);
+            QK_TRY(arm_timeout(Perr_));
+            QK_TRY(network(PX_, Pbase_, m, Py_, Perr_, stream_, false));
+            return cudaMemcpyAsync(h_out, Perr_, kOutHead + sizeof(float) * static_cast<size_t>(m),
+                                   cudaMemcpyDeviceToHost, stream_);
         },
         [&](const char* h, int64_t off, int64_t m) {
             const float* y = reinterpret_cast<const float*>(h);
@@ -968,12 +1001,14 @@ cudaError_t SurModel::price_quotes(const double* const (&cols)[10], const int32_
         [&](char* h_in, char* h_out, int64_t m) -> cudaError_t {
             const unsigned blocks = static_cast<unsigned>((m + kFeatRows - 1) / kFeatRows);
             const double* in = reinterpret_cast<const double*>(h_in);
-            double* price = reinterpret_cast<double*>(h_out);
+            double* price = reinterpret_cast<double*>(h_out + kOutHead);
             quote_features_kernel<<<blocks, kFeatRows, 0, stream_>>>(
                 in, m, box_, base_kind_, PX_, Pbase_, d_in_, reinterpret_cast<int32_t*>(price + m));
             QK_TRY(cudaGetLastError());
-            QK_TRY(predict_device(PX_, Pbase_, m, Py_, stream_));
-            quote_price_kernel<<<blocks, kFeatRows, 0, stream_>>>(d_in_, m, Py_, price);
+            QK_TRY(arm_timeout(Perr_));
+            QK_TRY(network(PX_, Pbase_, m, Py_, Perr_, stream_, false));
+            quote_price_kernel<<<blocks, kFeatRows, 0, stream_>>>(d_in_, m, Py_, price, Perr_,
+                                                                  reinterpret_cast<int*>(h_out));
             return cudaGetLastError();
         },
         [&](const char* h, int64_t off, int64_t m) {
@@ -1003,11 +1038,18 @@ cudaError_t SurModel::gradients(const double* features, const double* target, in
     }
     s.batch = n;
     s.steps_per_epoch = 1;
+    s.err = 0;
     QK_TRY(cudaMemcpy(state_, &s, sizeof s, cudaMemcpyHostToDevice));
+    QK_TRY(arm_timeout(&state_->err));
     StepLaunch step;
     QK_TRY(prepare_steps(false, &step));
     QK_TRY(run_step(step, stream_));
     QK_TRY(cudaStreamSynchronize(stream_));
+    QK_TRY(cudaMemcpy(&s, state_, sizeof s, cudaMemcpyDeviceToHost));
+    if (s.err != 0) {
+        pipeline_code_ = s.err;
+        return cudaErrorLaunchTimeout;
+    }
     std::vector<float> G(SurLayout::total);
     QK_TRY(cudaMemcpy(G.data(), G_, G.size() * sizeof(float), cudaMemcpyDeviceToHost));
     float l = 0.0f;
@@ -1048,10 +1090,16 @@ int SurModel::steps_done() const {
     return s.step;
 }
 
-int SurModel::device_error() {
-    SurState s{};
-    if (cudaMemcpy(&s, state_, sizeof s, cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
-    return s.err;
+int SurModel::take_pipeline_code() {
+    const int code = pipeline_code_;
+    pipeline_code_ = 0;
+    return code;
+}
+
+// The injected form of a wait that ran out in the kernels of the next launch.
+cudaError_t SurModel::arm_timeout(int* err) {
+    if (injected_fault(kFaultTimeout) == cudaSuccess) return cudaSuccess;
+    return cudaMemsetAsync(err, 1, sizeof(int), stream_);
 }
 
 // Checkpoint: "QKSURv02", layout size, base kind, the box, the state, P, M, V

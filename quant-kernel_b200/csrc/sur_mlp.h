@@ -45,7 +45,7 @@ struct SurState {
     int steps_per_epoch;
     int batch;
     float lr0, beta1, beta2, eps;
-    int err;           // GEMM error word
+    int err;           // error word of the training and device-inference kernels
     int step_begin;    // first step of the current schedule
     int pad[2];
 };
@@ -108,9 +108,15 @@ public:
     const SurBox& box() const { return box_; }
     int device() const { return device_; }
     int steps_done() const;
-    int device_error();
+    // The error code a tensor-core kernel of the last failed call recorded (a
+    // call that finds one returns cudaErrorLaunchTimeout), cleared by reading; 0
+    // if none.
+    int take_pipeline_code();
 
 private:
+    cudaError_t network(const __nv_bfloat16* x_rows, const float* base, int64_t n, float* y, int* err,
+                        cudaStream_t st, bool layered);
+    cudaError_t arm_timeout(int* err);
     cudaError_t ensure_batch_buffers(int batch);
     cudaError_t ensure_predict_buffers(int64_t rows, size_t in_row);
     cudaError_t ensure_layered_buffers(int64_t rows);
@@ -152,8 +158,11 @@ private:
     int64_t pred_rows_ = 0;
     int sm_count_ = 0;
     __nv_bfloat16 *PX_ = nullptr, *PH1_ = nullptr, *PH2_ = nullptr;
-    float* Py_ = nullptr;
+    // a chunk's error word (16 bytes) and outputs, one copy to the host
+    int* Perr_ = nullptr;
+    float* Py_ = nullptr;  // Perr_ + 4
     float* Pbase_ = nullptr;
+    int pipeline_code_ = 0;
     // host calls: device room for one chunk's inputs
     double* d_in_ = nullptr;
     size_t d_in_bytes_ = 0;
