@@ -1292,12 +1292,8 @@ template <int BN, int EPI>
 cudaError_t launch_t(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& a, int splits,
                      cudaStream_t st) {
     constexpr size_t smem = kStages * (kABytes + BN * kBK * 2) + 1024;
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(umma_gemm_kernel<BN, EPI>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    });
+    static DeviceOnce once;
+    const cudaError_t attr_err = allow_shared(once, umma_gemm_kernel<BN, EPI>, smem);
     if (attr_err != cudaSuccess) return attr_err;
     dim3 grid((a.M + kBM - 1) / kBM, a.N / BN, splits);
     umma_gemm_kernel<BN, EPI><<<grid, kGemmThreads, smem, st>>>(ta, tb, a);
@@ -1308,12 +1304,8 @@ cudaError_t launch_t(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArg
 
 cudaError_t launch_mlp_infer(const CUtensorMap& tx, const CUtensorMap& tw1, const CUtensorMap& tw2,
                              const CUtensorMap& tw3, const InferArgs& a, int ctas, cudaStream_t st) {
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(mlp_infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(kInferSmem));
-    });
+    static DeviceOnce once;
+    const cudaError_t attr_err = allow_shared(once, mlp_infer_kernel, kInferSmem);
     if (attr_err != cudaSuccess) return attr_err;
     if (a.n <= 0) return cudaSuccess;
     const int64_t tiles = (a.n + kBM - 1) / kBM;
@@ -1323,12 +1315,8 @@ cudaError_t launch_mlp_infer(const CUtensorMap& tx, const CUtensorMap& tw1, cons
 }
 
 cudaError_t launch_mlp_train(const TrainMaps& maps, const TrainArgs& a, cudaStream_t st) {
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(kTrainSmem));
-    });
+    static DeviceOnce once;
+    const cudaError_t attr_err = allow_shared(once, mlp_train_kernel, kTrainSmem);
     if (attr_err != cudaSuccess) return attr_err;
     if (a.batch <= 0 || a.batch % kBM != 0) return cudaErrorInvalidValue;
     return launch_dependent(mlp_train_kernel, a.batch / kBM, kTrainThreads, kTrainSmem, st, maps, a);

@@ -20,6 +20,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "device_once.h"
+
 namespace qkb {
 
 enum : int {
@@ -56,10 +58,18 @@ struct InferArgs {
     float* y;                // [n]
     int* err;                // error word (0 = ok)
 };
-// tx: x [n][64] and tw1: W1 [256][64] read through their first 16 columns
-// (make_tmap_bf16_k16: the 9 features and their zero padding; boxes 16 x 128
-// and 16 x 256, 32-byte swizzle); tw2, tw3: [256][256] (boxes 64 x 256).
-// ctas: persistent grid size (one CTA per SM).
+// Lets `kernel` use `bytes` of dynamic shared memory on the current device.
+template <typename... P>
+cudaError_t allow_shared(DeviceOnce& once, void (*kernel)(P...), size_t bytes) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    return once.run(dev, [&] {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(bytes));
+    });
+}
+
 // Launches a kernel that may start while the previous one of the stream still
 // runs: it calls griddepcontrol.wait before it touches what that one writes.
 // A training step is two short kernels; with the set-up of each under the tail
@@ -81,6 +91,10 @@ cudaError_t launch_dependent(void (*kernel)(P...), int grid, int threads, size_t
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// tx: x [n][64] and tw1: W1 [256][64] read through their first 16 columns
+// (make_tmap_bf16_k16: the 9 features and their zero padding; boxes 16 x 128
+// and 16 x 256, 32-byte swizzle); tw2, tw3: [256][256] (boxes 64 x 256).
+// ctas: persistent grid size (one CTA per SM).
 cudaError_t launch_mlp_infer(const CUtensorMap& tx, const CUtensorMap& tw1, const CUtensorMap& tw2,
                              const CUtensorMap& tw3, const InferArgs& a, int ctas, cudaStream_t st);
 

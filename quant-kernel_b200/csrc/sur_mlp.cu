@@ -16,7 +16,6 @@
 #include <cstring>
 #include <map>
 #include <memory>
-#include <mutex>
 #include <numeric>
 #include <random>
 #include <vector>
@@ -708,13 +707,8 @@ cudaError_t SurModel::prepare_steps(bool update, StepLaunch* s) {
 }
 
 cudaError_t SurModel::run_step(const StepLaunch& s, cudaStream_t st) {
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(kUpdSmem));
-    });
-    QK_TRY(attr_err);
+    static DeviceOnce once;
+    QK_TRY(allow_shared(once, update_kernel, kUpdSmem));
     QK_TRY(launch_mlp_train(s.maps, s.train, st));
     constexpr int kQuads = kW1Quads + 2 * kWQuads;
     return launch_dependent(update_kernel, kBiasBlocks + 1 + (kQuads + kUpdThreads - 1) / kUpdThreads, kUpdThreads,
