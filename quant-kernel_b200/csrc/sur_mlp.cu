@@ -533,6 +533,7 @@ SurModel::~SurModel() {
     if (state_) cudaFree(state_);
     if (blocks_done_) cudaFree(blocks_done_);
     if (d_in_) cudaFree(d_in_);
+    if (uploaded_) cudaEventDestroy(uploaded_);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -540,6 +541,7 @@ cudaError_t SurModel::init(uint64_t seed, const SurBox& box) {
     QK_TRY(cudaGetDevice(&device_));
     box_ = box;
     QK_TRY(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
+    QK_TRY(cudaEventCreateWithFlags(&uploaded_, cudaEventDisableTiming));
     QK_TRY(dalloc(&P_, SurLayout::total));
     QK_TRY(dalloc(&M_, SurLayout::total));
     QK_TRY(dalloc(&V_, SurLayout::total));
@@ -750,8 +752,8 @@ cudaError_t SurModel::train(int epochs, int batch, float lr0, uint64_t shuffle_s
     std::iota(perm.begin(), perm.end(), 0);
     // the gather reads perm[(step % spe) * batch + i]: the permutation goes up
     // rotated, in two pieces, so that the epoch starts at its beginning whatever
-    // step0 % spe is.  The copies run on the stream, after the epoch before, and
-    // have read perm when they return: the next shuffle overlaps this epoch.
+    // step0 % spe is.  The copies run on the stream, after the epoch before; the
+    // next shuffle waits for them and overlaps this epoch.
     const int64_t head = static_cast<int64_t>(spe - step0 % spe) * batch;
     const int64_t all = static_cast<int64_t>(spe) * batch;
     auto upload = [&](int64_t to, int64_t from, int64_t count) -> cudaError_t {
@@ -759,13 +761,21 @@ cudaError_t SurModel::train(int epochs, int batch, float lr0, uint64_t shuffle_s
         return cudaMemcpyAsync(perm_ + to, perm.data() + from, static_cast<size_t>(count) * sizeof(int32_t),
                                cudaMemcpyHostToDevice, stream_);
     };
-    for (int e = 0; e < epochs; ++e) {
-        std::shuffle(perm.begin(), perm.end(), rng);
-        QK_TRY(upload(all - head, 0, head));
-        QK_TRY(upload(0, head, all - head));
-        for (int j = 0; j < spe; ++j) QK_TRY(run_step(step, stream_));
-    }
-    QK_TRY(cudaStreamSynchronize(stream_));
+    auto enqueue_epochs = [&]() -> cudaError_t {
+        for (int e = 0; e < epochs; ++e) {
+            if (e > 0) QK_TRY(cudaEventSynchronize(uploaded_));
+            std::shuffle(perm.begin(), perm.end(), rng);
+            QK_TRY(upload(all - head, 0, head));
+            QK_TRY(upload(0, head, all - head));
+            QK_TRY(cudaEventRecord(uploaded_, stream_));
+            for (int j = 0; j < spe; ++j) QK_TRY(run_step(step, stream_));
+        }
+        return cudaSuccess;
+    };
+    const cudaError_t enqueued = enqueue_epochs();
+    const cudaError_t ran = cudaStreamSynchronize(stream_);  // also after an error: perm goes
+    QK_TRY(enqueued);
+    QK_TRY(ran);
     QK_TRY(cudaMemcpy(&s, state_, sizeof s, cudaMemcpyDeviceToHost));
     if (s.err != 0) {
         pipeline_code_ = s.err;

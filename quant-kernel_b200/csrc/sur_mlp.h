@@ -130,6 +130,7 @@ private:
 
     int device_ = -1;
     cudaStream_t stream_ = nullptr;
+    cudaEvent_t uploaded_ = nullptr;  // an epoch's permutation has left the host
     SurBox box_{};
     int32_t base_kind_ = kSurBaseBsmMeanVar;
     // parameters, Adam moments, gradient
