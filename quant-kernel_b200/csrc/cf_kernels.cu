@@ -659,7 +659,9 @@ bool g_cf_ready[kMaxDev] = {};
 
 namespace {
 
-// The Gauss-Legendre table of the current device, uploaded on first use.
+// The Gauss-Legendre table of the current device, uploaded on first use and
+// waited for: the kernels run on non-blocking streams, which the default
+// stream's copies are not ordered before.
 cudaError_t ensure_gl_table() {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -671,6 +673,7 @@ cudaError_t ensure_gl_table() {
         gl64(x, w);
         if ((e = cudaMemcpyToSymbol(c_gl_x, x, sizeof x)) != cudaSuccess) return e;
         if ((e = cudaMemcpyToSymbol(c_gl_w, w, sizeof w)) != cudaSuccess) return e;
+        if ((e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess) return e;
         g_cf_ready[dev] = true;
     }
     return cudaSuccess;

@@ -492,6 +492,15 @@ __global__ void refresh_kernel(const float* __restrict__ P, __nv_bfloat16* W1b, 
     }
 }
 
+// Host memory to the device, after the default stream's earlier work (a
+// caller's inference there) and done when it returns: cudaMemcpy alone returns
+// when the source has been read, and its transfer is not ordered before the
+// kernels of a non-blocking stream -- they met half of the parameters before it.
+cudaError_t put(void* dst, const void* src, size_t bytes) {
+    QK_TRY(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+    return cudaStreamSynchronize(cudaStreamLegacy);
+}
+
 bool tmap(CUtensorMap* m, const void* base, int64_t rows, int64_t cols, int box_rows) {
     return make_tmap_bf16(m, base, static_cast<uint64_t>(rows), static_cast<uint64_t>(cols),
                           static_cast<uint32_t>(box_rows));
@@ -615,11 +624,11 @@ cudaError_t SurModel::set_dataset(const double* features, const double* target, 
     QK_TRY(dalloc(&Xall_, static_cast<size_t>(n) * kSurInPad));
     QK_TRY(dalloc(&Tall_, static_cast<size_t>(n)));
     QK_TRY(dalloc(&perm_, static_cast<size_t>(n)));
-    QK_TRY(cudaMemcpy(Xall_, rows.data(), rows.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice));
-    QK_TRY(cudaMemcpy(Tall_, t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice));
+    QK_TRY(put(Xall_, rows.data(), rows.size() * sizeof(__nv_bfloat16)));
+    QK_TRY(put(Tall_, t.data(), t.size() * sizeof(float)));
     std::vector<int32_t> id(static_cast<size_t>(n));
     std::iota(id.begin(), id.end(), 0);
-    QK_TRY(cudaMemcpy(perm_, id.data(), id.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    QK_TRY(put(perm_, id.data(), id.size() * sizeof(int32_t)));
     n_data_ = n;
     return cudaSuccess;
 }
@@ -743,7 +752,7 @@ cudaError_t SurModel::train(int epochs, int batch, float lr0, uint64_t shuffle_s
     s.err = 0;
     // steps_per_epoch and batch change the gather: keep the step counter and
     // make epoch boundaries relative to it
-    QK_TRY(cudaMemcpy(state_, &s, sizeof s, cudaMemcpyHostToDevice));
+    QK_TRY(put(state_, &s, sizeof s));
     QK_TRY(arm_timeout(&state_->err));
     StepLaunch step;
     QK_TRY(prepare_steps(true, &step));
@@ -1043,7 +1052,7 @@ cudaError_t SurModel::gradients(const double* features, const double* target, in
     s.batch = n;
     s.steps_per_epoch = 1;
     s.err = 0;
-    QK_TRY(cudaMemcpy(state_, &s, sizeof s, cudaMemcpyHostToDevice));
+    QK_TRY(put(state_, &s, sizeof s));
     QK_TRY(arm_timeout(&state_->err));
     StepLaunch step;
     QK_TRY(prepare_steps(false, &step));
@@ -1083,7 +1092,7 @@ cudaError_t SurModel::set_parameters(const double* in) {
     for (int r = 0; r < kSurHid; ++r)
         for (int c = 0; c < kSurIn; ++c) P[SurLayout::W1 + r * kSurInPad + c] = static_cast<float>(in[k++]);
     for (int i = SurLayout::b1; i <= SurLayout::b4; ++i) P[i] = static_cast<float>(in[k++]);
-    QK_TRY(cudaMemcpy(P_, P.data(), P.size() * sizeof(float), cudaMemcpyHostToDevice));
+    QK_TRY(put(P_, P.data(), P.size() * sizeof(float)));
     QK_TRY(refresh_bf16(stream_));
     return cudaStreamSynchronize(stream_);
 }
@@ -1150,10 +1159,10 @@ cudaError_t SurModel::load(const char* path) {
     box_ = box;
     base_kind_ = kind;
     s.err = 0;
-    QK_TRY(cudaMemcpy(state_, &s, sizeof s, cudaMemcpyHostToDevice));
-    QK_TRY(cudaMemcpy(P_, buf.data(), SurLayout::total * sizeof(float), cudaMemcpyHostToDevice));
-    QK_TRY(cudaMemcpy(M_, buf.data() + SurLayout::total, SurLayout::total * sizeof(float), cudaMemcpyHostToDevice));
-    QK_TRY(cudaMemcpy(V_, buf.data() + 2 * SurLayout::total, SurLayout::total * sizeof(float), cudaMemcpyHostToDevice));
+    QK_TRY(put(state_, &s, sizeof s));
+    QK_TRY(put(P_, buf.data(), SurLayout::total * sizeof(float)));
+    QK_TRY(put(M_, buf.data() + SurLayout::total, SurLayout::total * sizeof(float)));
+    QK_TRY(put(V_, buf.data() + 2 * SurLayout::total, SurLayout::total * sizeof(float)));
     QK_TRY(refresh_bf16(stream_));
     return cudaStreamSynchronize(stream_);
 }
