@@ -679,17 +679,24 @@ constexpr double kZMax = 8.6;
 // Whether option o stays inside fp64_math's ranges, and then the starting
 // values of its sums: powers of two above 4 max y and 16 max y^2, from the
 // exponents of spot, strike and the largest path and weight factors.
-// Factors up to e^300 with spot, strike in [1e-100, 1e20] keep every y below
-// 1e152, so y^2 and its sums stay finite.  NaN constants fail the comparison.
+// Spot and strike in [1e-100, 1e20] and the factors below keep y^2 and its sums
+// far inside FP64's range.  A biased sum holds 106 bits below its bias, so the
+// bias may lie at most 2^45 above the smaller of spot and strike (2^40 here and
+// 5 bits of room): payoffs of that size then sum to 2^-60 of their total, far
+// below its last bit.  That is path factors up to e^27, four times the log-range
+// of an option at 50% volatility and two years; wilder ones take the general
+// unit, whose sums have no bias.  NaN constants fail the comparisons.
 __device__ __forceinline__ bool fp64_bounds(const McOption& o, double& b_y, double& b_q) {
     const double sh = o.model == kImportanceSampling ? fabs(o.d[2]) : 0.0;
     const double path = fabs(o.d[0]) + fabs(o.d[1]) * (kZMax + sh);
     const double weight = sh * (kZMax + 1.5 * sh);
-    if (!(path + weight <= 300.0 && o.spot >= 1e-100 && o.spot <= 1e20 && o.strike >= 1e-100 &&
+    if (!(path + weight <= 28.0 && o.spot >= 1e-100 && o.spot <= 1e20 && o.strike >= 1e-100 &&
           o.strike <= 1e20))
         return false;
-    const int32_t top = max(__double2hiint(o.spot), __double2hiint(o.strike)) >> 20;
+    const int32_t es = __double2hiint(o.spot) >> 20, ek = __double2hiint(o.strike) >> 20;
+    const int32_t top = max(es, ek);
     const int32_t grow = (int32_t)((float)(path + weight) * 1.4427f);
+    if (top - min(es, ek) + grow > 40) return false;
     // y <= (spot + strike) 2^(grow + 1) < 2^(top + grow + 3), biased exponent
     b_y = __hiloint2double((top + grow + 5) << 20, 0);
     b_q = b_y * b_y;
