@@ -42,15 +42,24 @@ constexpr int64_t kMinTerminalTiles = 32;
 constexpr int64_t kSmallBatchTiles = 296;
 // Two units a thread instead of four for long one-factor paths: no spills under
 // Euler's register bound, 66 registers instead of 80 for Milstein, a shorter
-// last wave; but a tile's fixed cost weighs on half the paths.
-// Four and two, us a call of 48 options: Euler at 126 steps 147 and 139 with
-// 2400 tiles (of four), 463 and 449 with 9600, 928 and 899 with 20016; Milstein
-// 95 and 90 with 1200, 260 and 255 with 4800, 478 and 480 with 9600 (719 and
-// 715 at 200 steps); at 24 steps and 4800 tiles four wins (Euler 88.1 and 89.6,
-// Milstein 89.5 and 92.9).
+// last wave; but a tile's fixed cost weighs on half the paths, so short paths
+// and full chips want four.  Two against four, by steps, in % of a call of 48
+// options (12 to 480 options lie within 2%):
+//   Euler     600 tiles  24: -3   60: -5    72: -4    126: -6   252: -8
+//            4800        24: +3   60: -2    72: -2    126: -5   252: -6
+//           20016        24: +6   60: 0     72: -0.5  126: -3   252: -4
+//   Milstein  600        24: 0    60: -3    72: -4    126: -5   252: -7
+//            4800        24: +5   60: 0     72: -1    126: -1.4 180: -2.5
+//            9600        24: +9   72: +1.4  126: +0.5 180: -0.5 252: -1.1
+//           20016        24: +9   72: +1.6  126: +0.6 180: -0.3 252: -1.1
+// Euler at 126 steps: 146.8 and 138.8 us with 2400 tiles, 926 and 898 with 20016.
 constexpr int64_t kLongPathSteps = 72;
 constexpr int64_t kMilsteinTiles = 6000, kMilsteinSteps = 180;
-constexpr int32_t kHostResultOptions = 64;
+// Two 8-byte stores an option over PCIe against a copy's launch.  The copy was
+// slower at every size measured: 33.6 against 30.0 us with one antithetic option
+// of 1000 paths, 34.2 and 29.9 with 64, 49.9 and 43.9 with 256, 64.2 and 58.2 with
+// 512, 87.3 and 83.0 with 1024 (Heston 98.4 and 92.8); beyond, not measured.
+constexpr int32_t kHostResultOptions = 1024;
 
 double nan_value() { return std::numeric_limits<double>::quiet_NaN(); }
 
@@ -525,9 +534,8 @@ cudaError_t Plan::build(const BatchInput& in, int32_t flags, std::string* err) {
     // more threads
     if (!persistent_ && !tuned_shape && !(flags & (kFlagStepUnroll2 | kFlagAutotune)))
         cfg_.upt = stepwise_batch_upt(cfg_, family_);
-    // Two 8-byte stores an option over PCIe against a copy's launch: a small
-    // batch's results go straight to the pinned buffer (one quote, with a
-    // single upload in place of three operations: 45 -> 25 us in the library)
+    // a small batch's results go straight to the pinned buffer (one quote, with
+    // a single upload in place of three operations: 45 -> 25 us in the library)
     one_shot_ = (flags & kFlagOneShot) != 0;
     host_results_ = one_shot_ && in.n <= kHostResultOptions;
     // QK_PLAN_STEP_UNROLL2: two step blocks per loop iteration where compiled
