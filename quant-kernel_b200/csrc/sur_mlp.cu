@@ -30,7 +30,8 @@ namespace qkb {
 namespace {
 
 constexpr int kPredChunk = 65536;
-constexpr size_t kOutHead = 4 * sizeof(int);  // a chunk's error word before its results
+// A chunk's error word before its results, which keep their alignment.
+constexpr size_t kOutHead = 256;
 
 #define QK_TRY(x)                                \
     do {                                         \
@@ -211,8 +212,8 @@ quote_price_kernel(const double* __restrict__ fix, int64_t n, const float* __res
     const int64_t i = static_cast<int64_t>(blockIdx.x) * kFeatRows + threadIdx.x;
     if (i >= n) return;
     if (i == 0) *out_err = *err;
-    const double spot = fix[i];  // 0: not the network's
-    const double call = spot != 0.0 ? spot * static_cast<double>(y[i]) : 0.0;
+    const double spot = fix[i], network = static_cast<double>(y[i]);
+    const double call = spot != 0.0 ? spot * network : 0.0;  // 0: not the network's
     out[i] = call - fix[n + i] + fix[2 * n + i];
 }
 
@@ -302,12 +303,14 @@ struct Adam {
     }
 };
 
-__device__ __forceinline__ void update_one(const UpdateArgs& a, int idx, float g) {
+// `failed`: the training pass did not complete, its sums are not gradients (read
+// at the kernel's start, ahead of the sums: at the update it cost 0.4 us a step).
+__device__ __forceinline__ void update_one(const UpdateArgs& a, bool failed, int idx, float g) {
     if (!a.update) {
         a.G[idx] = g;
         return;
     }
-    if (a.st->err != 0) return;  // a failed pass: its sums are not gradients
+    if (failed) return;
     float p = a.P[idx], m = a.M[idx], v = a.V[idx];
     Adam(*a.st)(g, p, m, v);
     a.P[idx] = p;
@@ -315,7 +318,7 @@ __device__ __forceinline__ void update_one(const UpdateArgs& a, int idx, float g
     a.V[idx] = v;
 }
 
-__device__ __forceinline__ void update_columns(const UpdateArgs& a, int block) {
+__device__ __forceinline__ void update_columns(const UpdateArgs& a, bool failed, int block) {
     const int lane = threadIdx.x & 31, pair = threadIdx.x >> 5;
     const int which = block >> 5, chunk = block & 31;
     const uint32_t* x = reinterpret_cast<const uint32_t*>((which < 3 ? a.dz[which] : a.h3) + chunk * 128 + lane) + pair;
@@ -362,11 +365,11 @@ __device__ __forceinline__ void update_columns(const UpdateArgs& a, int block) {
     if (lane < 2) {
         const int off = which == 0 ? SurLayout::b1 : which == 1 ? SurLayout::b2
                       : which == 2 ? SurLayout::b3 : SurLayout::w4;
-        update_one(a, off + chunk * 8 + pair * 2 + lane, lane == 0 ? s0 : s1);
+        update_one(a, failed, off + chunk * 8 + pair * 2 + lane, lane == 0 ? s0 : s1);
     }
 }
 
-__device__ __forceinline__ void update_loss(const UpdateArgs& a, float* s1, float* s2) {
+__device__ __forceinline__ void update_loss(const UpdateArgs& a, bool failed, float* s1, float* s2) {
     // chains t and t + 128 of 256
     const int t = threadIdx.x;
     float d1[2] = {}, d2[2] = {};
@@ -397,11 +400,11 @@ __device__ __forceinline__ void update_loss(const UpdateArgs& a, float* s1, floa
     if (t == 0) {
         const int k = a.st->step;
         if (k >= 0 && k < a.loss_cap) a.loss_hist[k] = s2[0] / static_cast<float>(a.batch);
-        update_one(a, SurLayout::b4, s1[0]);
+        update_one(a, failed, SurLayout::b4, s1[0]);
     }
 }
 
-__device__ __forceinline__ void update_weights(const UpdateArgs& a, int e, uint4* ring) {
+__device__ __forceinline__ void update_weights(const UpdateArgs& a, bool failed, int e, uint4* ring) {
     if (e >= kW1Quads + 2 * kWQuads) return;
     // W1's slabs hold the first 16 columns; the padding's gradient is zero and
     // leaves it zero
@@ -427,7 +430,7 @@ __device__ __forceinline__ void update_weights(const UpdateArgs& a, int e, uint4
         *reinterpret_cast<float4*>(a.G + idx) = g;
         return;
     }
-    if (a.st->err != 0) return;
+    if (failed) return;
     float4 p = *reinterpret_cast<float4*>(a.P + idx);
     float4 m = *reinterpret_cast<float4*>(a.M + idx);
     float4 v = *reinterpret_cast<float4*>(a.V + idx);
@@ -457,12 +460,13 @@ __global__ void __launch_bounds__(kUpdThreads) update_kernel(const UpdateArgs a)
     // what the training pass wrote is read from here on
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
+    const bool failed = a.st->err != 0;
     if (b < kBiasBlocks) {
-        update_columns(a, b);
+        update_columns(a, failed, b);
     } else if (b == kBiasBlocks) {
-        update_loss(a, reinterpret_cast<float*>(ring), reinterpret_cast<float*>(ring) + 256);
+        update_loss(a, failed, reinterpret_cast<float*>(ring), reinterpret_cast<float*>(ring) + 256);
     } else {
-        update_weights(a, (b - kBiasBlocks - 1) * kUpdThreads + threadIdx.x, ring);
+        update_weights(a, failed, (b - kBiasBlocks - 1) * kUpdThreads + threadIdx.x, ring);
     }
     if (!a.update) return;
     // every block has read the step; the last one advances it
@@ -471,7 +475,7 @@ __global__ void __launch_bounds__(kUpdThreads) update_kernel(const UpdateArgs a)
         __threadfence();
         if (atomicAdd(a.blocks_done, 1u) == gridDim.x - 1) {
             *a.blocks_done = 0u;
-            if (a.st->err == 0) a.st->step += 1;
+            if (!failed) a.st->step += 1;
         }
     }
 }
@@ -752,10 +756,6 @@ cudaError_t SurModel::train(int epochs, int batch, float lr0, uint64_t shuffle_s
     s.err = 0;
     // steps_per_epoch and batch change the gather: keep the step counter and
     // make epoch boundaries relative to it
-    QK_TRY(put(state_, &s, sizeof s));
-    QK_TRY(arm_timeout(&state_->err));
-    StepLaunch step;
-    QK_TRY(prepare_steps(true, &step));
     std::mt19937_64 rng(shuffle_seed);
     std::vector<int32_t> perm(static_cast<size_t>(n_data_));
     std::iota(perm.begin(), perm.end(), 0);
@@ -771,18 +771,22 @@ cudaError_t SurModel::train(int epochs, int batch, float lr0, uint64_t shuffle_s
                                cudaMemcpyHostToDevice, stream_);
     };
     auto enqueue_epochs = [&]() -> cudaError_t {
+        QK_TRY(cudaMemcpyAsync(state_, &s, sizeof s, cudaMemcpyHostToDevice, stream_));
+        QK_TRY(arm_timeout(&state_->err));
+        StepLaunch step;
+        QK_TRY(prepare_steps(true, &step));
         for (int e = 0; e < epochs; ++e) {
             if (e > 0) QK_TRY(cudaEventSynchronize(uploaded_));
             std::shuffle(perm.begin(), perm.end(), rng);
             QK_TRY(upload(all - head, 0, head));
             QK_TRY(upload(0, head, all - head));
-            QK_TRY(cudaEventRecord(uploaded_, stream_));
+            if (e + 1 < epochs) QK_TRY(cudaEventRecord(uploaded_, stream_));
             for (int j = 0; j < spe; ++j) QK_TRY(run_step(step, stream_));
         }
         return cudaSuccess;
     };
     const cudaError_t enqueued = enqueue_epochs();
-    const cudaError_t ran = cudaStreamSynchronize(stream_);  // also after an error: perm goes
+    const cudaError_t ran = cudaStreamSynchronize(stream_);  // also after an error: perm and s go
     QK_TRY(enqueued);
     QK_TRY(ran);
     QK_TRY(cudaMemcpy(&s, state_, sizeof s, cudaMemcpyDeviceToHost));
@@ -807,9 +811,9 @@ cudaError_t SurModel::ensure_predict_buffers(int64_t rows, size_t in_row) {
     if (rows > pred_rows_) {
         pred_rows_ = 0;
         QK_TRY(dalloc(&PX_, static_cast<size_t>(rows) * kSurInPad));
-        QK_TRY(dalloc(&Perr_, static_cast<size_t>(rows) + 4));
+        QK_TRY(dalloc(&Perr_, static_cast<size_t>(rows) + kOutHead / sizeof(int)));
         QK_TRY(cudaMemsetAsync(Perr_, 0, kOutHead, stream_));
-        Py_ = reinterpret_cast<float*>(Perr_ + 4);
+        Py_ = reinterpret_cast<float*>(Perr_ + kOutHead / sizeof(int));
         QK_TRY(dalloc(&Pbase_, static_cast<size_t>(rows)));
         pred_rows_ = rows;
     }
@@ -1026,7 +1030,11 @@ cudaError_t SurModel::price_quotes(const double* const (&cols)[10], const int32_
         },
         [&](const char* h, int64_t off, int64_t m) {
             const int32_t* to = reinterpret_cast<const int32_t*>(h + sizeof(double) * static_cast<size_t>(m));
-            for (int64_t i = 0; i < m; ++i) {
+            // a vector loop first, the one below only where there are some:
+            // alone it took 20,000 quotes from 207 to 230 us
+            int any = 0;
+            for (int64_t i = 0; i < m; ++i) any |= to[i] == 1;
+            for (int64_t i = 0; any && i < m; ++i) {
                 if (to[i] != 1) continue;
                 outside->index.push_back(static_cast<int32_t>(off + i));
                 outside->option_type.push_back(option_type[off + i]);

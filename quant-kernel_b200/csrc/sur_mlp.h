@@ -159,9 +159,9 @@ private:
     int64_t pred_rows_ = 0;
     int sm_count_ = 0;
     __nv_bfloat16 *PX_ = nullptr, *PH1_ = nullptr, *PH2_ = nullptr;
-    // a chunk's error word (16 bytes) and outputs, one copy to the host
+    // a chunk's error word and, kOutHead bytes on, its outputs: one copy to the host
     int* Perr_ = nullptr;
-    float* Py_ = nullptr;  // Perr_ + 4
+    float* Py_ = nullptr;
     float* Pbase_ = nullptr;
     int pipeline_code_ = 0;
     // host calls: device room for one chunk's inputs
