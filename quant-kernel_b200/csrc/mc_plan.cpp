@@ -103,15 +103,19 @@ int32_t geti(const int32_t* a, int32_t i, int32_t dflt) { return a ? a[i] : dflt
 // |z| <= 5.769, above the sqrt(2 24 ln 2) = 5.768 of a 23-bit Box-Muller
 // radius, with room for FP32 rounding.  A factor that only grows counts as 1:
 // the floor may be met at any step of the block, not only its last.  +inf (no
-// floor-free blocks) where no whole block runs or the bound leaves less than a
-// hundredth of the spot.
+// floor-free blocks) where no whole block runs, where the bound leaves less than
+// a hundredth of the spot, or where a path four deviations down ends below it
+// (of a warp's 256 paths and more some then do, and it runs all again: Milstein
+// at 800% volatility, 48 options x 100001 paths x 126 steps, 433 us against 263).
 float stepwise_block_min(double m0, double b, double fl, double c, int32_t steps) {
     double inc = m0 - 5.769 * b;
     // c z^2 >= 0, and the quadratic's vertex
     if (c > 0.0) inc = std::max(inc, m0 - b * b / (4.0 * c));
     const double g = std::min(0.9999 + inc, 1.0);
     const double limit = 1.001 * fl / (g * g * g * g * g * g);
-    return steps >= 6 && g > 0.05 && limit <= 0.01 ? (float)limit
+    // log-state after all steps: drift m0 + c - b^2 / 2 and deviation b a step
+    const double low = std::exp((m0 + c - 0.5 * b * b) * steps - 4.0 * b * std::sqrt((double)steps));
+    return steps >= 6 && g > 0.05 && limit <= 0.01 && low >= limit ? (float)limit
                                                     : std::numeric_limits<float>::infinity();
 }
 
