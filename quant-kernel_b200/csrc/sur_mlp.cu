@@ -1030,15 +1030,22 @@ cudaError_t SurModel::price_quotes(const double* const (&cols)[10], const int32_
         },
         [&](const char* h, int64_t off, int64_t m) {
             const int32_t* to = reinterpret_cast<const int32_t*>(h + sizeof(double) * static_cast<size_t>(m));
-            // a vector loop first, the one below only where there are some:
-            // alone it took 20,000 quotes from 207 to 230 us
-            int any = 0;
-            for (int64_t i = 0; i < m; ++i) any |= to[i] == 1;
-            for (int64_t i = 0; any && i < m; ++i) {
-                if (to[i] != 1) continue;
-                outside->index.push_back(static_cast<int32_t>(off + i));
-                outside->option_type.push_back(option_type[off + i]);
-                for (int c = 0; c < 10; ++c) outside->cols[c].push_back(cols[c][off + i]);
+            // a vector loop counts, the one below runs only where there are
+            // some: alone it took 20,000 quotes from 207 to 230 us
+            int64_t far = 0;
+            for (int64_t i = 0; i < m; ++i) far += to[i] == 1;
+            if (far > 0) {
+                const size_t at = outside->index.size();
+                outside->index.resize(at + static_cast<size_t>(far));
+                outside->option_type.resize(at + static_cast<size_t>(far));
+                int32_t* index = outside->index.data() + at;
+                for (int64_t i = 0, k = 0; k < far; ++i)
+                    if (to[i] == 1) index[k++] = static_cast<int32_t>(off + i);
+                for (int64_t k = 0; k < far; ++k) outside->option_type[at + k] = option_type[index[k]];
+                for (int c = 0; c < 10; ++c) {
+                    outside->cols[c].resize(at + static_cast<size_t>(far));
+                    for (int64_t k = 0; k < far; ++k) outside->cols[c][at + k] = cols[c][index[k]];
+                }
             }
             std::memcpy(out + off, h, sizeof(double) * static_cast<size_t>(m));
             if (route) std::memcpy(route + off, to, sizeof(int32_t) * static_cast<size_t>(m));
