@@ -76,13 +76,18 @@ PIPES = {"issue": float(ISSUE_PER_CLK), "xu": float(XU_PER_CLK), "fp64": float(F
 PROBE_KINDS = (("issue", 1), ("xu", 0), ("fp64", 3), ("ffma2_lanes", 2), ("xu_in_heston_mix", 4))
 
 
-
 def plan_upload_bytes(n: int) -> int:
     """Bytes a single-family batch of n options sends: 128-byte records, tile
     offsets (each padded to 256 bytes) and the work counter, one buffer."""
     def pad(x):
         return (x + 255) // 256 * 256
     return pad(128 * n) + pad(8 * (n + 1)) + 8
+
+
+def result_bytes(n: int) -> int:
+    """Bytes a batch call of n options gets back: prices and standard errors,
+    stored to pinned memory by the GPU, up to 1024; beyond, the prices copied."""
+    return 16 * n if n <= 1024 else 8 * n
 
 
 def measure_pipes(qk, device):
@@ -686,7 +691,7 @@ def main_gpu(args):
                    "parallelism": f"dp{world} (options sharded per rank, no collective)"},
         "prices_per_sec": world * n_opt * args.steps / (total_ms / 1e3),
         "e2e": {"value": world * units_per_step * args.steps / e2e_s, "unit": UNIT,
-                "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": n_opt * 8,
+                "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": result_bytes(n_opt),
                 "api": "qk_mcm_heston_monte_carlo_price_batch (host buffers)"},
         "gpu_launches": launches,
         "roofline": roofline,
@@ -1126,7 +1131,7 @@ def bsm_terminal_leg(qk, reps=20, f_mhz=1965.0, cpu=True):
     res = {"workload": "64 BSM calls/puts x 131072 paths (terminal GBM, antithetic pairs)",
            "dtype": "f64", "ms": ms, "paths_per_s": paths / (ms / 1e3), "e2e_ms": 1e3 * e2e,
            "e2e_paths_per_s": paths / e2e, "api": "qk_mcm_antithetic_variates_price_batch",
-           "h2d_bytes": plan_upload_bytes(n), "d2h_bytes": n * 8,
+           "h2d_bytes": plan_upload_bytes(n), "d2h_bytes": result_bytes(n),
            "roofline": {"bound": "fp64", "unit": "GFLOP/s",
                         "achieved": pairs * FP64_PER_PAIR / (kern_ms / 1e3) / 1e9,
                         "peak": fp64_peak / 1e9,

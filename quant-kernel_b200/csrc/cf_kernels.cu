@@ -353,11 +353,11 @@ __device__ __noinline__ Sums cf_general_nodes(const CfGeneral& g, int v) {
 
 // Bound by the FP64 pipe.  Three CTAs per SM (162 registers): the two values of
 // a node are independent chains, and what the compiler interleaves of them
-// hides more latency than more warps do (65536 options x 1024 nodes end to
-// end: 1.71 ms against 1.76, 1.76 and 1.80 with four, five and six CTAs; 1.82
-// with the exact M, whose prices are 5.6e-16 from an 80-bit evaluation where
-// the general form's are 1.0e-15; the general form for every option, packed
-// on the host, 6.60).
+// hides more latency than more warps do (four, five and six CTAs per SM ran 3,
+// 3 and 5% longer; M = beta - d by subtraction 6% shorter, but k2 t magnifies
+// its rounding: with the exact M prices are 5.6e-16 from an 80-bit evaluation,
+// the general form's 1.0e-15).  65536 options x 1024 nodes end to end 6.6 ->
+// 1.77 ms; the general form for every option 3.2-6.2 ms by its parameters.
 template <int WARPS>
 __global__ void __launch_bounds__(128, 3)
     heston_cf_kernel(const double* __restrict__ in, int32_t m, double* __restrict__ out) {
@@ -679,13 +679,17 @@ cudaError_t ensure_gl_table() {
     return cudaSuccess;
 }
 
-// A batch that fills the chip with one option per warp (4 a CTA, five CTAs on
-// each of 148 SMs) takes that form, whose per-option work is done by one warp
-// instead of four; below it four warps share an option, which divides a lone
-// quote's chain of nodes by four (one option, 1024 nodes: 61 us a call against
-// 85 before; 4097 options of 2048 nodes 0.28 ms against 0.73).  The sums are
-// the same bits.
-constexpr int32_t kWarpPerOption = 148 * 5 * 4;
+// From here on one warp takes an option, whose per-option work is then done once
+// instead of four times; below, four warps share it, which divides a lone
+// quote's chain of nodes by four.  The sums are the same bits.  Where the two
+// meet depends on the work an option has; one and four warps, us a call:
+//   CF 256 nodes    592: 49.5 51.6   1776: 63.8 72.7   2960: 82.7 85.2   4736: 108 120
+//     1024          148: 59.7 47.5    888: 82.8 71.6   2960: 133  134    4736: 188 197
+//     2048          148: 84.5 48.6   1184: 111  110    2960: 207  209    8192: 507 515
+//   COS 64 terms    592: 45.1 45.2    888: 49.3 57.5   2960: 57.5 68.4   4736: 73.4 92.2
+//     256           592: 50.5 50.7   1776: 63.2 63.5   2960: 68.7 76.7   4736: 88.0 98.8
+//     512           592: 88.3 57.7   1776: 100  75.6   2960: 108  84.7   8192: 188 178
+constexpr int32_t kWarpPerOption = 2960;
 
 cudaError_t launch_fourier(FourierMethod method, const double* d_in, int32_t m, double* d_out,
                            bool warp_per_option, cudaStream_t st) {

@@ -125,15 +125,17 @@ __device__ __forceinline__ double fp64_rsqrt_seed(double x) {
     return y;
 }
 
-// 1/x for normal x with a normal reciprocal: y + y e (1 + e), e = 1 - x y,
-// which leaves e^3 < 2^-57.
+// 1/x for normal x with a normal reciprocal: from 1/x = y (1 - e)^-1, e = 1 - x y,
+// the geometric series to its square (Householder's method of the third order
+// for 1/y - x), which leaves e^3 < 2^-57.
 __device__ __forceinline__ double fp64_rcp(double x) {
     const double y = fp64_rcp_seed(x);
     const double e = fma(-x, y, 1.0);
     return fma(y, fma(e, e, e), y);
 }
 
-// 1/sqrt(x), sqrt(x) for normal x > 0: t (1 + e/2 + 3 e^2/8), e = 1 - x y^2,
+// 1/sqrt(x), sqrt(x) for normal x > 0: from x^(-1/2) = y (1 - e)^(-1/2), e = 1 -
+// x y^2, the binomial series 1 + e/2 + 3 e^2/8 (the same method for y^-2 - x),
 // which leaves (5/16) e^3 < 2^-55 (e < 2^-18).
 __device__ __forceinline__ double fp64_rsqrt(double x) {
     const double y = fp64_rsqrt_seed(x);

@@ -11,7 +11,12 @@
 // double-double sums of y and y^2 (y = pair mean or payoff) are reduced
 // warp -> CTA in a fixed order and written to the tile's slot; the finalize
 // kernel merges an option's slots in tile order.  Results are therefore
-// deterministic and a batch reproduces the scalar call bit for bit.
+// deterministic.  A batch reproduces the scalar call: the terminal families'
+// tiles depend on the option alone, and a stepwise price is the same bits in any
+// grouping (its payoffs are whole multiples of a quarter of the strike's last
+// bit, so double-double sums of less than 2^50 strikes are exact).  Squares and
+// the likelihood-ratio weights have more bits: stepwise standard errors and
+// deltas agree to their final rounding where the units per thread differ.
 //
 // Reference loops restated (yluoc/Quant-Kernel):
 //   terminal   mc_engine.h:32-75   + model_concepts.h:93-102
@@ -670,9 +675,9 @@ __device__ __noinline__ Acc vr_units(const McOption* __restrict__ rec, uint32_t 
 // the double-double sums start at a power of two above every term, so that
 // each addition's error comes from a three-operation FastTwoSum instead of
 // TwoSum's six and its finiteness test.
-// Measured: 64 x 131072 antithetic paths, kernel 49.5 -> 33 us; 64 x 2^20
-// paths end to end, importance sampling 719 -> 483 us, control variates 634 ->
-// 437, stratified 635 -> 413, Halton 762 -> 360, Sobol 944 -> 378 us.
+// Measured: 64 x 131072 antithetic paths, kernel 49.5 -> 34 us; 64 x 2^20
+// paths end to end, importance sampling 714 -> 436 us, control variates 632 ->
+// 406, stratified 640 -> 366, Halton 757 -> 302, Sobol 940 -> 328 us.
 // ----------------------------------------------------------------------------
 
 // Largest |z|: Box-Muller radii reach sqrt(2 53 ln 2) = 8.572, Acklam's inverse

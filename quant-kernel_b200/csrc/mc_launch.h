@@ -25,8 +25,8 @@ enum : int {
 // the mixed benchmark batch ran 52.9 ms with four (persistent kernel, seven
 // CTAs per SM) against 56.1 ms with two stepwise units per thread; Heston
 // keeps two, whose four-unit body needs 79-93 registers.
-// Results do not depend on these (tile sums are exact double-double sums
-// merged in a fixed order).
+// Prices do not depend on these (double-double sums of payoffs are exact);
+// standard errors do in their final rounding.
 constexpr int kUptTerminal = 1;
 constexpr int kUptStepwise = 4;
 constexpr int kUptHeston = 2;
@@ -35,7 +35,8 @@ constexpr int kUptVr = 1;
 // The one family -> units-per-thread map: the persistent kernel's family
 // bodies, the tiling of every mixed plan and the default single-family
 // tiling take it (stepwise_batch_upt lowers the last for small batches and
-// long one-factor paths; the sums give the same bits).
+// long one-factor paths: the same price bits, standard errors to their final
+// rounding).
 constexpr int family_upt(int family) {
     return family == kFamTerminal ? kUptTerminal
          : family == kFamVr ? kUptVr

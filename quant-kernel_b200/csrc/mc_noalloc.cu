@@ -64,8 +64,8 @@ cudaStream_t g_stream_dev[kMaxDevices] = {};     // per-device stream, set once
 
 // Fixed launch shape: 256 threads x 2 pairs = 512 antithetic pairs per tile
 // pass.  The regular entry uses 128-thread CTAs; the same paths summed in
-// other tile groups agree to ~1e-15 relative (double-double sums), not always
-// bit for bit.
+// other tile groups give the same price bits (double-double sums of payoffs are
+// exact), and standard errors that may differ in their last one.
 constexpr int kBlock = 256;
 constexpr int kUpt = 2;
 

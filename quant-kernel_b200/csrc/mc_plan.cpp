@@ -314,8 +314,8 @@ int32_t tile_option(McOption& o, int block, int upt) {
     // tile's fixed cost -- record load, option search and the double-double
     // CTA reduction -- so large terminal options give each thread several
     // units, while keeping at least kMinTerminalTiles tiles to spread over
-    // the SMs.  A function of the option alone, like the rest of the
-    // geometry: a batch and a scalar call tile an option the same way.
+    // the SMs.  A function of the option and its units per thread alone: a batch
+    // and a scalar call tile a terminal option the same way.
     const int fam = family_of(o.model);
     if (fam == kFamTerminal || fam == kFamVr) {
         const int64_t cap = units / (per_iter * kMinTerminalTiles);
@@ -374,8 +374,9 @@ void PinnedBuf::release() {
 // steps) block 128 ran 2.4% faster than 256 with the same registers (six CTAs
 // of 128 per SM instead of three of 256: finer tiles, a shorter tail), and the
 // autotuner picked it for the mixed-model batch too.  One block size for every
-// family, and each family's units per thread from family_upt(), keep the
-// persistent and single-family tilings identical, so both give the same bits.
+// family, and each family's units per thread from family_upt(), give the
+// persistent and the family-grid mode the same tiles, and single-family batches
+// too, but for those that stepwise_batch_upt spreads over more threads.
 LaunchConfig default_config(int family) {
     LaunchConfig c;
     c.block = 128;
@@ -573,8 +574,8 @@ static int family_rank(int fam) {
 // Units per thread for a stepwise single-family batch: the family's own, or two
 // for long one-factor paths, while that makes at least kSmallBatchTiles tiles,
 // else halved (and halved again), which spreads the same paths over more warps.
-// A path's normals and arithmetic do not change, and tile sums are
-// double-double.
+// A path's normals and arithmetic do not change, and the payoffs' double-double
+// sums are exact: the same price bits as in any other batch.
 int Plan::stepwise_batch_upt(const LaunchConfig& cfg, int family) const {
     if (!family_is_stepwise(family)) return cfg.upt;
     // units reach 2^31 - 1

@@ -9,8 +9,9 @@
 //   * warp 1 / lane 0 issues tcgen05.mma (kind::f16, BF16 x BF16 -> FP32,
 //     M = 128, N = BN, K = 16 per instruction) from shared-memory descriptors
 //     into a TMEM accumulator, and frees a stage with tcgen05.commit;
-//   * all four warps then read the accumulator with tcgen05.ld (warp w owns
-//     TMEM lanes 32w..32w+31 = tile rows) and run the fused epilogue.
+//   * all eight warps then read the accumulator with tcgen05.ld (warp w reads
+//     TMEM lanes 32 (w % 4) .. + 31 = tile rows, column half w / 4) and run the
+//     fused epilogue.
 // Every mbarrier wait is bounded: on timeout the kernel records an error code
 // in *err, drains what it issued (again bounded), frees its TMEM and returns.
 #pragma once

@@ -149,10 +149,11 @@ features_kernel(const double* __restrict__ f, int64_t n, SurBox box, int32_t kin
 // checks of heston_monte_carlo.cpp:18-26 -- and writes the network's row (its
 // first 32 bytes, all that the fused kernel reads) and base; other routes get
 // a row of zeros.  fix holds what quote_price_kernel needs: (spot, S e^-qT, K
-// e^-rT) for a put, (spot, 0, 0) for a call, (0, -result, 0) for routes 1, 2.
+// e^-rT) for a put, (spot, 0, 0) for a call, (0, -result, 0) for routes 1, 2,
+// whose price the network's output does not enter, whatever it is.
 // Bound by the copy into the slot and PCIe (84 bytes an option): on the host,
 // the checks, bf16 rows and base took 180 ns an option on one thread (20,000
-// quotes 3.70 ms a call, now 0.23; 200,000 34 ms, now 1.46).
+// quotes 3.70 ms a call, now 0.21; 200,000 34 ms, now 1.27).
 __global__ void __launch_bounds__(kFeatRows)
 quote_features_kernel(const double* __restrict__ in, int64_t n, SurBox box, int32_t kind,
                       __nv_bfloat16* __restrict__ rows, float* __restrict__ base,

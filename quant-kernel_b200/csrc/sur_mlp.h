@@ -37,8 +37,8 @@ struct SurLayout {
     static constexpr int total = b4 + 4;  // padded to 16 bytes
 };
 
-// Training state read by the kernels of a captured step (graph replays see
-// the current values).
+// Training state on the device, read by a step's kernels: the launches of a
+// call are alike, the step counter and the schedule advance here.
 struct SurState {
     int step;          // completed optimiser steps
     int total_steps;   // cosine schedule length
