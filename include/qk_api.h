@@ -362,7 +362,7 @@ QK_EXPORT int32_t qk_mcm_plan_create(
     qk_mc_plan** out_plan);
 QK_EXPORT int32_t qk_mcm_plan_execute(qk_mc_plan* plan, void* stream);
 QK_EXPORT int32_t qk_mcm_plan_results(qk_mc_plan* plan, double* out_prices, double* out_stderr);
-/* Device pointers to the plan's result arrays (n doubles each). */
+/* Device pointers to the plan's result arrays (n doubles each, 256-byte aligned). */
 QK_EXPORT int32_t qk_mcm_plan_device_results(qk_mc_plan* plan, double** d_prices,
                                              double** d_stderr);
 /* Milliseconds of the last execute()'s simulate kernel (QK_PLAN_TIMING), and
